@@ -37,25 +37,34 @@ def _t():
     return _torch
 
 
-def _resolve(data, elem_bytes=None, stream=None):
-    """-> (pointer, element bytes, stream handle)"""
+def _handles(data, elem_bytes=None, stream=None):
+    """-> (address, element bytes, stream handle), as integers.
+
+    A small call is bound by its host path, so a tensor's stream is asked for
+    as the raw handle: torch's Stream object and the ctypes boxes around the
+    arguments cost 2.3 us of the 7.8 that a call on fp32 (64, 48, 4) took."""
     if hasattr(data, "data_ptr"):
-        torch = _t()
         if not data.is_cuda:
             raise ValueError("tensor must live on a CUDA device (use transpose_host for host tensors)")
         if not data.is_contiguous():
             raise ValueError("tensor must be contiguous")
         eb = data.element_size() if elem_bytes is None else int(elem_bytes)
         if stream is None:
-            stream = torch.cuda.current_stream(data.device).cuda_stream
+            stream = _t()._C._cuda_getCurrentRawStream(data.get_device())
         elif hasattr(stream, "cuda_stream"):
             stream = stream.cuda_stream
-        return ctypes.c_void_p(data.data_ptr()), eb, ctypes.c_void_p(int(stream))
+        return data.data_ptr(), eb, int(stream)
     if elem_bytes is None:
         raise ValueError("elem_bytes is required with a raw pointer")
     if hasattr(stream, "cuda_stream"):
         stream = stream.cuda_stream
-    return ctypes.c_void_p(int(data)), int(elem_bytes), ctypes.c_void_p(int(stream or 0))
+    return int(data), int(elem_bytes), int(stream or 0)
+
+
+def _resolve(data, elem_bytes=None, stream=None):
+    """-> (pointer, element bytes, stream handle)"""
+    p, eb, st = _handles(data, elem_bytes, stream)
+    return ctypes.c_void_p(p), eb, ctypes.c_void_p(st)
 
 
 class Functor:
@@ -122,8 +131,10 @@ def scatter_permute(fn, d3, d2, d1, data, *, elem_bytes=None, stream=None):
 
 
 def _shape_call(cfn, data, d1, d2, d3, elem_bytes=None, stream=None):
-    p, eb, st = _resolve(data, elem_bytes, stream)
-    check(cfn(p, int(d1), int(d2), int(d3), eb, st))
+    p, eb, st = _handles(data, elem_bytes, stream)
+    status = cfn(p, int(d1), int(d2), int(d3), eb, st)
+    if status:
+        check(status)
 
 
 def transpose(data, d1, d2, d3, *, elem_bytes=None, stream=None):

@@ -39,14 +39,22 @@ def _check_dims(x: torch.Tensor, dim0: int, dim1: int) -> None:
         raise ValueError("t213.transpose_ needs a contiguous tensor")
 
 
+def _strides(shape) -> list:
+    """Strides of a new contiguous tensor of this shape."""
+    st = [1] * len(shape)
+    for i in range(len(shape) - 2, -1, -1):
+        st[i] = st[i + 1] * max(1, shape[i + 1])
+    return st
+
+
 def _impl(x: torch.Tensor, dim0: int = -2, dim1: int = -1) -> torch.Tensor:
     _check_dims(x, dim0, dim1)
-    d1, d2 = x.size(-1), x.size(-2)
-    d3 = math.prod(x.shape[:-2])
-    if x.numel():
+    *lead, d2, d1 = x.shape
+    d3 = math.prod(lead)
+    if d1 and d2 and d3:
         _transpose(x, d1, d2, d3)
-    shape = tuple(x.shape[:-2]) + (d1, d2)
-    return x.as_strided_(shape, torch.empty(shape, device="meta").stride())
+    shape = (*lead, d1, d2)
+    return x.as_strided_(shape, _strides(shape))
 
 
 torch.library.impl(_LIB, "transpose_", "CUDA")(_impl)
@@ -90,7 +98,7 @@ def _permute_impl(x: torch.Tensor, dims) -> torch.Tensor:
         ref_dims = [x.size(n - 1 - a) for a in range(n)]
         ref_perm = [n - 1 - p[n - 1 - j] for j in range(n)]
         _permute(x, ref_dims, ref_perm)
-    return x.as_strided_(shape, torch.empty(shape, device="meta").stride())
+    return x.as_strided_(shape, _strides(shape))
 
 
 @torch.library.impl(_LIB, "permute_", "CPU")
