@@ -411,11 +411,16 @@ namespace t213 {
 std::shared_ptr<Plan> group_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int *status, bool search_slice) {
   std::shared_ptr<Plan> P = get_plan(d1, d2, d3, eb, T213_PLAN_AUTO, 0, status);
   if (!P) return nullptr;
+  if (P->kind == T213_PLAN_SLICE) {
+    // A caller that plans as requests arrive leaves the tensors whose one-pass
+    // form is the aligned one, which run best on their own launch; the others
+    // take their best plan of two sweeps or more.
+    const bool aligned = (d1 * eb) % 16 == 0 && (d2 * eb) % 16 == 0 && d1 * d2 * d3 * eb <= (16ll << 20);
+    if (aligned && !search_slice) return nullptr;
+    P = get_plan(d1, d2, d3, eb, kPlanSweeps, 0, status);
+    if (!P) return nullptr;
+  }
   if (plan_fits_batch(*P)) return P;
-  // a tensor whose own plan is the one-pass slice plan runs best on its own
-  // launch; searching the other families builds their cycle tables, which a
-  // caller planning as requests arrive cannot afford
-  if (P->kind == T213_PLAN_SLICE && !search_slice) return nullptr;
   // the cheapest other family whose passes fit the persistent kernel's
   // shared memory
   std::shared_ptr<Plan> best;
@@ -583,7 +588,8 @@ int t213_batch_create(const t213_tensor_desc *tensors, int32_t count, t213_batch
     std::shared_ptr<Plan> P;
     if (d.d1 * d.d2 * d.d3 > 0) {
       P = d.plan_kind == T213_PLAN_AUTO ? group_plan(d.d1, d.d2, d.d3, d.elem_bytes, &rc, true) : nullptr;
-      if (!P) P = get_plan(d.d1, d.d2, d.d3, d.elem_bytes, d.plan_kind, 0, &rc);
+      if (!P)
+        P = get_plan(d.d1, d.d2, d.d3, d.elem_bytes, d.plan_kind == T213_PLAN_AUTO ? kPlanSweeps : d.plan_kind, 0, &rc);
       if (!P) return fail(rc);
       if (!plan_fits_batch(*P) || d.d1 * d.d2 * d.d3 * d.elem_bytes > direct_threshold()) B->spill.push_back(i);
     }

@@ -162,10 +162,31 @@ int launch_tile_swap(char *data, int64_t d3, int64_t m, int64_t n, int64_t t, in
 int launch_band_transpose(char *data, int64_t n_bands, int64_t R, int64_t C, int eb, cudaStream_t st,
                           LaunchStats *ls);
 int64_t band_smem_bytes(int64_t R, int64_t C, int eb);
-// One-pass transpose of slices held whole in a cluster's shared memory.
-int launch_slice(char *data, int64_t d3, int64_t m, int64_t n, int eb, cudaStream_t st, LaunchStats *ls);
+// One-pass transpose of slices held whole in the shared memory of a team of
+// CTAs (k_hold.cuh): the tiling for any base address and, where the pitches
+// allow it, the one of the vector form for 16-byte aligned bases.
+enum HoldMode { HOLD_CTA = 0, HOLD_CLUSTER = 1, HOLD_GRID = 2 };  // a team: one CTA, a cluster, more CTAs
+struct HoldGeom {
+  bool ok = false;
+  bool packed = false;
+  int mode = 0, form = 0;
+  uint32_t tm = 0, tn = 0, TC = 0, T = 0, ctas = 0, teams = 0, S = 0, P = 0;
+  double est_us = 0;  // modelled time of the launch
+};
+struct HoldReady;  // what a launch asks of the device and prepares, once per plan
+struct HoldPlan {
+  HoldGeom any, vec;
+  std::shared_ptr<HoldReady> ready;
+};
+// we: 16-byte words per element (wide elements, eb == 16), else 1.
+void hold_plan(HoldPlan &hp, int64_t m, int64_t n, int eb, int64_t we, int64_t d3);
+// launch_slice could not have all its CTAs resident, or no barrier slot is
+// left: nothing was launched, the caller takes another plan.
+constexpr int kHoldNoSlot = -2;
+int launch_slice(const HoldPlan &hp, char *data, int64_t d3, int64_t m, int64_t n, int eb, int64_t we,
+                 cudaStream_t st, LaunchStats *ls);
 bool slice_fits(int64_t m, int64_t n, int eb);
-std::string describe_slice(int64_t m, int64_t n, int eb, int64_t d3);
+std::string describe_slice(const HoldPlan &hp);
 // Grouped one-pass slices (the batched form): the rows per CTA H and padded
 // pitch P of a slice split over an 8-CTA cluster (false if it does not fit),
 // and one launch of the grouped kernel over device SliceEntry records.

@@ -1,5 +1,6 @@
-// One-pass 213 transpose of slices that fit a thread-block cluster's shared
-// memory (up to 16 CTAs of about 220 KB: slices of a few MB).
+// Grouped one-pass 213 transpose of many tensors' slices in one launch (the
+// batched form, on request); each slice fits a thread-block cluster's shared
+// memory.
 //
 // A cluster of K CTAs takes one slice (m = d2 rows of n = d1 elements) at a
 // time.  CTA r loads source rows [r*H, (r+1)*H) into its shared memory (row
@@ -157,17 +158,6 @@ __device__ __forceinline__ void cluster_coords(uint32_t &rank, uint32_t &K, int6
     u0 = blockIdx.x / K;
     ustride = gridDim.x / K;
   }
-}
-
-template <int EB, bool VEC, bool CLUSTER>
-__global__ void __launch_bounds__(kSliceThreads)
-    k_slice(char *__restrict__ data, int64_t d3, uint32_t m, uint32_t n, uint32_t H, uint32_t P) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  uint32_t rank, K;
-  int64_t u0, ustride;
-  cluster_coords<CLUSTER>(rank, K, u0, ustride);
-  const int64_t slice_bytes = (int64_t)m * n * EB;
-  for (int64_t u = u0; u < d3; u += ustride) slice_item<EB, VEC, CLUSTER>(data + u * slice_bytes, m, n, H, P, rank, K, smem_raw);
 }
 
 // Many tensors' slices in one launch (the batched form): entry e has d3

@@ -986,44 +986,7 @@ namespace {
 constexpr int64_t kSliceSmemCap = 220 * 1024;
 constexpr int kSliceGroupK = 8;  // cluster size of the batched form's grouped slice launch
 
-struct SliceCfg {
-  int K = 0;
-  uint32_t H = 0, P = 0;
-  int64_t smem = 0;
-  bool vec = false;
-};
-
-// Cluster size, rows per CTA and padded row pitch for one-pass slices; K = 0
-// when the slice does not fit 16 CTAs.  The smallest cluster that holds the
-// slice, doubled (up to 8) while the slices still leave SMs idle.
-SliceCfg slice_config(int64_t m, int64_t n, int eb, int64_t d3, const void *data) {
-  SliceCfg c;
-  if (m < 2 || n < 2 || m > (1 << 24) || n > (1 << 24)) return c;
-  int64_t P = (n * eb + 15) / 16 * 16;
-  if ((P / 16) % 2 == 0) P += 16;  // consecutive rows in different 16-byte bank groups
-  auto rows = [&](int K) -> int64_t {
-    if (K == 1) return m;
-    return ((m + K - 1) / K + 31) / 32 * 32;
-  };
-  int K = 0;
-  for (int k : {1, 2, 4, 8, 16})
-    if (rows(k) * P <= kSliceSmemCap) {
-      K = k;
-      break;
-    }
-  if (!K) return c;
-  (void)d3;  // the launch widens the cluster when slices leave SMs idle
-  c.K = K;
-  c.H = (uint32_t)rows(K);
-  c.P = (uint32_t)P;
-  c.smem = (int64_t)c.H * P;
-  c.vec = (n * eb) % 16 == 0 && (m * eb) % 16 == 0 && ((uintptr_t)data % 16) == 0;
-  return c;
-}
-
 }  // namespace
-
-bool slice_fits(int64_t m, int64_t n, int eb) { return slice_config(m, n, eb, 1, nullptr).K > 0; }
 
 bool slice_group_params(int64_t m, int64_t n, int eb, const void *data, uint32_t *H, uint32_t *P, bool *vec) {
   if (m < 2 || n < 2 || m > (1 << 24) || n > (1 << 24)) return false;
@@ -1047,96 +1010,6 @@ int launch_slice_group(const void *entries, int32_t n_entries, int64_t n_items, 
   const int64_t clusters = std::min<int64_t>(n_items, res);
   return launch_k(kern, clusters * kSliceGroupK, kSliceThreads, smem, kSliceGroupK, st,
                   (const SliceEntry *)entries, n_entries, n_items);
-}
-
-std::string describe_slice(int64_t m, int64_t n, int eb, int64_t d3) {
-  SliceCfg c = slice_config(m, n, eb, d3, nullptr);
-  char buf[96];
-  snprintf(buf, sizeof buf, "slice(cluster=%d rows/cta=%u smem=%lldK)", c.K, c.H, (long long)(c.smem / 1024));
-  return buf;
-}
-
-int launch_slice(char *data, int64_t d3, int64_t m, int64_t n, int eb, cudaStream_t st, LaunchStats *ls) {
-  if (d3 <= 0 || m <= 0 || n <= 0) return T213_OK;
-  const SliceCfg c0 = slice_config(m, n, eb, d3, data);
-  if (!c0.K) {
-    set_error("slice does not fit a cluster's shared memory");
-    return T213_ERR_UNSUPPORTED;
-  }
-  int status = T213_ERR_UNSUPPORTED;
-  auto go = [&](auto kern) {
-    // The cluster size: from the smallest that holds a slice, doubled (up to
-    // 8, with at least 32 rows per CTA) while that lowers waves x bytes per
-    // CTA, the time of a launch in which every slice costs one CTA's load
-    // and write of its share.  E.g. 16 slices of fp32 512 x 384 take 16
-    // clusters of 4 (one wave of 198 KB per CTA), not 16 clusters of 8,
-    // which would need two waves when 15 of them are resident.
-    SliceCfg c = c0;
-    auto cost = [&](const SliceCfg &x) -> double {
-      int res = 0;
-      if (x.K > 1) {
-        if (prep_kernel(kern, x.smem, x.K)) return 1e30;
-        res = clusters_resident((const void *)kern, kSliceThreads, x.smem, x.K);
-      } else {
-        if (prep_kernel(kern, x.smem, 1)) return 1e30;
-        occupancy_cached((const void *)kern, kSliceThreads, x.smem, 1, &res);
-        res *= dev_info().sms;
-      }
-      if (res < 1) return 1e30;
-      return (double)((d3 + res - 1) / res) * (double)x.smem;
-    };
-    double best = cost(c);
-    for (int K = c0.K * 2; K <= 8 && m / K >= 32; K *= 2) {
-      SliceCfg x = c0;
-      x.K = K;
-      x.H = (uint32_t)(((m + K - 1) / K + 31) / 32 * 32);
-      x.smem = (int64_t)x.H * x.P;
-      const double cx = cost(x);
-      if (cx < best) {
-        best = cx;
-        c = x;
-      }
-    }
-    int64_t clusters = d3;
-    if (c.K > 1) {
-      const int res = clusters_resident((const void *)kern, kSliceThreads, c.smem, c.K);
-      if (res < 1) {
-        status = cuda_status(cudaErrorInvalidConfiguration, "slice cluster cannot be resident");
-        return;
-      }
-      clusters = std::min<int64_t>(d3, res);
-    } else {
-      int per_sm = 1;
-      occupancy_cached((const void *)kern, kSliceThreads, c.smem, 1, &per_sm);
-      clusters = std::min<int64_t>(d3, (int64_t)std::max(1, per_sm) * dev_info().sms);
-    }
-    status = launch_k(kern, clusters * c.K, kSliceThreads, c.smem, c.K, st, data, d3, (uint32_t)m, (uint32_t)n, c.H,
-                      c.P);
-    if (ls) ls->launches++;
-  };
-  // a cluster kernel when the smallest cluster that holds a slice has more
-  // than one CTA, else (one CTA per slice) the plain form
-  auto pick = [&](auto EBc) {
-    constexpr int EB = decltype(EBc)::value;
-    if (c0.vec) {
-      if (c0.K > 1 || m / 2 >= 32) go(k_slice<EB, true, true>);
-      else go(k_slice<EB, true, false>);
-    } else {
-      if (c0.K > 1 || m / 2 >= 32) go(k_slice<EB, false, true>);
-      else go(k_slice<EB, false, false>);
-    }
-  };
-  switch (eb) {
-    case 1: pick(IC<1>{}); break;
-    case 2: pick(IC<2>{}); break;
-    case 4: pick(IC<4>{}); break;
-    case 8: pick(IC<8>{}); break;
-    case 16: pick(IC<16>{}); break;
-    default:
-      set_error("unsupported element size");
-      return T213_ERR_UNSUPPORTED;
-  }
-  return status;
 }
 
 }  // namespace t213

@@ -1,0 +1,425 @@
+// Geometry and launch of the one-pass slice kernel (k_hold.cuh).
+#include <algorithm>
+#include <atomic>
+#include <cstdio>
+#include <cstdlib>
+#include <map>
+#include <thread>
+#include <tuple>
+#include <vector>
+
+#include "internal.h"
+#include "k_hold.cuh"
+
+namespace t213 {
+
+struct HoldReady {
+  std::mutex mu;
+  struct Form {
+    std::atomic<bool> ready{false};
+    HoldArgs args{};
+    const void *kern = nullptr;
+    int64_t smem = 0;
+    int resident = 1;  // teams resident at once
+    uint32_t *bars = nullptr;
+    int *status = nullptr;
+  } any, vec;
+};
+
+namespace {
+
+__device__ uint32_t g_hold_bars[(size_t)kHoldSlots * kHoldTeams * 8];
+
+// Shared memory of one CTA when two are resident on an SM.
+int64_t hold_budget() {
+  const DevInfo &d = dev_info();
+  const int64_t half = d.smem_per_sm / 2 - 1024 - 320;  // 1 KB reserved per CTA, the barrier flag, rounding
+  return std::min<int64_t>(half, d.smem_optin - 64) / 128 * 128;
+}
+
+int64_t up(int64_t x, int64_t u) { return (x + u - 1) / u * u; }
+
+// Row pitch in shared memory (see the layout in k_hold.cuh): an odd number of
+// 16-byte blocks; whole 128-byte groups for the swizzled vector form.
+int64_t hold_pitch(int64_t tn, int eb, int64_t we, int form) {
+  if (form == HOLD_VEC) return up(tn * eb, 128);
+  if (form == HOLD_WIDE) return ((tn * we) | 1) * 16;
+  if (eb == 16) return (tn | 1) * 16;
+  return (((tn * eb + 15 - eb) / 16 + 1) | 1) * 16;  // the blocks that cover a piece at any offset
+}
+
+// Bytes of one region of a tile (the tile itself unless the elements are
+// smaller than 4 bytes).
+int64_t hold_region(int64_t tm, int64_t P, int eb, int form) {
+  if (form != HOLD_SCALAR) return tm * P;
+  const int64_t N = eb < 4 ? 4 / eb : 1, l = (tm + N - 1) / N;
+  return l * P + l / 8 * 16;
+}
+
+int64_t hold_tile_bytes(int64_t tm, int64_t tn, int64_t P, int eb, int form, bool packed) {
+  if (packed) return up(tm * tn * eb + 30, 128);
+  const int64_t N = form == HOLD_SCALAR && eb < 4 ? 4 / eb : 1;
+  return up(N * hold_region(tm, P, eb, form), 128);
+}
+
+// Narrow rows whose whole width is in the tile are kept packed: nothing is
+// lost to the 16-byte blocks of every row, and at strides with few common
+// factors with the 32 banks a column costs few conflicts.
+bool hold_packed(int64_t n, int eb, int form) {
+  if (form != HOLD_SCALAR || n * eb > 256) return false;
+  const int64_t stride = eb < 4 ? n : n * eb / 4;  // words from lane to lane
+  int64_t g = 1;
+  while (g < 32 && stride % (g * 2) == 0) g *= 2;
+  return n * eb < 32 || g <= std::max(1, eb / 4) * 2;
+}
+
+int lanes_log2(int64_t x) {
+  int l = 0;
+  while (l < 5 && (1 << l) < x) l++;
+  return l;
+}
+
+// The tiling of m x n slices of eb-byte elements (we 16-byte words each in the
+// wide form): tile sides, team size and mode with the smallest modelled time.
+//
+// Model (B200): an SM moves its CTAs' shares at most at 60 GB/s and all SMs
+// together at 6.4 TB/s; a slice costs a load and a store latency of
+// 1 us each and a barrier with its costlier launch (cluster 1.2 us, grid 2.5 us);
+// a slice of one CTA waits for no other; short row pieces cost
+// a 32-byte sector more per piece.
+bool hold_search(HoldGeom &g, int64_t m, int64_t n, int eb, int64_t we, int64_t d3, int form) {
+  const DevInfo &d = dev_info();
+  const int64_t E = eb * we;
+  const int64_t budget = hold_budget();
+  const int64_t slots = 2ll * d.sms;
+  const int64_t Q = form == HOLD_VEC ? 16 / eb : 1;
+  // tile sides in whole 32-byte sectors where the rows are
+  const int64_t un = std::max<int64_t>(Q, (n * E) % 32 == 0 && E < 32 ? 32 / E : 1);
+  const int64_t um = std::max<int64_t>(Q, (m * E) % 32 == 0 && E < 32 ? 32 / E : 1);
+  double best = 1e30;
+  g.ok = false;
+  for (int S = 1; S <= 2; S++) {
+    const int64_t tile_cap = budget / S;
+    const int64_t max_tiles = slots * S;
+    for (int64_t TC = 1; TC <= std::min<int64_t>(max_tiles, n); TC = TC < 48 ? TC + 1 : TC + TC / 16) {
+      const int64_t tn = std::min(n, up((n + TC - 1) / TC, un));
+      const int64_t tcs = (n + tn - 1) / tn;
+      const bool packed = tcs == 1 && hold_packed(n, eb, form);
+      const int64_t P = packed ? n * eb : hold_pitch(tn, eb, we, form);
+      auto fits = [&](int64_t tm) { return hold_tile_bytes(tm, tn, P, eb, form, packed) <= tile_cap; };
+      if (!fits(1)) continue;
+      int64_t tm_max = std::max<int64_t>(1, tile_cap / P);
+      if (tm_max > um) tm_max = tm_max / um * um;
+      while (tm_max > 1 && !fits(tm_max)) tm_max -= tm_max > 2 * um ? um : 1;
+      tm_max = tm_max / Q * Q;
+      if (tm_max < 1) continue;
+      tm_max = std::min(tm_max, m);
+      const int64_t trmin = (m + tm_max - 1) / tm_max;
+      for (int64_t tr = trmin; tr <= m; tr += tr < trmin + 6 ? 1 : std::max<int64_t>(1, tr / 4)) {
+        int64_t tm = std::min(m, up((m + tr - 1) / tr, um));
+        if (tm > tm_max) tm = tm_max;
+        const int64_t trs = (m + tm - 1) / tm;
+        const int64_t T = trs * tcs;
+        if (T > max_tiles) break;
+        const int64_t ctas = (T + S - 1) / S;
+        const int mode = ctas == 1 ? HOLD_CTA : ctas <= 16 ? HOLD_CLUSTER : HOLD_GRID;
+        if (S > 1 && mode != HOLD_GRID) continue;
+        const int64_t teams = std::min<int64_t>(d3, slots / ctas);
+        if (mode == HOLD_GRID && teams > kHoldTeams) continue;
+        const int64_t waves = (d3 + teams - 1) / teams;
+        const int64_t conc = teams * ctas, per_sm = (conc + d.sms - 1) / d.sms;
+        const double bw = std::min(60e9, 6.4e12 / (double)std::min<int64_t>(conc, d.sms)) / (double)per_sm;
+        const double share = (double)S * tm * tn * E;
+        // lanes left idle by tiles of a few rows more than a multiple of 32
+        const int64_t N = eb < 4 ? 4 / eb : 1, wd = form == HOLD_SCALAR ? (tm + N - 1) / N : 32;
+        const double idle = wd >= 32 ? 0.5 * (double)(up(wd, 32) - wd) / (double)wd : 0.0;
+        const double ineff = idle + 2.0 + 32.0 / (double)(tn * E) + 32.0 / (double)(tm * E);
+        const double bar = mode == HOLD_CTA ? 0.2e-6 : mode == HOLD_CLUSTER ? 1.2e-6 : 2.5e-6;
+        const double lat = waves > 1 && S > 1 ? 1.5e-6 : 2e-6;
+        const double t = waves * (lat + bar + share * ineff / bw);
+        if (t < best * 0.999) {
+          best = t;
+          g.ok = true;
+          g.tm = (uint32_t)tm;
+          g.tn = (uint32_t)tn;
+          g.TC = (uint32_t)tcs;
+          g.T = (uint32_t)T;
+          g.ctas = (uint32_t)ctas;
+          g.teams = (uint32_t)teams;
+          g.S = (uint32_t)S;
+          g.P = (uint32_t)P;
+          g.packed = packed;
+          g.mode = mode;
+          g.form = form;
+          g.est_us = t * 1e6;
+        }
+      }
+    }
+  }
+  return g.ok;
+}
+
+// Barrier slots of grid launches.  Launches on one stream run one after the
+// other and share a slot.  A captured launch may be replayed on any stream and
+// gets a slot of its own, given back when the graph and everything
+// instantiated from it are gone.
+struct HoldSlots {
+  std::mutex mu;
+  std::map<std::tuple<cudaStream_t, std::thread::id>, int> of_stream;
+  std::vector<int> free_list;
+  int next = 0;
+  int take() {
+    if (!free_list.empty()) {
+      const int s = free_list.back();
+      free_list.pop_back();
+      return s;
+    }
+    return next < kHoldSlots ? next++ : -1;
+  }
+};
+
+HoldSlots &hold_slots(int dev) {
+  static std::mutex mu;
+  static auto &all = *new std::map<int, HoldSlots>;  // never destroyed: graphs may outlive statics
+  std::lock_guard<std::mutex> lk(mu);
+  return all[dev];
+}
+
+struct HoldSlotLease {
+  int dev, slot;
+};
+
+void CUDART_CB hold_slot_return(void *p) {
+  auto *l = (HoldSlotLease *)p;
+  HoldSlots &hs = hold_slots(l->dev);
+  {
+    std::lock_guard<std::mutex> lk(hs.mu);
+    hs.free_list.push_back(l->slot);
+  }
+  delete l;
+}
+
+// -1 when no slot is left.
+int hold_slot(cudaStream_t st) {
+  const int dev = dev_info().id;
+  HoldSlots &hs = hold_slots(dev);
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  cudaGraph_t graph = nullptr;
+  if (cudaStreamGetCaptureInfo_v2(st, &cs, nullptr, &graph, nullptr, nullptr) != cudaSuccess) {
+    cudaGetLastError();
+    return -1;
+  }
+  if (cs == cudaStreamCaptureStatusActive) {
+    int slot;
+    {
+      std::lock_guard<std::mutex> lk(hs.mu);
+      slot = hs.take();
+    }
+    if (slot < 0) return -1;
+    auto *l = new HoldSlotLease{dev, slot};
+    cudaUserObject_t obj = nullptr;
+    if (cudaUserObjectCreate(&obj, l, hold_slot_return, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+      cudaGetLastError();
+      hold_slot_return(l);
+      return -1;
+    }
+    if (cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+      cudaGetLastError();
+      cudaUserObjectRelease(obj, 1);  // runs hold_slot_return
+      return -1;
+    }
+    return slot;
+  }
+  std::lock_guard<std::mutex> lk(hs.mu);
+  // the per-thread default stream is one handle for a stream of every thread
+  const auto key = std::make_tuple(st, st == cudaStreamPerThread ? std::this_thread::get_id() : std::thread::id());
+  auto it = hs.of_stream.find(key);
+  if (it != hs.of_stream.end()) return it->second;
+  const int slot = hs.take();
+  if (slot >= 0) hs.of_stream[key] = slot;
+  return slot;
+}
+
+uint32_t *hold_bars(int *status) {
+  static std::mutex mu;
+  static std::map<int, uint32_t *> ptr;
+  const int dev = dev_info().id;
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = ptr.find(dev);
+  if (it != ptr.end()) return it->second;
+  void *p = nullptr;
+  cudaError_t e = cudaGetSymbolAddress(&p, g_hold_bars);
+  if (e != cudaSuccess) {
+    *status = cuda_status(e, "slice barrier words");
+    return nullptr;
+  }
+  return ptr[dev] = (uint32_t *)p;
+}
+
+}  // namespace
+
+void hold_plan(HoldPlan &hp, int64_t m, int64_t n, int eb, int64_t we, int64_t d3) {
+  hp.ready = std::make_shared<HoldReady>();
+  if (we > 1) {
+    hold_search(hp.any, m, n, 16, we, d3, HOLD_WIDE);
+    return;
+  }
+  hold_search(hp.any, m, n, eb, 1, d3, HOLD_SCALAR);
+  if ((eb == 2 || eb == 4) && (n * eb) % 16 == 0 && (m * eb) % 16 == 0)
+    hold_search(hp.vec, m, n, eb, 1, d3, HOLD_VEC);
+}
+
+bool slice_fits(int64_t m, int64_t n, int eb) {
+  HoldGeom g;
+  return hold_search(g, m, n, eb, 1, 1, HOLD_SCALAR);
+}
+
+std::string describe_slice(const HoldPlan &hp) {
+  const HoldGeom &g = hp.vec.ok ? hp.vec : hp.any;
+  char buf[160];
+  snprintf(buf, sizeof buf, "slice(%s tiles=%u of %ux%u per cta=%u ctas=%u teams=%u%s)",
+           g.mode == HOLD_CTA ? "cta" : g.mode == HOLD_CLUSTER ? "cluster" : "grid", g.T, g.tm, g.tn, g.S, g.ctas,
+           g.teams, g.form == HOLD_VEC ? " vec" : "");
+  return buf;
+}
+
+namespace {
+
+int hold_prepare(HoldReady::Form &f, const HoldGeom &g, int64_t m, int64_t n, int eb, int64_t we) {
+  int status = T213_OK;
+  f.status = device_status_word(&status);
+  if (!f.status) return status;
+  HoldArgs &a = f.args;
+  a.slice_bytes = m * n * eb * we;
+  a.m = (uint32_t)m;
+  a.n = (uint32_t)n;
+  a.tm = g.tm;
+  a.tn = g.tn;
+  a.TC = g.TC;
+  a.T = g.T;
+  a.ctas = g.ctas;
+  a.teams = g.teams;
+  a.S = g.S;
+  a.P = g.P;
+  a.H = (uint32_t)hold_region(g.tm, g.P, eb, g.form);
+  a.packed = g.packed;
+  a.tile_bytes = (uint32_t)hold_tile_bytes(g.tm, g.tn, g.P, eb, g.form, g.packed);
+  a.mode = g.mode;
+  a.we = (uint32_t)we;
+  a.wediv = FastDiv<uint32_t>((uint64_t)we);
+  a.tcdiv = FastDiv<uint32_t>(g.TC);
+  if (g.form == HOLD_VEC) {
+    a.rbdiv = FastDiv<uint32_t>((uint64_t)(g.tm / (16 / eb) + 7) / 8);
+  } else if (g.form == HOLD_WIDE) {
+    a.lgs = lanes_log2(g.tm * we);
+  } else {
+    const int N = eb < 4 ? 4 / eb : 1;
+    const int64_t words = N == 1 ? g.tm : ((int64_t)g.tm + 2 * N - 2) / N;
+    a.lgs = lanes_log2(words);
+    a.rbdiv = FastDiv<uint32_t>((uint64_t)(words + (1 << a.lgs) - 1) >> a.lgs);
+  }
+  f.smem = (int64_t)g.S * a.tile_bytes;
+  switch (g.form == HOLD_WIDE ? 0 : g.form == HOLD_VEC ? -eb : eb) {
+    case 0:
+      f.kern = (const void *)k_hold<16, HOLD_WIDE>;
+      break;
+    case -2:
+      f.kern = (const void *)k_hold<2, HOLD_VEC>;
+      break;
+    case -4:
+      f.kern = (const void *)k_hold<4, HOLD_VEC>;
+      break;
+    case 1:
+      f.kern = (const void *)k_hold<1, HOLD_SCALAR>;
+      break;
+    case 2:
+      f.kern = (const void *)k_hold<2, HOLD_SCALAR>;
+      break;
+    case 4:
+      f.kern = (const void *)k_hold<4, HOLD_SCALAR>;
+      break;
+    case 8:
+      f.kern = (const void *)k_hold<8, HOLD_SCALAR>;
+      break;
+    case 16:
+      f.kern = (const void *)k_hold<16, HOLD_SCALAR>;
+      break;
+    default:
+      set_error("unsupported element size");
+      return T213_ERR_UNSUPPORTED;
+  }
+  if (!kernel_attr_once(f.kern, f.smem, g.mode == HOLD_CLUSTER ? (int)g.ctas : 1))
+    return cuda_status(cudaGetLastError(), "cudaFuncSetAttribute(slice)");
+  if (g.mode == HOLD_GRID) {
+    f.bars = hold_bars(&status);
+    if (!f.bars) return status;
+    f.resident = (int)g.teams;
+  } else {
+    occupancy_cached(f.kern, kHoldThreads, f.smem, (int)g.ctas, &f.resident);
+    if (g.mode == HOLD_CTA) f.resident *= dev_info().sms;
+    f.resident = std::max(1, f.resident);
+  }
+  return T213_OK;
+}
+
+}  // namespace
+
+int launch_slice(const HoldPlan &hp, char *data, int64_t d3, int64_t m, int64_t n, int eb, int64_t we,
+                 cudaStream_t st, LaunchStats *ls) {
+  if (d3 <= 0 || m <= 0 || n <= 0) return T213_OK;
+  const bool vec = hp.vec.ok && (uintptr_t)data % 16 == 0;
+  const HoldGeom &g = vec ? hp.vec : hp.any;
+  if (!g.ok) {
+    set_error("slice does not fit the chip's shared memory");
+    return T213_ERR_UNSUPPORTED;
+  }
+  HoldReady::Form &f = vec ? hp.ready->vec : hp.ready->any;
+  if (!f.ready.load(std::memory_order_acquire)) {
+    std::lock_guard<std::mutex> lk(hp.ready->mu);
+    if (!f.ready.load(std::memory_order_relaxed)) {
+      const int rc = hold_prepare(f, g, m, n, eb, we);
+      if (rc) return rc;
+      f.ready.store(true, std::memory_order_release);
+    }
+  }
+  HoldArgs a = f.args;
+  a.d3 = d3;
+  // persistent: as many teams as are resident at once
+  a.teams = (uint32_t)std::min<int64_t>(f.resident, d3);
+  if (g.mode == HOLD_GRID) {
+    a.slot = hold_slot(st);
+    if (a.slot < 0) return kHoldNoSlot;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(a.teams * a.ctas, 1, 1);
+  cfg.blockDim = dim3(kHoldThreads, 1, 1);
+  cfg.dynamicSmemBytes = (size_t)f.smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  if (g.mode == HOLD_CLUSTER) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = g.ctas;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.numAttrs = 1;
+  } else if (g.mode == HOLD_GRID) {
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.numAttrs = 1;
+  }
+  cfg.attrs = attr;
+  uint32_t *bars = f.bars;
+  int *status = f.status;
+  void *args[] = {&data, &a, &bars, &status};
+  const cudaError_t e = cfg.numAttrs ? cudaLaunchKernelExC(&cfg, f.kern, args)
+                                     : cudaLaunchKernel(f.kern, cfg.gridDim, cfg.blockDim, args, cfg.dynamicSmemBytes, st);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    cudaGetLastError();
+    return kHoldNoSlot;  // fewer SMs than the device reports (a partitioned GPU)
+  }
+  if (e != cudaSuccess) return cuda_status(e, "k_hold launch");
+  if (ls) ls->launches++;
+  return T213_OK;
+}
+
+}  // namespace t213

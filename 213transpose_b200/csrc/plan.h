@@ -20,6 +20,7 @@ struct PassDesc {
   std::shared_ptr<CycleTable> table;
   int64_t t = 0;                     // PT_TILE: block side
   int64_t R = 0, C = 0, bands = 0;   // PT_BAND: band shape, bands per slice
+  HoldPlan hold;                     // PT_SLICE: the tiling
   const char *name() const;
 };
 
@@ -34,6 +35,8 @@ struct Plan {
   Variant var;          // kernel choices pinned by the tuner (default: none)
 };
 
+// Internal kind: the automatic choice among the plans of two and more sweeps.
+constexpr int kPlanSweeps = -1;
 // Builds the plan of a family (T213_PLAN_*; AUTO picks).  t = 0 lets the
 // planner choose the block/band size.  Cached per device.
 std::shared_ptr<Plan> get_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int kind, int64_t t, int *status);

@@ -30,11 +30,15 @@ int cuda_status(cudaError_t e, const char *where) {
 const DevInfo &dev_info() {
   static std::mutex mu;
   static std::map<int, DevInfo> cache;
+  // asked several times by every call: the thread's last answer, which stays
+  // where it is in the map, needs no lock
+  thread_local const DevInfo *last = nullptr;
   int dev = 0;
   cudaGetDevice(&dev);
+  if (last && last->id == dev) return *last;
   std::lock_guard<std::mutex> lk(mu);
   auto it = cache.find(dev);
-  if (it != cache.end()) return it->second;
+  if (it != cache.end()) return *(last = &it->second);
   DevInfo d;
   d.id = dev;
   int v = 0;
@@ -81,6 +85,10 @@ char *workspace(cudaStream_t st, size_t bytes, int *status) {
   return p;
 }
 
+// A variable of the module rather than an allocation: it is zero from the
+// start, and a first call inside a stream capture may take its address.
+__device__ int g_status_word[64];
+
 int *device_status_word(int *status) {
   static std::mutex mu;
   static std::map<int, int *> words;
@@ -88,18 +96,13 @@ int *device_status_word(int *status) {
   std::lock_guard<std::mutex> lk(mu);
   auto it = words.find(dev);
   if (it != words.end()) return it->second;
-  int *p = nullptr;
-  cudaError_t e = cudaMalloc(&p, 256);
-  if (e == cudaSuccess) e = cudaMemset(p, 0, 256);
-  // the memset runs on the legacy stream, which kernels on non-blocking
-  // streams do not wait for: let it land before any pass can record a status
-  if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+  void *p = nullptr;
+  cudaError_t e = cudaGetSymbolAddress(&p, g_status_word);
   if (e != cudaSuccess) {
     *status = cuda_status(e, "status word");
     return nullptr;
   }
-  words[dev] = p;
-  return p;
+  return words[dev] = (int *)p;
 }
 
 void release_stream_workspace(cudaStream_t st) {
@@ -334,7 +337,7 @@ std::string fmt_plan(const Plan &P) {
         snprintf(buf, sizeof buf, "row_gather(fn=%d)%s", p.fn.kind, describe_row_gather(p.m, p.n, P.eb, nullptr).substr(10).c_str());
         break;
       case PT_SLICE:
-        snprintf(buf, sizeof buf, "%s", describe_slice(p.m, p.n, P.eb, P.d3).c_str());
+        snprintf(buf, sizeof buf, "%s", describe_slice(p.hold).c_str());
         break;
       case PT_SEG:
         snprintf(buf, sizeof buf, "segment_cycles(S=%lld seg=%lldB cycles=%lld chunks=%lld carry=%lld maxlen=%lld)",
@@ -526,14 +529,15 @@ int build_plan(Plan &P, int kind, int64_t t) {
       return add_seg_pass(P, ps, t * eb, true);
     }
     case T213_PLAN_SLICE: {
-      if (!slice_fits(m, n, eb)) {
-        set_error("slice plan needs a slice that fits a 16-CTA cluster's shared memory");
-        return T213_ERR_UNSUPPORTED;
-      }
       PassDesc sp;
       sp.type = PT_SLICE;
       sp.m = m;
       sp.n = n;
+      if (m >= 2 && n >= 2 && m <= (1 << 30) && n <= (1 << 30)) hold_plan(sp.hold, m, n, eb, 1, d3);
+      if (!sp.hold.any.ok) {
+        set_error("slice plan needs a slice that fits the chip's shared memory");
+        return T213_ERR_UNSUPPORTED;
+      }
       P.passes.push_back(sp);
       return T213_OK;
     }
@@ -707,7 +711,7 @@ std::shared_ptr<Plan> get_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int k
     }
   }
   std::shared_ptr<Plan> best;
-  if (kind != T213_PLAN_AUTO) {
+  if (kind != T213_PLAN_AUTO && kind != kPlanSweeps) {
     best = new_plan(d1, d2, d3, eb);
     int st = build_plan(*best, kind, t);
     if (st) {
@@ -734,17 +738,30 @@ std::shared_ptr<Plan> get_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int k
       cands.push_back({T213_PLAN_BANDS, tr, estimate_cost(T213_PLAN_BANDS, m, n, tr, eb, d3)});
       int64_t tc = pick_band_t_t(m, n, eb);
       cands.push_back({T213_PLAN_BANDS_T, tc, estimate_cost(T213_PLAN_BANDS_T, m, n, tc, eb, d3)});
-      // The one-pass cluster plan (T213_PLAN_SLICE) wins where launch latency
-      // dominates: small tensors whose rows are 16-byte multiples both ways.
-      // Measured on B200: fp32 (256, 128, 64) 0.0126 ms against 0.0190 for
-      // BLOCKS; fp32 (512, 384, 16) 0.0192 against 0.0244 (clusters of 4, one
-      // wave).  Its element-wise form (other alignments) won on fp64
-      // (45, 600, 2) (0.015 against 0.025 ms) but lost badly on 1-byte
-      // (1000, 999, 1) (0.26 against 0.15 ms).  So it is ranked for tensors
-      // up to 16 MB with aligned rows only, and is otherwise taken when
-      // forced or chosen by the tuner.
-      if (slice_fits(m, n, eb) && (n * eb) % 16 == 0 && (m * eb) % 16 == 0 && d1 * d2 * d3 * eb <= (16ll << 20))
-        cands.push_back({T213_PLAN_SLICE, 0, 1.0});
+      // The one-pass plan (T213_PLAN_SLICE) is the fastest wherever a slice
+      // fits the chip, but for two classes.  Square slices of whole tiles are
+      // one sweep of tile swaps without a barrier: 16-byte
+      // (1024, 1024, 4) 24.8 us against 31.1, fp32 (2048, 2048, 8) 51.2 against
+      // 58.2; at 8 MB and below they tie or lose.  A single small slice that needs a cooperative launch (more than
+      // 16 CTAs) and has a block or band plan with segments of 256 bytes or
+      // more keeps that plan up to 4 MB: such a launch starts only when the whole
+      // chip is free of other streams' kernels, for a gain of a few us.
+      if (kind == T213_PLAN_AUTO) {
+        auto P = new_plan(d1, d2, d3, eb);
+        if (build_plan(*P, T213_PLAN_SLICE, 0) == T213_OK) {
+          const HoldPlan &hp = P->passes[0].hold;
+          const bool coop = hp.any.mode == HOLD_GRID;
+          const double total = (double)d1 * d2 * d3 * eb;
+          bool seg = false;
+          for (const Cand &c : cands) seg = seg || (eb >= 4 && c.est < 1e8 && c.t * eb >= 256 && c.t * eb % 16 == 0);
+          const bool square = m == n && tb == m && tile_eff(tb, eb) >= 0.9 && total > (8 << 20);
+          if (!square && !(coop && seg && total <= (4 << 20))) {
+            P->est_cost = plan_cost(*P);
+            best = P;
+          }
+        }
+      }
+      if (!best) {
       // The Catanzaro decomposition both ways: the reference's dispatcher
       // takes C2R when d1 >= d2, else R2C (src/transpose.cu:117-123); here
       // both are costed, since which one keeps its rows inside shared
@@ -769,6 +786,7 @@ std::shared_ptr<Plan> get_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int k
           best = P;
           break;
         }
+      }
       }
       if (!best) {
         *status = T213_ERR_UNSUPPORTED;
@@ -867,7 +885,12 @@ int run_plan(const Plan &P, char *data, cudaStream_t st, LaunchStats *ls) {
           rc = launch_seg_cycles(*p.table, gd, g, slice_bytes, p.seg_bytes, st, ls, nullptr, 0);
           break;
         case PT_SLICE:
-          rc = launch_slice(gd, g, p.m, p.n, P.eb, st, ls);
+          rc = launch_slice(p.hold, gd, g, p.m, p.n, P.eb, 1, st, ls);
+          if (rc == kHoldNoSlot) {
+            // the slices' CTAs cannot all be resident here: another plan
+            auto alt = get_plan(P.d1, P.d2, g, P.eb, kPlanSweeps, 0, &rc);
+            if (alt) rc = run_plan(*alt, gd, st, ls);
+          }
           break;
       }
       if (rc) return rc;

@@ -8,6 +8,7 @@
 // and the variants, and the planner re-derives the block or band size for
 // each concrete shape.  The cache persists as a text file, one entry per line.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <map>
@@ -45,12 +46,14 @@ ClassKey class_of(int64_t d1, int64_t d2, int64_t d3, int eb) {
 }
 
 std::mutex g_mu;
+std::atomic<bool> g_empty{true};  // nothing tuned or loaded: the automatic choice need not look
 std::map<ClassKey, Entry> g_cache;                                     // per shape class
 std::map<std::tuple<int64_t, int64_t, int64_t, int>, Entry> g_exact;  // per exact shape, wins
 
 }  // namespace
 
 int tuner_lookup_internal(int64_t d1, int64_t d2, int64_t d3, int eb, int *kind, int64_t *t, Variant *v) {
+  if (g_empty.load(std::memory_order_acquire)) return T213_ERR_NOT_READY;
   std::lock_guard<std::mutex> lk(g_mu);
   auto ex = g_exact.find(std::make_tuple(d1, d2, d3, eb));
   if (ex != g_exact.end()) {
@@ -83,6 +86,7 @@ int t213_tuner_lookup(int64_t d1, int64_t d2, int64_t d3, int32_t elem_bytes, in
 
 int t213_tuner_clear(void) {
   std::lock_guard<std::mutex> lk(g_mu);
+  g_empty.store(true, std::memory_order_release);
   g_cache.clear();
   g_exact.clear();
   return T213_OK;
@@ -126,14 +130,17 @@ int t213_tuner_load(const char *path) {
     // older files have no variant (and no block size on shape lines)
     const int nc = sscanf(line, "class %d %d %d %d %d %d %d", &k.eb, &k.l1, &k.l2, &k.l3, &k.lg, &kind, &var);
     if (nc >= 6 && kind >= T213_PLAN_AUTO && kind <= T213_PLAN_SLICE) {
+      g_empty.store(false, std::memory_order_release);
       g_cache[k] = Entry{kind, 0, nc == 7 ? var : 0};
       continue;
     }
     var = 0;
     const int ns = sscanf(line, "shape %lld %lld %lld %d %d %lld %d", &a, &b, &c, &eb, &kind, &t, &var);
-    if (ns >= 5 && kind >= T213_PLAN_AUTO && kind <= T213_PLAN_SLICE)
+    if (ns >= 5 && kind >= T213_PLAN_AUTO && kind <= T213_PLAN_SLICE) {
+      g_empty.store(false, std::memory_order_release);
       g_exact[std::make_tuple((int64_t)a, (int64_t)b, (int64_t)c, eb)] =
           Entry{kind, ns >= 6 ? (int64_t)t : 0, ns == 7 ? var : 0};
+    }
   }
   fclose(f);
   return T213_OK;
@@ -235,6 +242,7 @@ int t213_tune_shape(void *scratch_data, int64_t d1, int64_t d2, int64_t d3, int3
   if (e != cudaSuccess) return cuda_status(e, "tuning");
   {
     std::lock_guard<std::mutex> lk(g_mu);
+    g_empty.store(false, std::memory_order_release);
     g_cache[class_of(d1, d2, d3, elem_bytes)] = Entry{best.kind, 0, best.var};
     g_exact[std::make_tuple(d1, d2, d3, (int)elem_bytes)] = best;
   }
