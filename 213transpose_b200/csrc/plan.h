@@ -37,6 +37,11 @@ struct Plan {
 
 // Internal kind: the automatic choice among the plans of two and more sweeps.
 constexpr int kPlanSweeps = -1;
+// Internal kinds kPlanOnePassOr - family: the one-pass plan where it applies,
+// else the named family.
+constexpr int kPlanOnePassOr = -16;
+// Internal kind: the one-pass plan of elements of eb = a multiple of 16 bytes.
+constexpr int kPlanWideSlice = -2;
 // Builds the plan of a family (T213_PLAN_*; AUTO picks).  t = 0 lets the
 // planner choose the block/band size.  Cached per device.
 std::shared_ptr<Plan> get_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int kind, int64_t t, int *status);
@@ -51,10 +56,6 @@ int run_plan(const Plan &p, char *data, cudaStream_t st, LaunchStats *ls);
 // Extra device memory a run of the plan needs beyond the tensor (carries and
 // scratch fallbacks), in bytes.
 size_t plan_workspace_bytes(const Plan &p);
-
-// Explicit C2R / R2C / skinny plans with the reference's argument convention.
-std::shared_ptr<Plan> make_c2r_plan(int64_t d1, int64_t d2, int64_t d3, int eb, bool skinny, int *status);
-std::shared_ptr<Plan> make_r2c_plan(int64_t d1, int64_t d2, int64_t d3, int eb, bool skinny, int *status);
 
 int64_t ext_gcd(int64_t a, int64_t b, int64_t *mmi);
 

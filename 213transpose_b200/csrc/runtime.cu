@@ -711,9 +711,26 @@ std::shared_ptr<Plan> get_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int k
     }
   }
   std::shared_ptr<Plan> best;
-  if (kind != T213_PLAN_AUTO && kind != kPlanSweeps) {
+  if (kind == kPlanWideSlice) {
+    // no passes: a slice of these elements does not fit the chip
     best = new_plan(d1, d2, d3, eb);
-    int st = build_plan(*best, kind, t);
+    best->kind = T213_PLAN_SLICE;
+    PassDesc sp;
+    sp.type = PT_SLICE;
+    sp.m = d2;
+    sp.n = d1;
+    if (d1 * d2 * eb < (64 << 20)) hold_plan(sp.hold, d2, d1, 16, eb / 16, d3);
+    if (sp.hold.any.ok) best->passes.push_back(sp);
+  } else if (kind != T213_PLAN_AUTO && kind != kPlanSweeps) {
+    best = new_plan(d1, d2, d3, eb);
+    int st = T213_ERR_UNSUPPORTED;
+    if (kind <= kPlanOnePassOr) {
+      if (d1 == 1 || d2 == 1)
+        st = build_plan(*best, T213_PLAN_IDENTITY, 0);
+      else if (d1 * d2 * eb < (64 << 20))  // above the shared memory of any chip
+        st = build_plan(*best, T213_PLAN_SLICE, 0);
+    }
+    if (st) st = build_plan(*best, kind <= kPlanOnePassOr ? kPlanOnePassOr - kind : kind, t);
     if (st) {
       *status = st;
       return nullptr;
@@ -809,24 +826,6 @@ std::shared_ptr<Plan> get_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int k
     }
   }
   return best;
-}
-
-std::shared_ptr<Plan> make_c2r_plan(int64_t d1, int64_t d2, int64_t d3, int eb, bool skinny, int *status) {
-  *status = T213_OK;
-  auto P = new_plan(d1, d2, d3, eb);
-  P->kind = skinny ? T213_PLAN_SKINNY : T213_PLAN_C2R;
-  c2r_passes(*P, d2, d1, skinny);
-  P->desc = fmt_plan(*P);
-  return P;
-}
-
-std::shared_ptr<Plan> make_r2c_plan(int64_t d1, int64_t d2, int64_t d3, int eb, bool skinny, int *status) {
-  *status = T213_OK;
-  auto P = new_plan(d1, d2, d3, eb);
-  P->kind = skinny ? T213_PLAN_SKINNY : T213_PLAN_R2C;
-  r2c_passes(*P, d2, d1, skinny);
-  P->desc = fmt_plan(*P);
-  return P;
 }
 
 size_t plan_workspace_bytes(const Plan &p) {
@@ -958,31 +957,20 @@ int run_shape(void *data, int64_t d1, int64_t d2, int64_t d3, int32_t eb, int ki
   rc = prefetch_if_managed(data, (size_t)(d1 * d2 * d3 * eb), st);
   if (rc) return rc;
   std::shared_ptr<Plan> P;
-  switch (which) {
-    case 0:
-      P = get_plan(d1, d2, d3, eb, kind, t, &rc);
-      break;
-    case 1:
-      P = make_c2r_plan(d1, d2, d3, eb, false, &rc);
-      break;
-    case 2:
-      P = make_r2c_plan(d1, d2, d3, eb, false, &rc);
-      break;
-    case 3:
-      if (d2 > 32) {
-        set_error("skinny C2R needs d2 <= 32");
-        return T213_ERR_INVALID_ARGUMENT;
-      }
-      P = make_c2r_plan(d1, d2, d3, eb, true, &rc);
-      break;
-    case 4:
-      if (d2 > 32) {
-        set_error("skinny R2C needs d2 <= 32");
-        return T213_ERR_INVALID_ARGUMENT;
-      }
-      P = make_r2c_plan(d1, d2, d3, eb, true, &rc);
-      break;
+  // The decomposition's entry points are transposes too: C2R and skinny C2R
+  // of (d1, d2), R2C and skinny R2C of the shape they make, (d2, d1).  They
+  // take the one-pass plan where a slice fits the chip (fp32 r2c to
+  // (2000, 3001, 4): 78 us by its gathers, 52 us in one pass), else their own
+  // passes, from the plan cache (building them cost 20 us a call).
+  if ((which == 3 || which == 4) && d2 > 32) {
+    set_error(which == 3 ? "skinny C2R needs d2 <= 32" : "skinny R2C needs d2 <= 32");
+    return T213_ERR_INVALID_ARGUMENT;
   }
+  if (which == 2 || which == 4) std::swap(d1, d2);
+  if (which == 1) kind = kPlanOnePassOr - T213_PLAN_C2R;
+  if (which == 2) kind = kPlanOnePassOr - T213_PLAN_R2C;
+  if (which >= 3) kind = kPlanOnePassOr - T213_PLAN_SKINNY;
+  P = get_plan(d1, d2, d3, eb, kind, t, &rc);
   if (!P) return rc ? rc : T213_ERR_UNSUPPORTED;
   return run_plan(*P, (char *)data, st, nullptr);
 }
@@ -1183,7 +1171,27 @@ int t213_permute(void *data, int32_t rank, const int64_t *dims, const int32_t *p
     } else if (g1 == 1 || g2 == 1) {
       rc = T213_OK;  // the memory layout does not change
     } else {
-      // segments of E bytes: [g2][g1] -> [g1][g2] in each of the g3 slices
+      // segments of E bytes: [g2][g1] -> [g1][g2] in each of the g3 slices.
+      // Below 512 bytes in the one-pass form where a slice fits the chip,
+      // from there on by the cycle walkers, whose bulk copies then reach 5
+      // TB/s (B200, one-pass against cycles, us): 64 B (512, 64, 32) 26 / 225,
+      // 128 B (64, 512, 16) 29 / 133, 256 B (8, 2048, 32) 60 / 84, 512 B
+      // (4, 2048, 16) 31 / 27, 1 KB (4, 2048, 16) 61 / 53.
+      rc = kHoldNoSlot;
+      if (E % 16 == 0 && E < 512 && (uintptr_t)data % 16 == 0) {
+        auto P = get_plan(g1, g2, g3, (int)E, kPlanWideSlice, 0, &rc);
+        if (!P) return rc;
+        rc = kHoldNoSlot;
+        if (!P->passes.empty()) {
+          PassTimer tm("slice", (cudaStream_t)stream);
+          rc = launch_slice(P->passes[0].hold, (char *)data, g3, g2, g1, 16, E / 16, (cudaStream_t)stream, nullptr);
+        }
+      }
+      if (rc != kHoldNoSlot) {
+        if (rc) return rc;
+        std::rotate(cur.begin() + q0, cur.begin() + p + 1, cur.begin() + k + 1);
+        continue;
+      }
       PermSpec ps;
       ps.kind = 0;
       ps.A = g2;

@@ -91,3 +91,36 @@ def test_captured_launches_and_streams(cuda, oracle, t213):
         assert np.array_equal(from_device(d), w)
     assert t213.device_status() == 0
     del g
+
+
+@pytest.mark.parametrize("shape", [(3001, 4000, 1, 4), (1000, 999, 2, 8), (9001, 30, 3, 4), (500001, 30, 1, 4)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_named_directions(cuda, oracle, t213, shape):
+    """The decomposition's entry points over slices that fit the chip and
+    slices that do not (those run the named passes)."""
+    d1, d2, d3, eb = shape
+    x = oracle.random_bits(d1 * d2 * d3, eb, d1)
+    want = oracle.gather213(x.view(np.dtype((np.void, eb))), d1, d2, d3).view(np.uint8)
+    calls = [lambda v: t213.c2r_transpose(v, d1, d2, d3, elem_bytes=eb),
+             lambda v: t213.r2c_transpose(v, d2, d1, d3, elem_bytes=eb)]
+    if d2 <= 32:
+        calls.append(lambda v: t213.skinny_c2r_transpose(v, d1, d2, d3, elem_bytes=eb))
+    for call in calls:
+        dev = to_device(cuda, x)
+        call(dev)
+        cuda.cuda.synchronize()
+        assert np.array_equal(from_device(dev), want)
+
+
+@pytest.mark.parametrize("e", (80, 256, 496))
+@pytest.mark.parametrize("dims", [(13, 1000, 2), (300, 7, 5), (33, 31, 40), (600, 80, 2)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_wide_elements(cuda, t213, dims, e):
+    """Merged leading axes of a rank-N permutation as elements of several
+    16-byte words."""
+    h, s, b = dims
+    g = cuda.Generator(device="cuda").manual_seed(e + h)
+    x = cuda.empty(b * s * h * e, dtype=cuda.uint8, device="cuda").random_(0, 256, generator=g)
+    want = x.view(b, s, h, e).permute(0, 2, 1, 3).contiguous().view(-1)
+    t213.permute(x, [e, h, s, b], [0, 2, 1, 3], elem_bytes=1)
+    assert cuda.equal(x, want)
