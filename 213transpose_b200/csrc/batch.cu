@@ -179,7 +179,8 @@ bool plan_fits_batch(const Plan &p) {
       case PT_BAND:
         if (q.R * q.C * p.eb > kBatchHalf) return false;
         break;
-      case PT_SLICE:  // a cluster launch of its own; no executor in the persistent kernel
+      case PT_SLICE:  // launches of their own; no executor in the persistent kernel
+      case PT_RAGGED:
         return false;
       default:
         break;
@@ -411,11 +412,11 @@ namespace t213 {
 std::shared_ptr<Plan> group_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int *status, bool search_slice) {
   std::shared_ptr<Plan> P = get_plan(d1, d2, d3, eb, T213_PLAN_AUTO, 0, status);
   if (!P) return nullptr;
-  if (P->kind == T213_PLAN_SLICE) {
+  if (P->kind == T213_PLAN_SLICE || P->kind == kPlanRagged) {
     // A caller that plans as requests arrive leaves the tensors whose one-pass
     // form is the aligned one, which run best on their own launch; the others
     // take their best plan of two sweeps or more.
-    const bool aligned = (d1 * eb) % 16 == 0 && (d2 * eb) % 16 == 0 && d1 * d2 * d3 * eb <= (16ll << 20);
+    const bool aligned = P->kind == T213_PLAN_SLICE && (d1 * eb) % 16 == 0 && (d2 * eb) % 16 == 0 && d1 * d2 * d3 * eb <= (16ll << 20);
     if (aligned && !search_slice) return nullptr;
     P = get_plan(d1, d2, d3, eb, kPlanSweeps, 0, status);
     if (!P) return nullptr;

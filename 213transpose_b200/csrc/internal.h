@@ -40,6 +40,8 @@ int *device_status_word(int *status);
 // Grow-only scratch buffer per (device, stream).  Calls on one stream run in
 // order, so they can share it; calls on different streams never do.
 char *workspace(cudaStream_t st, size_t bytes, int *status);
+// Whether the stream's workspace already holds this many bytes.
+bool workspace_ready(cudaStream_t st, size_t bytes);
 // Frees the workspace of one stream (before the stream is destroyed).
 void release_stream_workspace(cudaStream_t st);
 
@@ -185,7 +187,7 @@ void hold_plan(HoldPlan &hp, int64_t m, int64_t n, int eb, int64_t we, int64_t d
 constexpr int kHoldNoSlot = -2;
 int launch_slice(const HoldPlan &hp, char *data, int64_t d3, int64_t m, int64_t n, int eb, int64_t we,
                  cudaStream_t st, LaunchStats *ls);
-bool slice_fits(int64_t m, int64_t n, int eb);
+int64_t hold_cluster_bytes();  // shared memory of the largest team that needs no cooperative launch
 std::string describe_slice(const HoldPlan &hp);
 // Grouped one-pass slices (the batched form): the rows per CTA H and padded
 // pitch P of a slice split over an 8-CTA cluster (false if it does not fit),
@@ -245,6 +247,33 @@ int launch_seg_cycles(const CycleTable &ct, char *data, int64_t d3, int64_t slic
                       size_t carry_override_bytes);
 size_t seg_cycles_carry_bytes(const CycleTable &ct, int64_t d3, int64_t seg_bytes);
 int seg_cycles_team(int64_t seg_bytes, int aw);
+
+// Two sweeps for slices larger than the chip, whatever their sides: the longer
+// side is cut into q parts of t elements and a remainder of r, so that a band
+// of t rows (or t columns) fits the chip.  `cols` (n >= m): the r last columns
+// are saved, the segments of t elements permuted so that every band's lie
+// together, the bands transposed, and the r last output rows written.  Else
+// the inverse: the r last rows saved, bands transposed into segments, the
+// segments permuted, the r last output columns written.
+struct RaggedPlan {
+  bool ok = false, cols = false;
+  int64_t t = 0, q = 0, r = 0, small = 0;
+  HoldPlan hold;
+  PermSpec perm;
+  std::shared_ptr<CycleTable> table;
+};
+bool ragged_geometry(RaggedPlan &rp, int64_t m, int64_t n, int eb, int64_t d3);
+int ragged_table(RaggedPlan &rp, int eb, int64_t d3);  // builds the cycle table
+size_t ragged_workspace(const RaggedPlan &rp, int eb, int64_t d3);
+int ragged_launches(const RaggedPlan &rp);
+// kHoldNoSlot: nothing was launched, the caller takes another plan.
+int launch_ragged(const RaggedPlan &rp, char *data, int64_t d3, int64_t m, int64_t n, int eb, cudaStream_t st,
+                  LaunchStats *ls);
+// The band pass of a ragged plan (launch_hold.cu), and whether it could run
+// now; `slot` from hold_rag_ready.
+int hold_rag_ready(const RaggedPlan &rp, int eb, cudaStream_t st, int *slot);
+int launch_hold_rag(const RaggedPlan &rp, char *data, int64_t d3, int64_t slice_bytes, int eb, int slot,
+                    cudaStream_t st);
 
 // ----------------------------------------------------------------- timing --
 // Per-pass CUDA-event timing (enabled by t213_pass_timing_enable).

@@ -35,7 +35,9 @@ constexpr int kHoldThreads = 512;
 constexpr int kHoldSlots = 4096;  // barrier slots: one per stream, one per captured launch
 constexpr int kHoldTeams = 20;    // grid teams of a launch (17 CTAs or more each)
 
-enum HoldForm { HOLD_SCALAR = 0, HOLD_VEC = 1, HOLD_WIDE = 2 };
+// RAG_DST / RAG_SRC: scalar tiles of one band of a ragged band plan, whose
+// output columns / source rows lie as the segments of rows with a remainder.
+enum HoldForm { HOLD_SCALAR = 0, HOLD_VEC = 1, HOLD_WIDE = 2, HOLD_RAG_DST = 3, HOLD_RAG_SRC = 4 };
 
 struct HoldArgs {
   int64_t d3, slice_bytes;
@@ -48,6 +50,16 @@ struct HoldArgs {
   int32_t lgs;  // log2 of the lanes that share an output column
   uint32_t we;       // wide form: 16-byte words per element
   FastDiv<uint32_t> wediv, tcdiv, rbdiv;
+  // ragged bands: m x n is a band, nb bands per slice; segment s of a slice
+  // (seg_bytes long, q to a row of rag_pitch bytes) at
+  // (s / q) * rag_pitch + (s % q) * seg_bytes
+  FastDiv<uint32_t> qdiv;
+  uint32_t nb, seg_bytes;
+  int64_t rag_pitch;
+  __device__ __forceinline__ uint64_t seg_at(uint32_t s) const {
+    const uint32_t r = qdiv.div(s);
+    return (uint64_t)r * (uint64_t)rag_pitch + (uint64_t)(s - r * qdiv.get()) * seg_bytes;
+  }
 };
 
 // ---- tiles -------------------------------------------------------------------
@@ -60,22 +72,29 @@ struct HoldArgs {
 // bank line, the offset rotates over the 4 words of a block from row to row,
 // and the extra block separates rows 8 apart.  A packed tile (all columns of
 // narrow rows) is one contiguous piece.
-template <int EB>
-__device__ __forceinline__ uint32_t hold_row(const HoldArgs &a, uint32_t i, uint32_t lo, uint32_t pitch_lo) {
+template <int EB, int FORM>
+__device__ __forceinline__ uint32_t hold_row(const HoldArgs &a, uint32_t i, uint32_t lo, uint32_t pitch_lo,
+                                             uint32_t s0) {
   constexpr uint32_t N = EB < 4 ? 4 / EB : 1;
-  if (a.packed) return (lo & 15u) + i * (a.n * EB);
   const uint32_t l = i / N, b = i % N;
-  return b * a.H + l * a.P + (l >> 3) * 16 + ((lo + i * pitch_lo) & 15u);
+  if constexpr (FORM == HOLD_RAG_SRC) {
+    return b * a.H + l * a.P + (l >> 3) * 16 + ((lo + (uint32_t)a.seg_at(s0 + i)) & 15u);
+  } else {
+    if (a.packed) return (lo & 15u) + i * (a.n * EB);
+    return b * a.H + l * a.P + (l >> 3) * 16 + ((lo + i * pitch_lo) & 15u);
+  }
 }
 
+// `slice` is the slice, or the band's rows (RAG_DST), or the start of the
+// slice that the band belongs to (RAG_SRC, with s0 the band's first segment).
 template <int EB, int FORM>
 __device__ __forceinline__ void hold_load(const char *slice, const HoldArgs &a, uint32_t r0, uint32_t c0,
-                                          unsigned char *s) {
+                                          unsigned char *s, uint32_t s0) {
   uint32_t rows = min(a.tm, a.m - r0), cols = min(a.tn, a.n - c0);
   const uint32_t E = EB * (FORM == HOLD_WIDE ? a.we : 1);
   const uint32_t pitch = a.n * E;  // a slice is far below 4 GB
-  const char *g0 = slice + (size_t)r0 * pitch + (size_t)c0 * E;
-  if (FORM == HOLD_SCALAR && a.packed) {
+  const char *g0 = slice + (FORM == HOLD_RAG_SRC ? 0 : (size_t)r0 * pitch) + (size_t)c0 * E;
+  if ((FORM == HOLD_SCALAR || FORM == HOLD_RAG_DST) && a.packed) {
     const uint32_t sh = (uint32_t)(uintptr_t)g0 & 15u;
     const char *g = g0 - sh;
     const uint32_t nc = (sh + rows * pitch + 15) >> 4;
@@ -90,7 +109,7 @@ __device__ __forceinline__ void hold_load(const char *slice, const HoldArgs &a, 
   uint32_t i = threadIdx.x / nc, c = threadIdx.x - i * nc;
 #pragma unroll 4
   for (; i < rows;) {
-    const char *g = g0 + (size_t)(i * pitch);
+    const char *g = g0 + (FORM == HOLD_RAG_SRC ? (size_t)a.seg_at(s0 + r0 + i) : (size_t)(i * pitch));
     if constexpr (FORM == HOLD_VEC) {
       constexpr uint32_t Q = 16 / EB;
       cp_async<16>(s + i * a.P + ((c ^ ((i / Q) & 7u)) << 4), g + c * 16);
@@ -111,9 +130,11 @@ __device__ __forceinline__ void hold_load(const char *slice, const HoldArgs &a, 
   }
 }
 
+// `slice` is where the columns go, `from` where the rows came from (hold_load's
+// `slice`), s0 the band's first segment.
 template <int EB, int FORM>
-__device__ __forceinline__ void hold_store(char *slice, const HoldArgs &a, uint32_t r0, uint32_t c0,
-                                           const unsigned char *s) {
+__device__ __forceinline__ void hold_store(char *slice, const char *from, const HoldArgs &a, uint32_t r0, uint32_t c0,
+                                           const unsigned char *s, uint32_t s0) {
   using E = typename ElemT<EB>::type;
   const uint32_t rows = min(a.tm, a.m - r0), cols = min(a.tn, a.n - c0);
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -167,7 +188,9 @@ __device__ __forceinline__ void hold_store(char *slice, const HoldArgs &a, uint3
     constexpr uint32_t N = EB < 4 ? 4 / EB : 1;
     constexpr uint32_t U = EB == 16 ? 4 : EB == 4 ? 16 : 8;
     const uint32_t L = 1u << a.lgs, G = 32u >> a.lgs, li = lane & (L - 1), sub = lane >> a.lgs;
-    const uint32_t lo = (uint32_t)(uintptr_t)(slice + (size_t)(r0 * a.n + c0) * EB), plo = a.n * EB;
+    const uint32_t plo = a.n * EB;
+    const uint32_t lo = (uint32_t)(uintptr_t)from + (FORM == HOLD_RAG_SRC ? c0 * EB : (r0 * a.n + c0) * EB);
+    const uint32_t sr = s0 + r0;  // RAG_SRC: the segment of the tile's first row
     const uint32_t words = N == 1 ? rows : (rows + 2 * N - 2) / N;  // one more covers every offset
     const uint32_t nrb = (words + L - 1) >> a.lgs, ncg = (cols + U * G * N - 1) / (U * G * N) * N;
     const bool full = rows == a.tm;
@@ -181,9 +204,20 @@ __device__ __forceinline__ void hold_store(char *slice, const HoldArgs &a, uint3
       const uint32_t ps = G * N * EB;
       const uint32_t left = (cols - 1 - j0) / (G * N) + 1;  // column steps of this lane
       if constexpr (N == 1) {
-        const unsigned char *p = s + hold_row<EB>(a, w, lo, plo) + j0 * EB;
-        char *g = slice + (size_t)(o + w * EB);
+        const unsigned char *p = s + hold_row<EB, FORM>(a, w, lo, plo, sr) + j0 * EB;
         E v[U];
+        if constexpr (FORM == HOLD_RAG_DST) {
+          char *g = slice + (size_t)((r0 + w) * EB);
+          const uint32_t sj = s0 + c0 + j0;
+#pragma unroll
+          for (uint32_t q = 0; q < U; q++)
+            if (q < left) v[q] = *reinterpret_cast<const E *>(p + q * ps);
+#pragma unroll
+          for (uint32_t q = 0; q < U; q++)
+            if (q < left) *reinterpret_cast<E *>(g + a.seg_at(sj + q * G)) = v[q];
+          continue;
+        }
+        char *g = slice + (size_t)(o + w * EB);
         if (left >= U) {
 #pragma unroll
           for (uint32_t q = 0; q < U; q++) v[q] = *reinterpret_cast<const E *>(p + q * ps);
@@ -194,13 +228,35 @@ __device__ __forceinline__ void hold_store(char *slice, const HoldArgs &a, uint3
           for (uint32_t q = 0; q < U; q++)
             if (q < left) *reinterpret_cast<E *>(g + (size_t)(q * gs)) = *reinterpret_cast<const E *>(p + q * ps);
         }
+      } else if constexpr (FORM == HOLD_RAG_DST) {
+        // the offset of an output row is its own: column by column
+        for (uint32_t q = 0; q < min(left, U); q++) {
+          char *g = slice + a.seg_at(s0 + c0 + j0 + q * (G * N)) + (size_t)(r0 * EB);
+          const uint32_t h = ((uint32_t)(uintptr_t)g & 3u) / EB;
+          const int32_t e0 = (int32_t)(w * N) - (int32_t)h;
+          uint32_t v = 0;
+#pragma unroll
+          for (uint32_t b = 0; b < N; b++)
+            v |= (uint32_t) * reinterpret_cast<const E *>(
+                     s + hold_row<EB, FORM>(a, min((uint32_t)max(e0 + (int32_t)b, 0), rows - 1), lo, plo, sr) +
+                     j0 * EB + q * ps)
+                 << (8 * EB * b);
+          g += (int64_t)e0 * EB;
+          if (e0 >= 0 && e0 + (int32_t)N <= (int32_t)rows) {
+            *reinterpret_cast<uint32_t *>(g) = v;
+          } else {
+#pragma unroll
+            for (uint32_t b = 0; b < N; b++)
+              if ((uint32_t)(e0 + (int32_t)b) < rows) *reinterpret_cast<E *>(g + b * EB) = (E)(v >> (8 * EB * b));
+          }
+        }
       } else {
         const uint32_t h = (((uint32_t)(uintptr_t)slice + o) & 3u) / EB;
         const int32_t e0 = (int32_t)(w * N) - (int32_t)h;
         const unsigned char *p[N];
 #pragma unroll
         for (uint32_t b = 0; b < N; b++)
-          p[b] = s + hold_row<EB>(a, min((uint32_t)max(e0 + (int32_t)b, 0), rows - 1), lo, plo) + j0 * EB;
+          p[b] = s + hold_row<EB, FORM>(a, min((uint32_t)max(e0 + (int32_t)b, 0), rows - 1), lo, plo, sr) + j0 * EB;
         uint32_t v[U];
 #pragma unroll
         for (uint32_t q = 0; q < U; q++) {
@@ -291,13 +347,35 @@ __global__ void __launch_bounds__(kHoldThreads, 2)
     r0 = tr * a.tm;
     c0 = (t - tr * a.TC) * a.tn;
   };
+  // item k: a slice, or a band of one.  RAG_DST takes a slice's bands from the
+  // last to the first, because a band's columns reach past the end of its
+  // rows into those of the band after it, which the barrier of the item
+  // before has seen loaded; RAG_SRC takes them from the first to the last.
+  // The next item's rows never overlap this item's columns, so they are
+  // loaded while those are written.
+  auto item = [&](int64_t kk, char *&slice, char *&from, uint32_t &s0) {
+    if constexpr (FORM == HOLD_RAG_DST || FORM == HOLD_RAG_SRC) {
+      const int64_t sl = kk / a.nb;
+      const uint32_t b = FORM == HOLD_RAG_DST ? a.nb - 1 - (uint32_t)(kk - sl * a.nb) : (uint32_t)(kk - sl * a.nb);
+      const size_t band = (size_t)b * a.m * a.n * EB;
+      char *base = data + sl * a.slice_bytes;
+      slice = FORM == HOLD_RAG_DST ? base : base + band;
+      from = FORM == HOLD_RAG_DST ? base + band : base;
+      s0 = b * (FORM == HOLD_RAG_DST ? a.n : a.m);
+    } else {
+      slice = from = data + kk * a.slice_bytes;
+      s0 = 0;
+    }
+  };
+  char *slice, *from;
+  uint32_t s0;
+  item(k, slice, from, s0);
   {
-    const char *slice = data + k * a.slice_bytes;
     uint32_t q = 0;
     for (uint32_t t = rank; t < a.T; t += a.ctas, q++) {
       uint32_t r0, c0;
       tile_pos(t, r0, c0);
-      hold_load<EB, FORM>(slice, a, r0, c0, smem_raw + (size_t)q * a.tile_bytes);
+      hold_load<EB, FORM>(from, a, r0, c0, smem_raw + (size_t)q * a.tile_bytes, s0);
     }
   }
   for (;;) {
@@ -317,21 +395,26 @@ __global__ void __launch_bounds__(kHoldThreads, 2)
         return;
       }
     }
-    char *slice = data + k * a.slice_bytes;
     const int64_t next = k + a.teams;
+    char *nslice = slice, *nfrom = from;
+    uint32_t ns0 = s0;
+    if (next < a.d3) item(next, nslice, nfrom, ns0);
     uint32_t q = 0;
     for (uint32_t t = rank; t < a.T; t += a.ctas, q++) {
       uint32_t r0, c0;
       tile_pos(t, r0, c0);
       unsigned char *buf = smem_raw + (size_t)q * a.tile_bytes;
-      hold_store<EB, FORM>(slice, a, r0, c0, buf);
+      hold_store<EB, FORM>(slice, from, a, r0, c0, buf, s0);
       if (next < a.d3) {
-        __syncthreads();  // every thread has read the tile: the next slice's may land
-        hold_load<EB, FORM>(data + next * a.slice_bytes, a, r0, c0, buf);
+        __syncthreads();  // every thread has read the tile: the next item's may land
+        hold_load<EB, FORM>(nfrom, a, r0, c0, buf, ns0);
       }
     }
     if (next >= a.d3) break;
     k = next;
+    slice = nslice;
+    from = nfrom;
+    s0 = ns0;
   }
 }
 

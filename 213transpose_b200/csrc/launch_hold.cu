@@ -1,6 +1,7 @@
 // Geometry and launch of the one-pass slice kernel (k_hold.cuh).
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <map>
@@ -51,14 +52,14 @@ int64_t hold_pitch(int64_t tn, int eb, int64_t we, int form) {
 // Bytes of one region of a tile (the tile itself unless the elements are
 // smaller than 4 bytes).
 int64_t hold_region(int64_t tm, int64_t P, int eb, int form) {
-  if (form != HOLD_SCALAR) return tm * P;
+  if (form == HOLD_VEC || form == HOLD_WIDE) return tm * P;
   const int64_t N = eb < 4 ? 4 / eb : 1, l = (tm + N - 1) / N;
   return l * P + l / 8 * 16;
 }
 
 int64_t hold_tile_bytes(int64_t tm, int64_t tn, int64_t P, int eb, int form, bool packed) {
   if (packed) return up(tm * tn * eb + 30, 128);
-  const int64_t N = form == HOLD_SCALAR && eb < 4 ? 4 / eb : 1;
+  const int64_t N = form != HOLD_VEC && form != HOLD_WIDE && eb < 4 ? 4 / eb : 1;
   return up(N * hold_region(tm, P, eb, form), 128);
 }
 
@@ -66,7 +67,7 @@ int64_t hold_tile_bytes(int64_t tm, int64_t tn, int64_t P, int eb, int form, boo
 // lost to the 16-byte blocks of every row, and at strides with few common
 // factors with the 32 banks a column costs few conflicts.
 bool hold_packed(int64_t n, int eb, int form) {
-  if (form != HOLD_SCALAR || n * eb > 256) return false;
+  if ((form != HOLD_SCALAR && form != HOLD_RAG_DST) || n * eb > 256) return false;
   const int64_t stride = eb < 4 ? n : n * eb / 4;  // words from lane to lane
   int64_t g = 1;
   while (g < 32 && stride % (g * 2) == 0) g *= 2;
@@ -96,6 +97,7 @@ bool hold_search(HoldGeom &g, int64_t m, int64_t n, int eb, int64_t we, int64_t 
   // tile sides in whole 32-byte sectors where the rows are
   const int64_t un = std::max<int64_t>(Q, (n * E) % 32 == 0 && E < 32 ? 32 / E : 1);
   const int64_t um = std::max<int64_t>(Q, (m * E) % 32 == 0 && E < 32 ? 32 / E : 1);
+  const bool rag = form == HOLD_RAG_DST || form == HOLD_RAG_SRC;  // one team: a slice's bands in order
   double best = 1e30;
   g.ok = false;
   for (int S = 1; S <= 2; S++) {
@@ -124,14 +126,15 @@ bool hold_search(HoldGeom &g, int64_t m, int64_t n, int eb, int64_t we, int64_t 
         const int64_t ctas = (T + S - 1) / S;
         const int mode = ctas == 1 ? HOLD_CTA : ctas <= 16 ? HOLD_CLUSTER : HOLD_GRID;
         if (S > 1 && mode != HOLD_GRID) continue;
-        const int64_t teams = std::min<int64_t>(d3, slots / ctas);
+        if (rag && mode != HOLD_GRID) continue;
+        const int64_t teams = rag ? 1 : std::min<int64_t>(d3, slots / ctas);
         if (mode == HOLD_GRID && teams > kHoldTeams) continue;
         const int64_t waves = (d3 + teams - 1) / teams;
         const int64_t conc = teams * ctas, per_sm = (conc + d.sms - 1) / d.sms;
         const double bw = std::min(60e9, 6.4e12 / (double)std::min<int64_t>(conc, d.sms)) / (double)per_sm;
         const double share = (double)S * tm * tn * E;
         // lanes left idle by tiles of a few rows more than a multiple of 32
-        const int64_t N = eb < 4 ? 4 / eb : 1, wd = form == HOLD_SCALAR ? (tm + N - 1) / N : 32;
+        const int64_t N = eb < 4 ? 4 / eb : 1, wd = form != HOLD_VEC && form != HOLD_WIDE ? (tm + N - 1) / N : 32;
         const double idle = wd >= 32 ? 0.5 * (double)(up(wd, 32) - wd) / (double)wd : 0.0;
         const double ineff = idle + 2.0 + 32.0 / (double)(tn * E) + 32.0 / (double)(tm * E);
         const double bar = mode == HOLD_CTA ? 0.2e-6 : mode == HOLD_CLUSTER ? 1.2e-6 : 2.5e-6;
@@ -269,10 +272,7 @@ void hold_plan(HoldPlan &hp, int64_t m, int64_t n, int eb, int64_t we, int64_t d
     hold_search(hp.vec, m, n, eb, 1, d3, HOLD_VEC);
 }
 
-bool slice_fits(int64_t m, int64_t n, int eb) {
-  HoldGeom g;
-  return hold_search(g, m, n, eb, 1, 1, HOLD_SCALAR);
-}
+int64_t hold_cluster_bytes() { return 16 * hold_budget(); }
 
 std::string describe_slice(const HoldPlan &hp) {
   const HoldGeom &g = hp.vec.ok ? hp.vec : hp.any;
@@ -319,7 +319,38 @@ int hold_prepare(HoldReady::Form &f, const HoldGeom &g, int64_t m, int64_t n, in
     a.rbdiv = FastDiv<uint32_t>((uint64_t)(words + (1 << a.lgs) - 1) >> a.lgs);
   }
   f.smem = (int64_t)g.S * a.tile_bytes;
-  switch (g.form == HOLD_WIDE ? 0 : g.form == HOLD_VEC ? -eb : eb) {
+  switch (g.form == HOLD_WIDE ? 0 : g.form == HOLD_VEC ? -eb : g.form == HOLD_RAG_DST ? 100 + eb
+          : g.form == HOLD_RAG_SRC ? 200 + eb : eb) {
+    case 101:
+      f.kern = (const void *)k_hold<1, HOLD_RAG_DST>;
+      break;
+    case 102:
+      f.kern = (const void *)k_hold<2, HOLD_RAG_DST>;
+      break;
+    case 104:
+      f.kern = (const void *)k_hold<4, HOLD_RAG_DST>;
+      break;
+    case 108:
+      f.kern = (const void *)k_hold<8, HOLD_RAG_DST>;
+      break;
+    case 116:
+      f.kern = (const void *)k_hold<16, HOLD_RAG_DST>;
+      break;
+    case 201:
+      f.kern = (const void *)k_hold<1, HOLD_RAG_SRC>;
+      break;
+    case 202:
+      f.kern = (const void *)k_hold<2, HOLD_RAG_SRC>;
+      break;
+    case 204:
+      f.kern = (const void *)k_hold<4, HOLD_RAG_SRC>;
+      break;
+    case 208:
+      f.kern = (const void *)k_hold<8, HOLD_RAG_SRC>;
+      break;
+    case 216:
+      f.kern = (const void *)k_hold<16, HOLD_RAG_SRC>;
+      break;
     case 0:
       f.kern = (const void *)k_hold<16, HOLD_WIDE>;
       break;
@@ -353,7 +384,9 @@ int hold_prepare(HoldReady::Form &f, const HoldGeom &g, int64_t m, int64_t n, in
   if (g.mode == HOLD_GRID) {
     f.bars = hold_bars(&status);
     if (!f.bars) return status;
-    f.resident = (int)g.teams;
+    int per_sm = 1;
+    occupancy_cached(f.kern, kHoldThreads, f.smem, 1, &per_sm);
+    f.resident = (int64_t)per_sm * dev_info().sms >= (int64_t)g.teams * g.ctas ? (int)g.teams : 0;
   } else {
     occupancy_cached(f.kern, kHoldThreads, f.smem, (int)g.ctas, &f.resident);
     if (g.mode == HOLD_CTA) f.resident *= dev_info().sms;
@@ -362,34 +395,7 @@ int hold_prepare(HoldReady::Form &f, const HoldGeom &g, int64_t m, int64_t n, in
   return T213_OK;
 }
 
-}  // namespace
-
-int launch_slice(const HoldPlan &hp, char *data, int64_t d3, int64_t m, int64_t n, int eb, int64_t we,
-                 cudaStream_t st, LaunchStats *ls) {
-  if (d3 <= 0 || m <= 0 || n <= 0) return T213_OK;
-  const bool vec = hp.vec.ok && (uintptr_t)data % 16 == 0;
-  const HoldGeom &g = vec ? hp.vec : hp.any;
-  if (!g.ok) {
-    set_error("slice does not fit the chip's shared memory");
-    return T213_ERR_UNSUPPORTED;
-  }
-  HoldReady::Form &f = vec ? hp.ready->vec : hp.ready->any;
-  if (!f.ready.load(std::memory_order_acquire)) {
-    std::lock_guard<std::mutex> lk(hp.ready->mu);
-    if (!f.ready.load(std::memory_order_relaxed)) {
-      const int rc = hold_prepare(f, g, m, n, eb, we);
-      if (rc) return rc;
-      f.ready.store(true, std::memory_order_release);
-    }
-  }
-  HoldArgs a = f.args;
-  a.d3 = d3;
-  // persistent: as many teams as are resident at once
-  a.teams = (uint32_t)std::min<int64_t>(f.resident, d3);
-  if (g.mode == HOLD_GRID) {
-    a.slot = hold_slot(st);
-    if (a.slot < 0) return kHoldNoSlot;
-  }
+int hold_enqueue(const HoldReady::Form &f, const HoldGeom &g, HoldArgs &a, char *data, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(a.teams * a.ctas, 1, 1);
   cfg.blockDim = dim3(kHoldThreads, 1, 1);
@@ -415,9 +421,106 @@ int launch_slice(const HoldPlan &hp, char *data, int64_t d3, int64_t m, int64_t 
                                      : cudaLaunchKernel(f.kern, cfg.gridDim, cfg.blockDim, args, cfg.dynamicSmemBytes, st);
   if (e == cudaErrorCooperativeLaunchTooLarge) {
     cudaGetLastError();
-    return kHoldNoSlot;  // fewer SMs than the device reports (a partitioned GPU)
+    return kHoldNoSlot;
   }
-  if (e != cudaSuccess) return cuda_status(e, "k_hold launch");
+  return e == cudaSuccess ? T213_OK : cuda_status(e, "k_hold launch");
+}
+
+int hold_form_ready(HoldReady &r, HoldReady::Form &f, const HoldGeom &g, int64_t m, int64_t n, int eb, int64_t we) {
+  if (f.ready.load(std::memory_order_acquire)) return T213_OK;
+  std::lock_guard<std::mutex> lk(r.mu);
+  if (f.ready.load(std::memory_order_relaxed)) return T213_OK;
+  const int rc = hold_prepare(f, g, m, n, eb, we);
+  if (rc == T213_OK) f.ready.store(true, std::memory_order_release);
+  return rc;
+}
+
+}  // namespace
+
+bool ragged_geometry(RaggedPlan &rp, int64_t m, int64_t n, int eb, int64_t d3) {
+  rp.ok = false;
+  rp.cols = n >= m;
+  const int64_t big = std::max(m, n), small = std::min(m, n);
+  const int64_t u = std::max(1, 16 / eb);
+  const double chip = 2.0 * dev_info().sms * (double)hold_budget();
+  const int64_t q0 = std::max<int64_t>(2, (int64_t)std::ceil((double)m * (double)n * eb / chip));
+  for (int64_t q = q0; q <= q0 + q0 / 4 + 4; q++) {
+    int64_t t = big / q;
+    if (t >= 4 * u) t = t / u * u;  // segments of whole 16-byte blocks
+    if (t * eb < 256 || (double)q * small > 4.0e6) return false;
+    const int64_t r = big - q * t;
+    rp.hold = HoldPlan{};
+    rp.hold.ready = std::make_shared<HoldReady>();
+    if (!hold_search(rp.hold.any, rp.cols ? m : t, rp.cols ? t : n, eb, 1, d3 * q,
+                     rp.cols ? HOLD_RAG_SRC : HOLD_RAG_DST))
+      continue;
+    rp.t = t;
+    rp.q = q;
+    rp.r = r;
+    rp.small = small;
+    PermSpec ps;
+    ps.kind = 0;
+    ps.A = rp.cols ? m : q;
+    ps.Mid = 1;
+    ps.C = rp.cols ? q : n;
+    ps.S = q * small;
+    rp.perm = ps;
+    rp.ok = true;
+    return true;
+  }
+  return false;
+}
+
+int hold_rag_ready(const RaggedPlan &rp, int eb, cudaStream_t st, int *slot) {
+  HoldReady &r = *rp.hold.ready;
+  const int64_t m = rp.cols ? rp.small : rp.t, n = rp.cols ? rp.t : rp.small;
+  const int rc = hold_form_ready(r, r.any, rp.hold.any, m, n, eb, 1);
+  if (rc) return rc;
+  if (r.any.resident == 0) return kHoldNoSlot;
+  *slot = hold_slot(st);
+  return *slot < 0 ? kHoldNoSlot : T213_OK;
+}
+
+int launch_hold_rag(const RaggedPlan &rp, char *data, int64_t d3, int64_t slice_bytes, int eb, int slot,
+                    cudaStream_t st) {
+  const HoldReady::Form &f = rp.hold.ready->any;
+  HoldArgs a = f.args;
+  a.d3 = d3 * rp.q;
+  a.slice_bytes = slice_bytes;
+  a.teams = 1;
+  a.slot = slot;
+  a.nb = (uint32_t)rp.q;
+  a.qdiv = FastDiv<uint32_t>((uint64_t)rp.q);
+  a.seg_bytes = (uint32_t)(rp.t * eb);
+  a.rag_pitch = (rp.q * rp.t + rp.r) * eb;
+  return hold_enqueue(f, rp.hold.any, a, data, st);
+}
+
+int launch_slice(const HoldPlan &hp, char *data, int64_t d3, int64_t m, int64_t n, int eb, int64_t we,
+                 cudaStream_t st, LaunchStats *ls) {
+  if (d3 <= 0 || m <= 0 || n <= 0) return T213_OK;
+  const bool vec = hp.vec.ok && (uintptr_t)data % 16 == 0;
+  const HoldGeom &g = vec ? hp.vec : hp.any;
+  if (!g.ok) {
+    set_error("slice does not fit the chip's shared memory");
+    return T213_ERR_UNSUPPORTED;
+  }
+  HoldReady::Form &f = vec ? hp.ready->vec : hp.ready->any;
+  {
+    const int rc = hold_form_ready(*hp.ready, f, g, m, n, eb, we);
+    if (rc) return rc;
+  }
+  HoldArgs a = f.args;
+  a.d3 = d3;
+  if (f.resident == 0) return kHoldNoSlot;  // fewer SMs than the device reports (a partitioned GPU)
+  // persistent: as many teams as are resident at once
+  a.teams = (uint32_t)std::min<int64_t>(f.resident, d3);
+  if (g.mode == HOLD_GRID) {
+    a.slot = hold_slot(st);
+    if (a.slot < 0) return kHoldNoSlot;
+  }
+  const int rc = hold_enqueue(f, g, a, data, st);
+  if (rc) return rc;
   if (ls) ls->launches++;
   return T213_OK;
 }

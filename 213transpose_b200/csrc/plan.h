@@ -9,7 +9,7 @@
 
 namespace t213 {
 
-enum PassType { PT_COL = 1, PT_ROW = 2, PT_SEG = 3, PT_TILE = 4, PT_BAND = 5, PT_SLICE = 6 };
+enum PassType { PT_COL = 1, PT_ROW = 2, PT_SEG = 3, PT_TILE = 4, PT_BAND = 5, PT_SLICE = 6, PT_RAGGED = 7 };
 
 struct PassDesc {
   PassType type = PT_COL;
@@ -21,6 +21,7 @@ struct PassDesc {
   int64_t t = 0;                     // PT_TILE: block side
   int64_t R = 0, C = 0, bands = 0;   // PT_BAND: band shape, bands per slice
   HoldPlan hold;                     // PT_SLICE: the tiling
+  RaggedPlan ragged;                 // PT_RAGGED
   const char *name() const;
 };
 
@@ -32,6 +33,7 @@ struct Plan {
   std::vector<PassDesc> passes;
   std::string desc;
   double est_cost = 0;  // heuristic, in units of one full read+write sweep
+  int fallback = -1;    // kind that runs instead where this plan cannot (kPlanSweeps)
   Variant var;          // kernel choices pinned by the tuner (default: none)
 };
 
@@ -42,6 +44,10 @@ constexpr int kPlanSweeps = -1;
 constexpr int kPlanOnePassOr = -16;
 // Internal kind: the one-pass plan of elements of eb = a multiple of 16 bytes.
 constexpr int kPlanWideSlice = -2;
+// Internal kind: the automatic choice without the tuner's entries.
+constexpr int kPlanUntuned = -3;
+// Internal kind: the two-sweep plan of slices larger than the chip (PT_RAGGED).
+constexpr int kPlanRagged = 9;
 // Builds the plan of a family (T213_PLAN_*; AUTO picks).  t = 0 lets the
 // planner choose the block/band size.  Cached per device.
 std::shared_ptr<Plan> get_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int kind, int64_t t, int *status);

@@ -85,6 +85,13 @@ char *workspace(cudaStream_t st, size_t bytes, int *status) {
   return p;
 }
 
+bool workspace_ready(cudaStream_t st, size_t bytes) {
+  const int dev = dev_info().id;
+  std::lock_guard<std::mutex> lk(g_ws_mu);
+  auto it = g_ws.find({dev, st});
+  return bytes == 0 || (it != g_ws.end() && it->second.first && it->second.second >= bytes);
+}
+
 // A variable of the module rather than an allocation: it is zero from the
 // start, and a first call inside a stream capture may take its address.
 __device__ int g_status_word[64];
@@ -257,6 +264,8 @@ const char *PassDesc::name() const {
       return "band_transpose";
     case PT_SLICE:
       return "slice";
+    case PT_RAGGED:
+      return "ragged";
   }
   return "?";
 }
@@ -315,8 +324,8 @@ double seg_eff(int64_t seg_bytes) {
 
 std::string fmt_plan(const Plan &P) {
   VariantScope vs(P.var);  // the pass descriptions show the kernels this plan's variant picks
-  static const char *kn[] = {"auto", "c2r", "r2c", "skinny", "blocks", "bands", "bands_t", "identity", "slice"};
-  std::string s = kn[P.kind >= 0 && P.kind <= 8 ? P.kind : 0];
+  static const char *kn[] = {"auto", "c2r", "r2c", "skinny", "blocks", "bands", "bands_t", "identity", "slice", "ragged"};
+  std::string s = kn[P.kind >= 0 && P.kind <= kPlanRagged ? P.kind : 0];
   char buf[256];
   if (P.t) {
     snprintf(buf, sizeof buf, " t=%lld", (long long)P.t);
@@ -338,6 +347,12 @@ std::string fmt_plan(const Plan &P) {
         break;
       case PT_SLICE:
         snprintf(buf, sizeof buf, "%s", describe_slice(p.hold).c_str());
+        break;
+      case PT_RAGGED:
+        snprintf(buf, sizeof buf, "%s(q=%lld r=%lld seg=%lldB chunks=%lld carry=%lld) %s", p.ragged.cols ? "cols" : "rows",
+                 (long long)p.ragged.q, (long long)p.ragged.r, (long long)(p.ragged.t * P.eb),
+                 (long long)p.ragged.table->n_chunks, (long long)p.ragged.table->n_carry,
+                 describe_slice(p.ragged.hold).c_str());
         break;
       case PT_SEG:
         snprintf(buf, sizeof buf, "segment_cycles(S=%lld seg=%lldB cycles=%lld chunks=%lld carry=%lld maxlen=%lld)",
@@ -541,6 +556,21 @@ int build_plan(Plan &P, int kind, int64_t t) {
       P.passes.push_back(sp);
       return T213_OK;
     }
+    case kPlanRagged: {
+      PassDesc rp;
+      rp.type = PT_RAGGED;
+      rp.m = m;
+      rp.n = n;
+      if (!ragged_geometry(rp.ragged, m, n, eb, d3)) {
+        set_error("no bands of this slice fit the chip");
+        return T213_ERR_UNSUPPORTED;
+      }
+      const int st = ragged_table(rp.ragged, eb, d3);
+      if (st) return st;
+      P.t = rp.ragged.t;
+      P.passes.push_back(rp);
+      return T213_OK;
+    }
     case T213_PLAN_BANDS_T: {
       if (t <= 0) t = pick_band_t_t(m, n, eb);
       if (t <= 0 || n % t || !band_fits(m, t, eb)) {
@@ -569,6 +599,28 @@ int build_plan(Plan &P, int kind, int64_t t) {
   return T213_ERR_INVALID_ARGUMENT;
 }
 
+// Bytes of the column strips that a plan gathers.
+int64_t col_strip_bytes(const Plan &P) {
+  int64_t w = 1 << 20;
+  for (const PassDesc &p : P.passes) {
+    if (p.type != PT_COL) continue;
+    const std::string d = describe_col_gather_fn(p.fn, p.m, p.n, P.eb, nullptr);
+    const size_t at = d.find("W=");
+    if (at != std::string::npos) w = std::min<int64_t>(w, std::atoll(d.c_str() + at + 2) * P.eb);
+  }
+  return w;
+}
+
+// The ragged bands, in the units of the other estimates.  Measured on slices
+// larger than the chip (B200, times over that of one copy of the tensor, the
+// other plan / ragged, fp32 unless said): two gathers over 128-byte strips
+// 2.5-3.2 / 2.6-3.5, three gathers 4.0-5.6 / 2.8-3.8, narrower strips 5.5-8 /
+// 3.1-3.6, 1- and 2-byte gathers 6-40 / 3.5-5.9, rows or columns through
+// scratch 12-28 / 2.5-3.6; bands of aligned segments from 448 bytes 1.9-2.8 /
+// 2.6-4.8, unaligned ones 7.4 / 3.5 (8-byte elements 3.4 / 4.0), blocks of odd
+// sides 5.8 / 2.6.
+constexpr double kRaggedCost = 3.6;
+
 double plan_cost(const Plan &P) {
   double c = 0;
   for (const PassDesc &p : P.passes) {
@@ -590,9 +642,19 @@ double plan_cost(const Plan &P) {
       case PT_SLICE:
         c += 1 / 0.6;
         break;
+      case PT_RAGGED:
+        c += kRaggedCost;
+        break;
     }
   }
   return c;
+}
+
+// The cost of a C2R, R2C or skinny plan where the ragged bands are the
+// alternative: 1- and 2-byte elements and narrow strips count double.
+double gather_plan_cost(const Plan &P) {
+  const double c = plan_cost(P);
+  return P.eb < 4 || col_strip_bytes(P) < 128 ? 2 * c : c;
 }
 
 // Cheap estimate used to rank candidates before any cycle table is built.
@@ -690,7 +752,9 @@ bool plan_cached(int64_t d1, int64_t d2, int64_t d3, int eb, int kind, int64_t t
 std::shared_ptr<Plan> get_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int kind, int64_t t, int *status) {
   *status = T213_OK;
   const int dev = dev_info().id;
-  if (kind == T213_PLAN_AUTO) {
+  const bool untuned = kind == kPlanUntuned;
+  if (untuned) kind = T213_PLAN_AUTO;
+  if (kind == T213_PLAN_AUTO && !untuned) {
     int tk = 0;
     int64_t tt = 0;
     Variant tv;
@@ -730,7 +794,19 @@ std::shared_ptr<Plan> get_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int k
       else if (d1 * d2 * eb < (64 << 20))  // above the shared memory of any chip
         st = build_plan(*best, T213_PLAN_SLICE, 0);
     }
-    if (st) st = build_plan(*best, kind <= kPlanOnePassOr ? kPlanOnePassOr - kind : kind, t);
+    if (st && kind <= kPlanOnePassOr) {
+      const int family = kPlanOnePassOr - kind;
+      st = build_plan(*best, family, 0);
+      if (st == T213_OK && gather_plan_cost(*best) > kRaggedCost) {
+        auto R = new_plan(d1, d2, d3, eb);
+        if (build_plan(*R, kPlanRagged, 0) == T213_OK) {
+          R->fallback = family;
+          best = R;
+        }
+      }
+    } else if (st) {
+      st = build_plan(*best, kind, t);
+    }
     if (st) {
       *status = st;
       return nullptr;
@@ -756,23 +832,30 @@ std::shared_ptr<Plan> get_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int k
       int64_t tc = pick_band_t_t(m, n, eb);
       cands.push_back({T213_PLAN_BANDS_T, tc, estimate_cost(T213_PLAN_BANDS_T, m, n, tc, eb, d3)});
       // The one-pass plan (T213_PLAN_SLICE) is the fastest wherever a slice
-      // fits the chip, but for two classes.  Square slices of whole tiles are
-      // one sweep of tile swaps without a barrier: 16-byte
-      // (1024, 1024, 4) 24.8 us against 31.1, fp32 (2048, 2048, 8) 51.2 against
-      // 58.2; at 8 MB and below they tie or lose.  A single small slice that needs a cooperative launch (more than
-      // 16 CTAs) and has a block or band plan with segments of 256 bytes or
-      // more keeps that plan up to 4 MB: such a launch starts only when the whole
-      // chip is free of other streams' kernels, for a gain of a few us.
+      // fits the chip, but for three classes (B200, us).  Square slices of
+      // whole tiles are one sweep of tile swaps without a barrier: 16-byte
+      // (1024, 1024, 4) 24.8 against 31.1, fp32 (2048, 2048, 8) 51.2 against
+      // 58.2; at 8 MB and below they tie or lose.  Many slices of less than
+      // 32 KB are one sweep of bands or tiles that takes the next slice's load
+      // ahead: fp32 (48, 60, 12000) 51 against 81, (16, 16, 20000) 20 against
+      // 86, (100, 100, 1000), 40 KB, 21 either way.  A small slice that needs
+      // a cooperative launch (more than 16 CTAs' memory) and has a block or
+      // band plan of aligned segments of 256 bytes or more keeps that plan up
+      // to 4 MB: such a launch starts only when the whole chip is free of
+      // other streams' kernels, for a gain of a few us.
+      bool one_pass = false;  // a slice fits the chip
       if (kind == T213_PLAN_AUTO) {
         auto P = new_plan(d1, d2, d3, eb);
         if (build_plan(*P, T213_PLAN_SLICE, 0) == T213_OK) {
+          one_pass = true;
           const HoldPlan &hp = P->passes[0].hold;
-          const bool coop = hp.any.mode == HOLD_GRID;
+          const bool coop = hp.any.mode == HOLD_GRID && d1 * d2 * eb > hold_cluster_bytes();
           const double total = (double)d1 * d2 * d3 * eb;
           bool seg = false;
           for (const Cand &c : cands) seg = seg || (eb >= 4 && c.est < 1e8 && c.t * eb >= 256 && c.t * eb % 16 == 0);
           const bool square = m == n && tb == m && tile_eff(tb, eb) >= 0.9 && total > (8 << 20);
-          if (!square && !(coop && seg && total <= (4 << 20))) {
+          const bool crumbs = d3 > 2 * dev_info().sms && d1 * d2 * eb < (32 << 10);
+          if (!square && !crumbs && !(coop && seg && total <= (4 << 20))) {
             P->est_cost = plan_cost(*P);
             best = P;
           }
@@ -793,6 +876,30 @@ std::shared_ptr<Plan> get_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int k
         // ties go to the reference's choice
         const bool ref_choice = (k == T213_PLAN_C2R) == (d1 >= d2);
         cands.push_back({k, 0, plan_cost(tmp) * (ref_choice ? 1.0 : 1.0001)});
+      }
+      if (kind == T213_PLAN_AUTO && !one_pass) {
+        // The ragged bands against the others: the estimates of the classes
+        // that lose to them, or win, are set right here, where they are the
+        // alternative (kRaggedCost has the measurements).
+        for (Cand &c : cands) {
+          if (c.est >= 1e8) continue;
+          if (c.kind == T213_PLAN_C2R || c.kind == T213_PLAN_R2C) {
+            Plan tmp;
+            tmp.d1 = d1;
+            tmp.d2 = d2;
+            tmp.d3 = d3;
+            tmp.eb = eb;
+            build_plan(tmp, c.kind, 0);
+            if (gather_plan_cost(tmp) > plan_cost(tmp)) c.est *= 2;
+          } else if (!(m == n && c.t == m)) {
+            const bool bands = c.kind != T213_PLAN_BLOCKS;
+            if (c.t * eb % 16 == 0 && c.t * eb >= 448)
+              c.est = bands ? std::min(c.est, kRaggedCost - 0.1) : c.est;
+            else if (!(bands && eb >= 8 && c.t * eb >= 1024))
+              c.est += 4;
+          }
+        }
+        cands.push_back({kPlanRagged, 0, kRaggedCost});
       }
       std::sort(cands.begin(), cands.end(), [](const Cand &a, const Cand &b) { return a.est < b.est; });
       for (const Cand &c : cands) {
@@ -831,7 +938,9 @@ std::shared_ptr<Plan> get_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int k
 size_t plan_workspace_bytes(const Plan &p) {
   size_t w = 0;
   for (const PassDesc &q : p.passes)
-    if (q.type == PT_SEG && q.table) w = std::max(w, seg_cycles_carry_bytes(*q.table, p.d3, q.seg_bytes));
+    if (q.type == PT_RAGGED)
+      w = std::max(w, ragged_workspace(q.ragged, p.eb, p.d3));
+    else if (q.type == PT_SEG && q.table) w = std::max(w, seg_cycles_carry_bytes(*q.table, p.d3, q.seg_bytes));
   return w;
 }
 
@@ -882,6 +991,13 @@ int run_plan(const Plan &P, char *data, cudaStream_t st, LaunchStats *ls) {
           break;
         case PT_SEG:
           rc = launch_seg_cycles(*p.table, gd, g, slice_bytes, p.seg_bytes, st, ls, nullptr, 0);
+          break;
+        case PT_RAGGED:
+          rc = launch_ragged(p.ragged, gd, g, p.m, p.n, P.eb, st, ls);
+          if (rc == kHoldNoSlot) {
+            auto alt = get_plan(P.d1, P.d2, g, P.eb, P.fallback, 0, &rc);
+            if (alt) rc = run_plan(*alt, gd, st, ls);
+          }
           break;
         case PT_SLICE:
           rc = launch_slice(p.hold, gd, g, p.m, p.n, P.eb, 1, st, ls);
@@ -960,8 +1076,9 @@ int run_shape(void *data, int64_t d1, int64_t d2, int64_t d3, int32_t eb, int ki
   // The decomposition's entry points are transposes too: C2R and skinny C2R
   // of (d1, d2), R2C and skinny R2C of the shape they make, (d2, d1).  They
   // take the one-pass plan where a slice fits the chip (fp32 r2c to
-  // (2000, 3001, 4): 78 us by its gathers, 52 us in one pass), else their own
-  // passes, from the plan cache (building them cost 20 us a call).
+  // (2000, 3001, 4): 78 us by its gathers, 51 us in one pass), the ragged
+  // bands where those are the better ones, else their own passes, all from
+  // the plan cache (building a plan cost 20 us a call).
   if ((which == 3 || which == 4) && d2 > 32) {
     set_error(which == 3 ? "skinny C2R needs d2 <= 32" : "skinny R2C needs d2 <= 32");
     return T213_ERR_INVALID_ARGUMENT;
@@ -1291,6 +1408,9 @@ int t213_plan_launches(int64_t d1, int64_t d2, int64_t d3, int32_t elem_bytes, i
           break;
         case PT_SEG:
           n += (p.table->n_chunks > 0) + (p.table->n_carry > 0);
+          break;
+        case PT_RAGGED:
+          n += ragged_launches(p.ragged);
           break;
         default:
           n += 1;

@@ -189,7 +189,18 @@ int t213_tune_shape(void *scratch_data, int64_t d1, int64_t d2, int64_t d3, int3
       best = Entry{kind, t, 0};
     }
   }
-  if (best.kind == T213_PLAN_AUTO) {
+  // the ragged bands have no public name: where they are the automatic choice
+  // and win, the entry keeps that choice
+  bool found = best.kind != T213_PLAN_AUTO;
+  {
+    int rc = T213_OK;
+    auto P = get_plan(d1, d2, d3, elem_bytes, kPlanUntuned, 0, &rc);
+    if (P && P->kind == kPlanRagged && time_plan(kPlanUntuned, 0, Variant{}, nullptr) < best_ms) {
+      best = Entry{T213_PLAN_AUTO, 0, 0};
+      found = true;
+    }
+  }
+  if (!found) {
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     cudaGetLastError();
@@ -206,7 +217,7 @@ int t213_tune_shape(void *scratch_data, int64_t d1, int64_t d2, int64_t d3, int3
     }
   }
   // 3) the kernel variants of the passes the plan has, one choice at a time
-  {
+  if (best.kind != T213_PLAN_AUTO) {
     int rc = T213_OK;
     std::shared_ptr<Plan> P = get_plan(d1, d2, d3, elem_bytes, best.kind, best.t, &rc);
     bool has[8] = {false, false, false, false, false, false, false, false};
