@@ -43,6 +43,9 @@ struct t213_batch_st {
   cudaEvent_t fork = nullptr, join = nullptr;
   std::string desc;
   int64_t total_bytes = 0;
+  HoldRounds *rounds = nullptr;  // tensors of the one-pass kernel's rounds
+  bool serial = false;           // everything on the caller's stream, one launch after the other
+  std::vector<char> in_rounds;
   // limit of every dependency wait of the persistent kernel (nanoseconds of
   // %globaltimer); lowered only by t213_batch_debug_stall
   uint64_t wait_ns = kWaitNs;
@@ -573,7 +576,8 @@ int t213_batch_create(const t213_tensor_desc *tensors, int32_t count, t213_batch
     return code;
   };
 
-  // ---- plans ---------------------------------------------------------------
+  int64_t auto_bytes = 0;
+  std::vector<int> auto_tensors;
   for (int32_t i = 0; i < count; i++) {
     const t213_tensor_desc &d = tensors[i];
     if (d.d1 < 0 || d.d2 < 0 || d.d3 < 0 || (d.elem_bytes != 1 && d.elem_bytes != 2 && d.elem_bytes != 4 &&
@@ -586,13 +590,46 @@ int t213_batch_create(const t213_tensor_desc *tensors, int32_t count, t213_batch
       return fail(T213_ERR_INVALID_ARGUMENT);
     }
     B->total_bytes += d.d1 * d.d2 * d.d3 * d.elem_bytes;
+    if (d.plan_kind == T213_PLAN_AUTO && d.d1 > 1 && d.d2 > 1 && d.d3 > 0) {
+      auto_tensors.push_back(i);
+      auto_bytes += d.d1 * d.d2 * d.d3 * d.elem_bytes;
+    }
+  }
+
+  // ---- rounds -------------------------------------------------------------------
+  // Tensors of the automatic choice whose slices fit a round share one launch
+  // of the one-pass kernel; the others of that choice then run their own plan
+  // after it, on the caller's stream, since both take the whole chip.
+  // Measured on B200, rounds against the persistent kernel, us: 8 tensors of
+  // 0.3 MB 12 / 86, 64 of 0.1 MB 16 / 100, 8 of 16 MB 87 / 198; the batched
+  // workload of 512 tensors 6346 / 10558.  A batch of up to three small
+  // tensors stays in the persistent kernel, whose dependency waits
+  // t213_batch_debug_stall lets run out.
+  B->in_rounds.assign(count, 0);
+  B->serial = auto_tensors.size() > 3 || auto_bytes >= (8 << 20);
+  if (B->serial) {
+    std::vector<int> taken;
+    B->rounds = hold_rounds_create(tensors, auto_tensors, taken, &rc);
+    if (rc) return fail(rc);
+    for (int i : taken) B->in_rounds[i] = 1;
+  }
+
+  // ---- plans ---------------------------------------------------------------
+  for (int32_t i = 0; i < count; i++) {
+    const t213_tensor_desc &d = tensors[i];
     std::shared_ptr<Plan> P;
-    if (d.d1 * d.d2 * d.d3 > 0) {
-      P = d.plan_kind == T213_PLAN_AUTO ? group_plan(d.d1, d.d2, d.d3, d.elem_bytes, &rc, true) : nullptr;
-      if (!P)
-        P = get_plan(d.d1, d.d2, d.d3, d.elem_bytes, d.plan_kind == T213_PLAN_AUTO ? kPlanSweeps : d.plan_kind, 0, &rc);
-      if (!P) return fail(rc);
-      if (!plan_fits_batch(*P) || d.d1 * d.d2 * d.d3 * d.elem_bytes > direct_threshold()) B->spill.push_back(i);
+    if (d.d1 * d.d2 * d.d3 > 0 && !B->in_rounds[i]) {
+      if (d.plan_kind == T213_PLAN_AUTO && B->serial) {
+        P = get_plan(d.d1, d.d2, d.d3, d.elem_bytes, T213_PLAN_AUTO, 0, &rc);
+        if (!P) return fail(rc);
+        if (!P->passes.empty()) B->spill.push_back(i);
+      } else {
+        P = d.plan_kind == T213_PLAN_AUTO ? group_plan(d.d1, d.d2, d.d3, d.elem_bytes, &rc, true) : nullptr;
+        if (!P)
+          P = get_plan(d.d1, d.d2, d.d3, d.elem_bytes, d.plan_kind == T213_PLAN_AUTO ? kPlanSweeps : d.plan_kind, 0, &rc);
+        if (!P) return fail(rc);
+        if (!plan_fits_batch(*P) || d.d1 * d.d2 * d.d3 * d.elem_bytes > direct_threshold()) B->spill.push_back(i);
+      }
     }
     B->plans.push_back(P);
   }
@@ -601,7 +638,7 @@ int t213_batch_create(const t213_tensor_desc *tensors, int32_t count, t213_batch
   // Measured on the 455 small tensors of the batched workload: 4.76 ms with
   // the 150 that fit taken out of the persistent kernel into one grouped
   // cluster launch, against 4.36 ms without; so it is off by default.
-  std::vector<char> skip(count, 0);
+  std::vector<char> skip = B->in_rounds;
   for (int i : B->spill) skip[i] = 1;
   {
     const char *sv = getenv("T213_BATCH_SLICE");
@@ -690,24 +727,28 @@ int t213_batch_create(const t213_tensor_desc *tensors, int32_t count, t213_batch
   {
     const char *v = getenv("T213_BATCH_SMS");
     int sms = dev_info().sms;
-    if (!B->spill.empty()) sms = std::min(sms, v && atoi(v) > 0 ? atoi(v) : 96);
+    if (!B->spill.empty() && !B->serial) sms = std::min(sms, v && atoi(v) > 0 ? atoi(v) : 96);
     B->grid = per_sm * std::max(1, sms);
   }
-  if (!B->spill.empty()) {
+  if (!B->spill.empty() && !B->serial) {
     if ((e = cudaStreamCreateWithFlags(&B->side, cudaStreamNonBlocking)) ||
         (e = cudaEventCreateWithFlags(&B->fork, cudaEventDisableTiming)) ||
         (e = cudaEventCreateWithFlags(&B->join, cudaEventDisableTiming)))
       return fail(cuda_status(e, "batch side stream"));
   }
 
-  char buf[256];
+  char buf[384];
+  int n_rounds = 0;
+  for (char c : B->in_rounds) n_rounds += c;
   int64_t direct_bytes = 0;
   for (int i : B->spill) direct_bytes += tensors[i].d1 * tensors[i].d2 * tensors[i].d3 * tensors[i].elem_bytes;
   snprintf(buf, sizeof buf,
            "batch: %d tensors, %.1f MB; one-pass slices: %d tensors; persistent kernel: %d tensors, %zu passes, %zu "
-           "items, grid %d x %d threads; graph nodes: %d tensors, %.1f MB",
-           count, B->total_bytes / 1e6, (int)B->sliced.size(), count - (int)B->spill.size() - (int)B->sliced.size(),
-           B->h_passes.size(), B->h_items.size(), B->grid, kBatchThreads, (int)B->spill.size(), direct_bytes / 1e6);
+           "items, grid %d x %d threads; graph nodes: %d tensors, %.1f MB; rounds: %d of %d tensors",
+           count, B->total_bytes / 1e6, (int)B->sliced.size(),
+           count - (int)B->spill.size() - (int)B->sliced.size() - n_rounds,
+           B->h_passes.size(), B->h_items.size(), B->grid, kBatchThreads, (int)B->spill.size(), direct_bytes / 1e6, B->rounds ? hold_rounds_count(B->rounds) : 0,
+           n_rounds);
   B->desc = buf;
   *out = B;
   return T213_OK;
@@ -715,7 +756,8 @@ int t213_batch_create(const t213_tensor_desc *tensors, int32_t count, t213_batch
 
 static int batch_enqueue(t213_batch B, cudaStream_t st) {
   cudaError_t e;
-  if (!B->spill.empty()) {  // fork: the side stream starts after the caller's earlier work
+  const bool fork = !B->spill.empty() && !B->serial;
+  if (fork) {  // fork: the side stream starts after the caller's earlier work
     if ((e = cudaEventRecord(B->fork, st)) || (e = cudaStreamWaitEvent(B->side, B->fork, 0)))
       return cuda_status(e, "batch fork");
   }
@@ -732,11 +774,15 @@ static int batch_enqueue(t213_batch B, cudaStream_t st) {
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_status(e, "k_batch launch");
   }
-  for (int i : B->spill) {
-    int rc = run_plan(*B->plans[i], (char *)B->tensors[i].data, B->side, nullptr);
+  if (B->rounds) {
+    int rc = hold_rounds_launch(B->rounds, B->d_status, st);
     if (rc) return rc;
   }
-  if (!B->spill.empty()) {  // join
+  for (int i : B->spill) {
+    int rc = run_plan(*B->plans[i], (char *)B->tensors[i].data, fork ? B->side : st, nullptr);
+    if (rc) return rc;
+  }
+  if (fork) {  // join
     if ((e = cudaEventRecord(B->join, B->side)) || (e = cudaStreamWaitEvent(st, B->join, 0)))
       return cuda_status(e, "batch join");
   }
@@ -753,10 +799,13 @@ int t213_batch_execute(t213_batch B, t213_stream_t stream) {
   // first execute on this stream: reserve what capture cannot allocate, capture
   if (!B->spill.empty()) {
     int rc = T213_OK;
-    if (B->spill_ws && !workspace(B->side, B->spill_ws, &rc)) return rc;
+    const cudaStream_t ws_stream = B->serial ? st : B->side;
+    if (B->spill_ws && !workspace(ws_stream, B->spill_ws, &rc)) return rc;
     for (int i : B->spill)
-      for (const PassDesc &q : B->plans[i]->passes)
-        if (q.table && ((rc = q.table->ensure_uploaded(B->side)) || (rc = q.table->wait_uploaded()))) return rc;
+      for (const PassDesc &q : B->plans[i]->passes) {
+        CycleTable *ct = q.table ? q.table.get() : q.ragged.table.get();
+        if (ct && ((rc = ct->ensure_uploaded(ws_stream)) || (rc = ct->wait_uploaded()))) return rc;
+      }
     int *w = device_status_word(&rc);
     if (!w) return rc;
   }
@@ -878,6 +927,7 @@ int t213_batch_destroy(t213_batch B) {
   if (B->d_status) cudaFree(B->d_status);
   if (B->d_carry) cudaFree(B->d_carry);
   if (B->d_slices) cudaFree(B->d_slices);
+  hold_rounds_destroy(B->rounds);
   if (B->side) {
     release_stream_workspace(B->side);
     cudaStreamDestroy(B->side);

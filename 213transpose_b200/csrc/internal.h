@@ -187,6 +187,16 @@ void hold_plan(HoldPlan &hp, int64_t m, int64_t n, int eb, int64_t we, int64_t d
 constexpr int kHoldNoSlot = -2;
 int launch_slice(const HoldPlan &hp, char *data, int64_t d3, int64_t m, int64_t n, int eb, int64_t we,
                  cudaStream_t st, LaunchStats *ls);
+// Slices of many tensors in rounds of one cooperative launch (the batched
+// form).  create() takes those of `which` whose slices fit a round and lists
+// them in `taken`; null without an error when there is none, or when the CTAs
+// would not all be resident.
+struct HoldRounds;
+HoldRounds *hold_rounds_create(const t213_tensor_desc *tensors, const std::vector<int> &which,
+                               std::vector<int> &taken, int *status);
+void hold_rounds_destroy(HoldRounds *r);
+int hold_rounds_count(const HoldRounds *r);
+int hold_rounds_launch(HoldRounds *r, int *status_word, cudaStream_t st);
 int64_t hold_cluster_bytes();  // shared memory of the largest team that needs no cooperative launch
 std::string describe_slice(const HoldPlan &hp);
 // Grouped one-pass slices (the batched form): the rows per CTA H and padded

@@ -418,4 +418,102 @@ __global__ void __launch_bounds__(kHoldThreads, 2)
   }
 }
 
+// ---- many tensors in rounds -------------------------------------------------------
+// The batched form: the slices of many tensors, cut into tiles, are dealt to
+// the resident CTAs in rounds.  All tiles of a slice are in one round; a CTA
+// has some tiles of every round, as many bytes as any other, in one of two
+// buffers.  One grid barrier per round (every load of the round before any of
+// its stores) is overlapped with the loads of the next round, which is in
+// other slices: the barrier's latency costs nothing while rounds are large.
+struct RoundTensor {
+  HoldArgs a;
+  char *data;
+  int32_t kind;  // element bytes, negative for the vector form
+};
+struct RoundTile {
+  uint32_t tensor, slice, tile, off;  // tile of the slice, byte offset in the buffer
+};
+
+template <int EB, int FORM>
+__device__ __noinline__ void round_load(const RoundTensor &t, const RoundTile &ti, unsigned char *buf) {
+  const HoldArgs a = t.a;  // a copy: the tile's stores must not make the compiler read it again
+  const uint32_t tr = a.tcdiv.div(ti.tile);
+  hold_load<EB, FORM>(t.data + (int64_t)ti.slice * a.slice_bytes, a, tr * a.tm, (ti.tile - tr * a.TC) * a.tn,
+                      buf + ti.off, 0);
+}
+template <int EB, int FORM>
+__device__ __noinline__ void round_store(const RoundTensor &t, const RoundTile &ti, const unsigned char *buf) {
+  const HoldArgs a = t.a;
+  const uint32_t tr = a.tcdiv.div(ti.tile);
+  char *slice = t.data + (int64_t)ti.slice * a.slice_bytes;
+  hold_store<EB, FORM>(slice, slice, a, tr * a.tm, (ti.tile - tr * a.TC) * a.tn, buf + ti.off, 0);
+}
+
+__global__ void __launch_bounds__(kHoldThreads, 2)
+    k_hold_rounds(const RoundTensor *__restrict__ tensors, const RoundTile *__restrict__ tiles,
+                  const uint32_t *__restrict__ first, uint32_t rounds, uint32_t buf_bytes, uint32_t *counter,
+                  int *status) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ int ok_s;
+  const uint32_t G = gridDim.x;
+  auto load = [&](uint32_t r) {
+    unsigned char *buf = smem_raw + (size_t)(r & 1) * buf_bytes;
+    const uint32_t q0 = first[(size_t)r * G + blockIdx.x], q1 = first[(size_t)r * G + blockIdx.x + 1];
+    for (uint32_t q = q0; q < q1; q++) {
+      const RoundTile ti = tiles[q];
+      const RoundTensor &t = tensors[ti.tensor];
+      switch (t.kind) {
+        case 1: round_load<1, HOLD_SCALAR>(t, ti, buf); break;
+        case 2: round_load<2, HOLD_SCALAR>(t, ti, buf); break;
+        case 4: round_load<4, HOLD_SCALAR>(t, ti, buf); break;
+        case 8: round_load<8, HOLD_SCALAR>(t, ti, buf); break;
+        case 16: round_load<16, HOLD_SCALAR>(t, ti, buf); break;
+        case -2: round_load<2, HOLD_VEC>(t, ti, buf); break;
+        default: round_load<4, HOLD_VEC>(t, ti, buf); break;
+      }
+    }
+  };
+  load(0);
+  for (uint32_t r = 0; r < rounds; r++) {
+    cp_async_wait_all();
+    __syncthreads();  // this CTA's loads of round r have landed, its stores of round r - 1 are issued
+    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
+    if (r + 1 < rounds) load(r + 1);
+    if (threadIdx.x == 0) {
+      const uint32_t target = (r + 1) * G;
+      const uint64_t t0 = global_ns();
+      uint32_t spins = 0;
+      int ok = 1;
+      while (ld_acquire_u32(counter) < target) {
+        if ((++spins & 1023u) == 0 && global_ns() - t0 > kWaitNs) {
+          ok = 0;
+          break;
+        }
+      }
+      ok_s = ok;
+    }
+    __syncthreads();
+    if (!ok_s) {
+      cp_async_wait_all();
+      if (threadIdx.x == 0) atomicExch(status, 5 /* T213_ERR_TIMEOUT */);
+      return;
+    }
+    const unsigned char *buf = smem_raw + (size_t)(r & 1) * buf_bytes;
+    const uint32_t q0 = first[(size_t)r * G + blockIdx.x], q1 = first[(size_t)r * G + blockIdx.x + 1];
+    for (uint32_t q = q0; q < q1; q++) {
+      const RoundTile ti = tiles[q];
+      const RoundTensor &t = tensors[ti.tensor];
+      switch (t.kind) {
+        case 1: round_store<1, HOLD_SCALAR>(t, ti, buf); break;
+        case 2: round_store<2, HOLD_SCALAR>(t, ti, buf); break;
+        case 4: round_store<4, HOLD_SCALAR>(t, ti, buf); break;
+        case 8: round_store<8, HOLD_SCALAR>(t, ti, buf); break;
+        case 16: round_store<16, HOLD_SCALAR>(t, ti, buf); break;
+        case -2: round_store<2, HOLD_VEC>(t, ti, buf); break;
+        default: round_store<4, HOLD_VEC>(t, ti, buf); break;
+      }
+    }
+  }
+}
+
 }  // namespace t213

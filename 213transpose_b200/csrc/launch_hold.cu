@@ -285,11 +285,7 @@ std::string describe_slice(const HoldPlan &hp) {
 
 namespace {
 
-int hold_prepare(HoldReady::Form &f, const HoldGeom &g, int64_t m, int64_t n, int eb, int64_t we) {
-  int status = T213_OK;
-  f.status = device_status_word(&status);
-  if (!f.status) return status;
-  HoldArgs &a = f.args;
+void hold_args(HoldArgs &a, const HoldGeom &g, int64_t m, int64_t n, int eb, int64_t we) {
   a.slice_bytes = m * n * eb * we;
   a.m = (uint32_t)m;
   a.n = (uint32_t)n;
@@ -318,7 +314,14 @@ int hold_prepare(HoldReady::Form &f, const HoldGeom &g, int64_t m, int64_t n, in
     a.lgs = lanes_log2(words);
     a.rbdiv = FastDiv<uint32_t>((uint64_t)(words + (1 << a.lgs) - 1) >> a.lgs);
   }
-  f.smem = (int64_t)g.S * a.tile_bytes;
+}
+
+int hold_prepare(HoldReady::Form &f, const HoldGeom &g, int64_t m, int64_t n, int eb, int64_t we) {
+  int status = T213_OK;
+  f.status = device_status_word(&status);
+  if (!f.status) return status;
+  hold_args(f.args, g, m, n, eb, we);
+  f.smem = (int64_t)g.S * f.args.tile_bytes;
   switch (g.form == HOLD_WIDE ? 0 : g.form == HOLD_VEC ? -eb : g.form == HOLD_RAG_DST ? 100 + eb
           : g.form == HOLD_RAG_SRC ? 200 + eb : eb) {
     case 101:
@@ -523,6 +526,220 @@ int launch_slice(const HoldPlan &hp, char *data, int64_t d3, int64_t m, int64_t 
   if (rc) return rc;
   if (ls) ls->launches++;
   return T213_OK;
+}
+
+// ---- rounds ------------------------------------------------------------------------
+struct HoldRounds {
+  RoundTensor *d_tensors = nullptr;
+  RoundTile *d_tiles = nullptr;
+  uint32_t *d_first = nullptr, *d_counter = nullptr;
+  uint32_t rounds = 0, buf_bytes = 0, ctas = 0;
+};
+
+namespace {
+
+// Slices of more than this share of a round run their own plan, which has
+// twice the room.  Measured on B200, shares of 0.35 / 0.5 / 0.75, us: batches
+// of 64 tensors (630 MB) 405 / 404 / 421 and 457 / 453 / 460, of 512 tensors
+// 6372 / 6346 / 6458.
+constexpr double kRoundShare = 0.5;
+
+// Tiles of at most `cap` bytes with the least work: bytes with their padding,
+// a sector more per row piece, and idle lanes.
+bool round_tiling(HoldGeom &g, int64_t m, int64_t n, int eb, int form, int64_t cap) {
+  const int64_t Q = form == HOLD_VEC ? 16 / eb : 1;
+  const int64_t un = std::max<int64_t>(Q, (n * eb) % 32 == 0 ? 32 / std::min(eb, 32) : 1);
+  const int64_t um = std::max<int64_t>(Q, (m * eb) % 32 == 0 ? 32 / std::min(eb, 32) : 1);
+  double best = 1e30;
+  g.ok = false;
+  for (int64_t TC = 1; TC <= n; TC = TC < 64 ? TC + 1 : TC + TC / 16) {
+    const int64_t tn = std::min(n, up((n + TC - 1) / TC, un)), tcs = (n + tn - 1) / tn;
+    if (tn * eb < 64 && tn < n) break;
+    const bool packed = tcs == 1 && hold_packed(n, eb, form);
+    const int64_t P = packed ? n * eb : hold_pitch(tn, eb, 1, form);
+    auto fits = [&](int64_t tm) { return hold_tile_bytes(tm, tn, P, eb, form, packed) <= cap; };
+    int64_t tm = std::min(m, std::max<int64_t>(1, cap / P));
+    while (tm > 1 && !fits(tm)) tm--;
+    if (!fits(tm)) continue;
+    if (tm < m && tm > um) tm = tm / um * um;
+    tm = tm / Q * Q;
+    if (tm < 1) continue;
+    const int64_t trs = (m + tm - 1) / tm;
+    tm = std::min(tm, up((m + trs - 1) / trs, um));
+    const int64_t N = eb < 4 ? 4 / eb : 1, wd = form == HOLD_VEC ? 32 : (tm + N - 1) / N;
+    const double idle = wd >= 32 ? 0.5 * (double)(up(wd, 32) - wd) / (double)wd : 0.0;
+    const double c = (double)trs * tm * tcs * tn * eb * (idle + 2.0 + 32.0 / (tn * eb) + 32.0 / (tm * eb)) +
+                     (double)trs * tcs * 2048;  // a tile costs about as much as 2 KB more
+    if (c < best) {
+      best = c;
+      g.ok = true;
+      g.tm = (uint32_t)tm;
+      g.tn = (uint32_t)tn;
+      g.TC = (uint32_t)tcs;
+      g.T = (uint32_t)(trs * tcs);
+      g.ctas = g.teams = g.S = 1;
+      g.P = (uint32_t)P;
+      g.packed = packed;
+      g.mode = HOLD_GRID;
+      g.form = form;
+    }
+  }
+  return g.ok;
+}
+
+}  // namespace
+
+void hold_rounds_destroy(HoldRounds *r) {
+  if (!r) return;
+  cudaFree(r->d_tensors);
+  cudaFree(r->d_tiles);
+  cudaFree(r->d_first);
+  cudaFree(r->d_counter);
+  delete r;
+}
+
+HoldRounds *hold_rounds_create(const t213_tensor_desc *tensors, const std::vector<int> &which,
+                               std::vector<int> &taken, int *status) {
+  *status = T213_OK;
+  taken.clear();
+  const int64_t buf = hold_budget() / 2 / 128 * 128;
+  const int sms = dev_info().sms;
+  const uint32_t G = (uint32_t)(2 * sms);
+  const int64_t smem = 2 * buf;
+  if (!kernel_attr_once((const void *)k_hold_rounds, smem, 1)) {
+    *status = cuda_status(cudaGetLastError(), "cudaFuncSetAttribute(rounds)");
+    return nullptr;
+  }
+  int per_sm = 0;
+  occupancy_cached((const void *)k_hold_rounds, kHoldThreads, smem, 1, &per_sm);
+  if (per_sm < 2) return nullptr;
+  struct Slice {
+    uint32_t tensor, slice, T;
+    int64_t bytes;  // of one tile's buffer space
+    int64_t total;
+  };
+  std::vector<RoundTensor> ts;
+  std::vector<Slice> slices;
+  for (int i : which) {
+    const t213_tensor_desc &d = tensors[i];
+    const int eb = d.elem_bytes;
+    const bool vec = (eb == 2 || eb == 4) && (d.d1 * eb) % 16 == 0 && (d.d2 * eb) % 16 == 0 && (uintptr_t)d.data % 16 == 0;
+    const int64_t sb = d.d1 * d.d2 * eb;
+    HoldGeom g;
+    // small slices take tiles of half a buffer, so that tiles of several fit
+    if (d.d1 > (1 << 30) || d.d2 > (1 << 30) ||
+        !round_tiling(g, d.d2, d.d1, eb, vec ? HOLD_VEC : HOLD_SCALAR, sb < (2 << 20) ? buf / 2 : buf))
+      continue;
+    RoundTensor t{};
+    hold_args(t.a, g, d.d2, d.d1, eb, 1);
+    if ((int64_t)g.T > (int64_t)G * (buf / t.a.tile_bytes)) continue;  // more tiles than a round has places
+    if (sb > (int64_t)(kRoundShare * (double)G * (double)buf)) continue;
+    t.data = (char *)d.data;
+    t.kind = vec ? -eb : eb;
+    for (int64_t k = 0; k < d.d3; k++)
+      slices.push_back(Slice{(uint32_t)ts.size(), (uint32_t)k, g.T, (int64_t)t.a.tile_bytes, (int64_t)g.T * t.a.tile_bytes});
+    ts.push_back(t);
+    taken.push_back(i);
+  }
+  if (ts.empty()) return nullptr;
+  // Rounds: the largest slice left opens one, smaller ones fill it; every tile
+  // goes to the CTA with the least in its buffer.
+  std::stable_sort(slices.begin(), slices.end(), [](const Slice &a, const Slice &b) { return a.total > b.total; });
+  std::vector<RoundTile> tiles;
+  std::vector<uint32_t> first;
+  std::vector<std::vector<RoundTile>> mine(G);
+  std::vector<int64_t> used(G);
+  std::vector<char> done(slices.size(), 0);
+  size_t lo = 0;
+  const int64_t capacity = (int64_t)G * buf;
+  while (lo < slices.size()) {
+    for (uint32_t c = 0; c < G; c++) {
+      mine[c].clear();
+      used[c] = 0;
+    }
+    std::vector<std::pair<int64_t, uint32_t>> heap;  // (bytes used, CTA), least first
+    for (uint32_t c = 0; c < G; c++) heap.push_back({0, c});
+    auto gt = [](const std::pair<int64_t, uint32_t> &a, const std::pair<int64_t, uint32_t> &b) { return a > b; };
+    std::make_heap(heap.begin(), heap.end(), gt);
+    int64_t filled = 0;
+    int misses = 0;
+    for (size_t i = lo; i < slices.size() && misses < 16; i++) {
+      if (done[i]) continue;
+      const Slice &s = slices[i];
+      if (filled + s.total > capacity) {
+        misses++;
+        continue;
+      }
+      // all tiles or none: the least full CTA has room for one more as long as
+      // any has, so they all fit when the free places are enough
+      int64_t places = 0;
+      for (uint32_t c = 0; c < G && places < s.T; c++) places += (buf - used[c]) / s.bytes;
+      if (places < s.T) {
+        misses++;
+        continue;
+      }
+      for (uint32_t t = 0; t < s.T; t++) {
+        std::pop_heap(heap.begin(), heap.end(), gt);
+        auto &top = heap.back();
+        mine[top.second].push_back(RoundTile{s.tensor, s.slice, t, (uint32_t)top.first});
+        top.first += s.bytes;
+        used[top.second] = top.first;
+        std::push_heap(heap.begin(), heap.end(), gt);
+      }
+      filled += s.total;
+      done[i] = 1;
+    }
+    for (uint32_t c = 0; c < G; c++) {
+      first.push_back((uint32_t)tiles.size());
+      tiles.insert(tiles.end(), mine[c].begin(), mine[c].end());
+    }
+    const size_t was = lo;
+    while (lo < slices.size() && done[lo]) lo++;
+    if (lo == was) {  // cannot happen: an empty round takes every slice that was admitted
+      set_error("batch rounds: a slice fits no round");
+      *status = T213_ERR_UNSUPPORTED;
+      return nullptr;
+    }
+  }
+  first.push_back((uint32_t)tiles.size());
+  auto *r = new HoldRounds();
+  r->rounds = (uint32_t)((first.size() - 1) / G);
+  r->buf_bytes = (uint32_t)buf;
+  r->ctas = G;
+  cudaError_t e = cudaMalloc(&r->d_tensors, ts.size() * sizeof(RoundTensor));
+  if (!e) e = cudaMalloc(&r->d_tiles, tiles.size() * sizeof(RoundTile));
+  if (!e) e = cudaMalloc(&r->d_first, first.size() * sizeof(uint32_t));
+  if (!e) e = cudaMalloc(&r->d_counter, 256);
+  if (!e) e = cudaMemcpy(r->d_tensors, ts.data(), ts.size() * sizeof(RoundTensor), cudaMemcpyHostToDevice);
+  if (!e) e = cudaMemcpy(r->d_tiles, tiles.data(), tiles.size() * sizeof(RoundTile), cudaMemcpyHostToDevice);
+  if (!e) e = cudaMemcpy(r->d_first, first.data(), first.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
+  if (!e) e = cudaStreamSynchronize(0);  // the copies landed before any stream's launch
+  if (e) {
+    *status = cuda_status(e, "batch rounds");
+    hold_rounds_destroy(r);
+    return nullptr;
+  }
+  return r;
+}
+
+int hold_rounds_count(const HoldRounds *r) { return (int)r->rounds; }
+
+int hold_rounds_launch(HoldRounds *r, int *status_word, cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(r->d_counter, 0, sizeof(uint32_t), st);
+  if (e != cudaSuccess) return cuda_status(e, "batch rounds counter");
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(r->ctas, 1, 1);
+  cfg.blockDim = dim3(kHoldThreads, 1, 1);
+  cfg.dynamicSmemBytes = 2 * (size_t)r->buf_bytes;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  e = cudaLaunchKernelEx(&cfg, k_hold_rounds, (const RoundTensor *)r->d_tensors, (const RoundTile *)r->d_tiles,
+                         (const uint32_t *)r->d_first, r->rounds, r->buf_bytes, r->d_counter, status_word);
+  return e == cudaSuccess ? T213_OK : cuda_status(e, "k_hold_rounds launch");
 }
 
 }  // namespace t213
