@@ -170,7 +170,7 @@ int64_t band_smem_bytes(int64_t R, int64_t C, int eb);
 enum HoldMode { HOLD_CTA = 0, HOLD_CLUSTER = 1, HOLD_GRID = 2 };  // a team: one CTA, a cluster, more CTAs
 struct HoldGeom {
   bool ok = false;
-  bool packed = false;
+  bool packed = false, tmem = false;
   int mode = 0, form = 0;
   uint32_t tm = 0, tn = 0, TC = 0, T = 0, ctas = 0, teams = 0, S = 0, P = 0;
   double est_us = 0;  // modelled time of the launch

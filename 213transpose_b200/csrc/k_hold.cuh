@@ -46,6 +46,7 @@ struct HoldArgs {
   uint32_t ctas, teams, S;  // CTAs per team, teams, tiles per CTA (at most)
   uint32_t P, H, tile_bytes;  // shared-memory row pitch, region and tile size
   int32_t packed;             // narrow rows, one contiguous piece per tile
+  int32_t bulk;               // row pieces come by bulk copies
   int32_t mode, slot;
   int32_t lgs;  // log2 of the lanes that share an output column
   uint32_t we;       // wide form: 16-byte words per element
@@ -85,11 +86,29 @@ __device__ __forceinline__ uint32_t hold_row(const HoldArgs &a, uint32_t i, uint
   }
 }
 
+// Adds bytes that bulk copies will bring to what the barrier waits for.
+__device__ __forceinline__ void mbar_expect(uint64_t *mb, uint32_t bytes) {
+  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(mb)), "r"(bytes) : "memory");
+}
+// After a warp's last load of an item: the barrier's phase ends when every
+// warp has come here and every announced byte has landed.
+__device__ __forceinline__ void hold_loaded(uint64_t *mb) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(mb);
+}
+// Waits, bounded, for an item's loads of either kind.
+__device__ __forceinline__ bool hold_landed(uint64_t *mb, uint32_t &phase) {
+  cp_async_wait_all();
+  const bool ok = mbar_wait(mb, phase);
+  phase ^= 1u;
+  return __syncthreads_and(ok);
+}
+
 // `slice` is the slice, or the band's rows (RAG_DST), or the start of the
 // slice that the band belongs to (RAG_SRC, with s0 the band's first segment).
-template <int EB, int FORM>
+template <int EB, int FORM, uint32_t THREADS = kHoldThreads>
 __device__ __forceinline__ void hold_load(const char *slice, const HoldArgs &a, uint32_t r0, uint32_t c0,
-                                          unsigned char *s, uint32_t s0) {
+                                          unsigned char *s, uint32_t s0, uint64_t *mb) {
   uint32_t rows = min(a.tm, a.m - r0), cols = min(a.tn, a.n - c0);
   const uint32_t E = EB * (FORM == HOLD_WIDE ? a.we : 1);
   const uint32_t pitch = a.n * E;  // a slice is far below 4 GB
@@ -99,13 +118,28 @@ __device__ __forceinline__ void hold_load(const char *slice, const HoldArgs &a, 
     const char *g = g0 - sh;
     const uint32_t nc = (sh + rows * pitch + 15) >> 4;
 #pragma unroll 4
-    for (uint32_t c = threadIdx.x; c < nc; c += kHoldThreads) cp_async<16>(s + c * 16, g + c * 16);
+    for (uint32_t c = threadIdx.x; c < nc; c += THREADS) cp_async<16>(s + c * 16, g + c * 16);
     return;
   }
-  // thread t takes blocks t, t + 512, ... of the tile's rows x nc blocks and
+  if (FORM != HOLD_VEC && FORM != HOLD_WIDE && a.bulk) {
+    // row pieces long enough for a bulk copy each: one thread a row
+    constexpr uint32_t N = EB < 4 ? 4 / EB : 1;
+    for (uint32_t base = threadIdx.x & ~31u; base < rows; base += THREADS) {
+      const uint32_t i = base + (threadIdx.x & 31);
+      const char *g = g0 + (FORM == HOLD_RAG_SRC ? (size_t)a.seg_at(s0 + r0 + min(i, rows - 1)) : (size_t)(i * pitch));
+      const uint32_t sh = (uint32_t)(uintptr_t)g & 15u, l = i / N, b = i % N;
+      const uint32_t bytes = i < rows ? (sh + cols * EB + 15) & ~15u : 0;
+      const uint32_t sum = __reduce_add_sync(0xffffffffu, bytes);
+      if ((threadIdx.x & 31) == 0) mbar_expect(mb, sum);
+      __syncwarp();
+      if (bytes) bulk_g2s(s + b * a.H + l * a.P + (l >> 3) * 16, g - sh, bytes, mb);
+    }
+    return;
+  }
+  // thread t takes blocks t, t + THREADS, ... of the tile's rows x nc blocks and
   // carries (row, block) along: no lane idles at a row's end
   const uint32_t nc = FORM == HOLD_VEC ? cols * EB / 16 : FORM == HOLD_WIDE ? cols * a.we : (cols * EB + 31 - EB) / 16;
-  const uint32_t di = kHoldThreads / nc, dc = kHoldThreads - di * nc;
+  const uint32_t di = THREADS / nc, dc = THREADS - di * nc;
   uint32_t i = threadIdx.x / nc, c = threadIdx.x - i * nc;
 #pragma unroll 4
   for (; i < rows;) {
@@ -219,8 +253,13 @@ __device__ __forceinline__ void hold_store(char *slice, const char *from, const 
         }
         char *g = slice + (size_t)(o + w * EB);
         if (left >= U) {
+          if (a.lgs == 5) {  // consecutive columns: reads at constant offsets
 #pragma unroll
-          for (uint32_t q = 0; q < U; q++) v[q] = *reinterpret_cast<const E *>(p + q * ps);
+            for (uint32_t q = 0; q < U; q++) v[q] = *reinterpret_cast<const E *>(p + q * EB);
+          } else {
+#pragma unroll
+            for (uint32_t q = 0; q < U; q++) v[q] = *reinterpret_cast<const E *>(p + q * ps);
+          }
 #pragma unroll
           for (uint32_t q = 0; q < U; q++, g += gs) *reinterpret_cast<E *>(g) = v[q];
         } else {
@@ -229,18 +268,31 @@ __device__ __forceinline__ void hold_store(char *slice, const char *from, const 
             if (q < left) *reinterpret_cast<E *>(g + (size_t)(q * gs)) = *reinterpret_cast<const E *>(p + q * ps);
         }
       } else if constexpr (FORM == HOLD_RAG_DST) {
-        // the offset of an output row is its own: column by column
+        // the offset of an output row in its first word is the column's own:
+        // the N rows of the word are picked out of the 2 N - 1 that they can be
+        uint32_t ro[2 * N - 1];
+#pragma unroll
+        for (uint32_t b = 0; b < 2 * N - 1; b++)
+          ro[b] = hold_row<EB, FORM>(a, min((uint32_t)max((int32_t)(w * N + b) - (int32_t)(N - 1), 0), rows - 1), lo, plo, sr);
+        const uint32_t sj = s0 + c0 + j0;
+        char *g0 = slice + (size_t)(r0 * EB);
+#pragma unroll 4
         for (uint32_t q = 0; q < min(left, U); q++) {
-          char *g = slice + a.seg_at(s0 + c0 + j0 + q * (G * N)) + (size_t)(r0 * EB);
-          const uint32_t h = ((uint32_t)(uintptr_t)g & 3u) / EB;
-          const int32_t e0 = (int32_t)(w * N) - (int32_t)h;
+          char *g = g0 + a.seg_at(sj + q * (G * N));
+          const uint32_t h = ((uint32_t)(uintptr_t)g & 3u) / EB, at = N - 1 - h;
+          uint32_t x[2 * N - 1];
+#pragma unroll
+          for (uint32_t b = 0; b < 2 * N - 1; b++) x[b] = ro[b];
+#pragma unroll
+          for (uint32_t k = 1; k < N; k *= 2) {
+#pragma unroll
+            for (uint32_t b = 0; b + k < 2 * N - 1; b++) x[b] = at & k ? x[b + k] : x[b];
+          }
+          const unsigned char *p = s + j0 * EB + q * ps;
           uint32_t v = 0;
 #pragma unroll
-          for (uint32_t b = 0; b < N; b++)
-            v |= (uint32_t) * reinterpret_cast<const E *>(
-                     s + hold_row<EB, FORM>(a, min((uint32_t)max(e0 + (int32_t)b, 0), rows - 1), lo, plo, sr) +
-                     j0 * EB + q * ps)
-                 << (8 * EB * b);
+          for (uint32_t b = 0; b < N; b++) v |= (uint32_t) * reinterpret_cast<const E *>(p + x[b]) << (8 * EB * b);
+          const int32_t e0 = (int32_t)(w * N) - (int32_t)h;
           g += (int64_t)e0 * EB;
           if (e0 >= 0 && e0 + (int32_t)N <= (int32_t)rows) {
             *reinterpret_cast<uint32_t *>(g) = v;
@@ -303,14 +355,7 @@ __device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t *p) {
   return v;
 }
 
-__device__ __forceinline__ bool hold_grid_arrive_wait(uint32_t *bar, uint32_t ctas, uint32_t gen) {
-  uint32_t old;
-  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(bar) : "memory");
-  if (old == ctas - 1) {
-    asm volatile("st.relaxed.gpu.global.u32 [%0], 0;" ::"l"(bar) : "memory");
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(bar + 1), "r"(gen + 1) : "memory");
-    return true;
-  }
+__device__ __forceinline__ bool hold_grid_wait(uint32_t *bar, uint32_t ctas, uint32_t gen) {
   const uint64_t t0 = global_ns();
   uint32_t spins = 0;
   while (ld_acquire_u32(bar + 1) == gen) {
@@ -331,14 +376,31 @@ __device__ __forceinline__ bool hold_grid_arrive_wait(uint32_t *bar, uint32_t ct
   return true;
 }
 
+// Arrives; true when this was the last arrival, which also ends the barrier.
+__device__ __forceinline__ bool hold_grid_arrive(uint32_t *bar, uint32_t ctas, uint32_t gen) {
+  uint32_t old;
+  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(bar) : "memory");
+  if (old != ctas - 1) return false;
+  asm volatile("st.relaxed.gpu.global.u32 [%0], 0;" ::"l"(bar) : "memory");
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(bar + 1), "r"(gen + 1) : "memory");
+  return true;
+}
+
 template <int EB, int FORM>
 __global__ void __launch_bounds__(kHoldThreads, 2)
     k_hold(char *__restrict__ data, const __grid_constant__ HoldArgs a, uint32_t *bars, int *status) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ int ok_s;
+  __shared__ uint64_t mb;
   const uint32_t team = blockIdx.x / a.ctas, rank = blockIdx.x - team * a.ctas;
   int64_t k = team;
   if (k >= a.d3) return;
+  if (threadIdx.x == 0) {
+    mbar_init(&mb, kHoldThreads / 32);
+    fence_barrier_init();
+  }
+  __syncthreads();
+  uint32_t phase = 0;
   uint32_t *bar = bars ? bars + ((size_t)a.slot * kHoldTeams + team) * 8 : nullptr;
   uint32_t gen = 0;
   if (a.mode == HOLD_GRID && threadIdx.x == 0) gen = ld_relaxed_u32(bar + 1);
@@ -375,18 +437,23 @@ __global__ void __launch_bounds__(kHoldThreads, 2)
     for (uint32_t t = rank; t < a.T; t += a.ctas, q++) {
       uint32_t r0, c0;
       tile_pos(t, r0, c0);
-      hold_load<EB, FORM>(from, a, r0, c0, smem_raw + (size_t)q * a.tile_bytes, s0);
+      hold_load<EB, FORM>(from, a, r0, c0, smem_raw + (size_t)q * a.tile_bytes, s0, &mb);
     }
+    hold_loaded(&mb);
   }
   for (;;) {
-    cp_async_wait_all();
-    __syncthreads();  // the CTA's tiles have landed
+    // the CTA's tiles have landed; a copy that never does is reported, and
+    // the team's other CTAs run out of the same patience at their barrier
+    if (!hold_landed(&mb, phase)) {
+      if (threadIdx.x == 0) atomicExch(status, 5 /* T213_ERR_TIMEOUT */);
+      return;
+    }
     if (a.mode == HOLD_CLUSTER) {
       // execution order only: every thread has waited for its own copies
       asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
     } else if (a.mode == HOLD_GRID) {
       if (threadIdx.x == 0) {
-        ok_s = hold_grid_arrive_wait(bar, a.ctas, gen);
+        ok_s = hold_grid_arrive(bar, a.ctas, gen) || hold_grid_wait(bar, a.ctas, gen);
         gen++;
       }
       __syncthreads();
@@ -407,15 +474,271 @@ __global__ void __launch_bounds__(kHoldThreads, 2)
       hold_store<EB, FORM>(slice, from, a, r0, c0, buf, s0);
       if (next < a.d3) {
         __syncthreads();  // every thread has read the tile: the next item's may land
-        hold_load<EB, FORM>(nfrom, a, r0, c0, buf, ns0);
+        fence_proxy_async();
+        hold_load<EB, FORM>(nfrom, a, r0, c0, buf, ns0, &mb);
       }
     }
+    if (next < a.d3) hold_loaded(&mb);
     if (next >= a.d3) break;
     k = next;
     slice = nslice;
     from = nfrom;
     s0 = ns0;
   }
+}
+
+// ---- several slices per team: tensor memory as the second buffer -----------------
+// A team that takes one slice after the other would have to wait for the
+// barrier with nothing in flight once its tile fills the shared memory.  Here
+// a landed tile moves on to the SM's tensor memory (TMEM, 256 KB beside the
+// shared memory) before the barrier, in the order in which it will be written:
+// lane l of a warp's quarter holds output word l of a column, successive TMEM
+// columns successive matrix columns, so that a 32x32b load hands every lane
+// the words it writes and the transposition costs no second pass.  The shared
+// memory is free at once: the next slice's loads are in flight during the
+// barrier and the stores.  TMEM is used as memory only; a warp reads back what
+// it wrote itself.
+//
+// One CTA of 1024 threads per SM: a kernel that allocates tensor memory is
+// resident once per SM, whatever its size.
+constexpr int kTmemThreads = 1024;
+constexpr int kTmemCols = 512;
+constexpr int kTmemUnitCols = 16;  // one unit: 16 words per lane
+constexpr int kTmemWarpCols = kTmemCols / (kTmemThreads / 128);  // 8 warps share a quarter's lanes
+constexpr int kTmemUnits = kTmemWarpCols / kTmemUnitCols;        // per warp
+
+__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16};" ::"r"(addr),
+      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+      "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
+      "[%16];\n\ttcgen05.wait::ld.sync.aligned;"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(addr)
+      : "memory");
+}
+
+// The units of hold_store's scalar form with 16 words per lane.
+template <int EB>
+struct TmemUnit {
+  static constexpr uint32_t N = EB < 4 ? 4 / EB : 1;
+  static constexpr uint32_t W = EB < 4 ? 1 : EB / 4;  // words per element
+  static constexpr uint32_t U = kTmemUnitCols / W;    // column steps
+  uint32_t w, j0, left, gn;  // word, first column, column steps left (0: idle lane), columns per step
+  __device__ __forceinline__ TmemUnit(const HoldArgs &a, uint32_t u, uint32_t rows, uint32_t cols, uint32_t lane) {
+    const uint32_t L = 1u << a.lgs, G = 32u >> a.lgs, li = lane & (L - 1), sub = lane >> a.lgs;
+    const uint32_t words = N == 1 ? rows : (rows + 2 * N - 2) / N;
+    const uint32_t nrb = (words + L - 1) >> a.lgs;
+    const uint32_t cg = rows == a.tm ? a.rbdiv.div(u) : u / nrb;
+    w = ((u - cg * nrb) << a.lgs) + li;
+    gn = G * N;
+    j0 = cg / N * (U * gn) + cg % N * G + sub;
+    left = w < words && j0 < cols ? min((cols - 1 - j0) / gn + 1, U) : 0;
+  }
+  __device__ static __forceinline__ uint32_t count(const HoldArgs &a, uint32_t rows, uint32_t cols) {
+    const uint32_t L = 1u << a.lgs, G = 32u >> a.lgs;
+    const uint32_t words = N == 1 ? rows : (rows + 2 * N - 2) / N;
+    return ((words + L - 1) >> a.lgs) * ((cols + U * G * N - 1) / (U * G * N) * N);
+  }
+};
+
+template <int EB, int FORM>
+__device__ __forceinline__ void tmem_fill(const char *slice, const char *from, const HoldArgs &a, uint32_t r0,
+                                          uint32_t c0, const unsigned char *s, uint32_t s0, uint32_t taddr) {
+  using E = typename ElemT<EB>::type;
+  using TU = TmemUnit<EB>;
+  const uint32_t rows = min(a.tm, a.m - r0), cols = min(a.tn, a.n - c0);
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t plo = a.n * EB;
+  const uint32_t lo = (uint32_t)(uintptr_t)from + (FORM == HOLD_RAG_SRC ? c0 * EB : (r0 * a.n + c0) * EB);
+  const uint32_t sr = s0 + r0;
+  const uint32_t units = TU::count(a, rows, cols);
+  for (uint32_t u = warp; u < units; u += kTmemThreads / 32, taddr += kTmemUnitCols) {
+    const TU t(a, u, rows, cols, lane);
+    union {
+      uint32_t w[16];
+      E e[TU::U];
+    } v;
+    if constexpr (TU::N == 1) {
+      const unsigned char *p = s + hold_row<EB, FORM>(a, min(t.w, rows - 1), lo, plo, sr) + t.j0 * EB;
+#pragma unroll
+      for (uint32_t q = 0; q < TU::U; q++)
+        if (q < t.left) v.e[q] = *reinterpret_cast<const E *>(p + q * t.gn * EB);
+    } else {
+      const uint32_t h = (((uint32_t)(uintptr_t)slice + ((c0 + t.j0) * a.m + r0) * EB) & 3u) / EB;
+      const int32_t e0 = (int32_t)(t.w * TU::N) - (int32_t)h;
+      const unsigned char *p[TU::N];
+#pragma unroll
+      for (uint32_t b = 0; b < TU::N; b++)
+        p[b] = s + hold_row<EB, FORM>(a, min((uint32_t)max(e0 + (int32_t)b, 0), rows - 1), lo, plo, sr) + t.j0 * EB;
+#pragma unroll
+      for (uint32_t q = 0; q < 16; q++) {
+        v.w[q] = 0;
+        if (q < t.left) {
+#pragma unroll
+          for (uint32_t b = 0; b < TU::N; b++)
+            v.w[q] |= (uint32_t) * reinterpret_cast<const E *>(p[b] + q * t.gn * EB) << (8 * EB * b);
+        }
+      }
+    }
+    __syncwarp();
+    tmem_st16(taddr, v.w);
+  }
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+template <int EB, int FORM>
+__device__ __forceinline__ void tmem_drain(char *slice, const HoldArgs &a, uint32_t r0, uint32_t c0, uint32_t s0,
+                                           uint32_t taddr) {
+  using E = typename ElemT<EB>::type;
+  using TU = TmemUnit<EB>;
+  const uint32_t rows = min(a.tm, a.m - r0), cols = min(a.tn, a.n - c0);
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t units = TU::count(a, rows, cols);
+  for (uint32_t u = warp; u < units; u += kTmemThreads / 32, taddr += kTmemUnitCols) {
+    const TU t(a, u, rows, cols, lane);
+    union {
+      uint32_t w[16];
+      E e[TU::U];
+    } v;
+    __syncwarp();
+    tmem_ld16(taddr, v.w);
+    if constexpr (FORM == HOLD_RAG_DST) {
+      static_assert(TU::N == 1, "the byte offset of an output row is its own");
+      char *g = slice + (size_t)((r0 + t.w) * EB);
+      const uint32_t sj = s0 + c0 + t.j0;
+#pragma unroll
+      for (uint32_t q = 0; q < TU::U; q++)
+        if (q < t.left) *reinterpret_cast<E *>(g + a.seg_at(sj + q * t.gn)) = v.e[q];
+    } else {
+      const uint32_t o = ((c0 + t.j0) * a.m + r0) * EB, gs = t.gn * a.m * EB;
+      if constexpr (TU::N == 1) {
+        char *g = slice + (size_t)(o + t.w * EB);
+#pragma unroll
+        for (uint32_t q = 0; q < TU::U; q++, g += gs)
+          if (q < t.left) *reinterpret_cast<E *>(g) = v.e[q];
+      } else {
+        const uint32_t h = (((uint32_t)(uintptr_t)slice + o) & 3u) / EB;
+        const int32_t e0 = (int32_t)(t.w * TU::N) - (int32_t)h;
+        char *g = slice + (size_t)o + (int64_t)e0 * EB;
+        if (e0 >= 0 && e0 + (int32_t)TU::N <= (int32_t)rows) {
+#pragma unroll
+          for (uint32_t q = 0; q < 16; q++, g += gs)
+            if (q < t.left) *reinterpret_cast<uint32_t *>(g) = v.w[q];
+        } else {
+#pragma unroll
+          for (uint32_t b = 0; b < TU::N; b++)
+            if ((uint32_t)(e0 + (int32_t)b) < rows) {
+#pragma unroll
+              for (uint32_t q = 0; q < 16; q++)
+                if (q < t.left) *reinterpret_cast<E *>(g + (size_t)(q * gs) + b * EB) = (E)(v.w[q] >> (8 * EB * b));
+            }
+        }
+      }
+    }
+  }
+}
+
+template <int EB, int FORM>
+__global__ void __launch_bounds__(kTmemThreads, 1)
+    k_hold_tmem(char *__restrict__ data, const __grid_constant__ HoldArgs a, uint32_t *bars, int *status) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ int ok_s;
+  __shared__ uint32_t tbase_s;
+  __shared__ uint64_t mb;
+  if (threadIdx.x == 0) {
+    mbar_init(&mb, kTmemThreads / 32);
+    fence_barrier_init();
+  }
+  uint32_t phase = 0;
+  const uint32_t team = blockIdx.x / a.ctas, rank = blockIdx.x - team * a.ctas;
+  int64_t k = team;
+  const uint32_t warp = threadIdx.x >> 5;
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tbase_s)),
+                 "n"(kTmemCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  uint32_t *bar = bars + ((size_t)a.slot * kHoldTeams + team) * 8;
+  uint32_t gen = 0;
+  if (threadIdx.x == 0) gen = ld_relaxed_u32(bar + 1);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tbase = tbase_s;
+  // a warp reaches the 32 lanes of its quarter; the 8 warps of a quarter have
+  // an eighth of the columns each
+  const uint32_t taddr = tbase + ((warp & 3u) << 21) + (warp >> 2) * kTmemWarpCols;
+  const bool mine = rank < a.T;
+  const uint32_t tr = a.tcdiv.div(rank), r0 = tr * a.tm, c0 = (rank - tr * a.TC) * a.tn;
+  auto item = [&](int64_t kk, char *&slice, char *&from, uint32_t &s0) {
+    if constexpr (FORM == HOLD_RAG_DST || FORM == HOLD_RAG_SRC) {  // as in k_hold
+      const int64_t sl = kk / a.nb;
+      const uint32_t b = FORM == HOLD_RAG_DST ? a.nb - 1 - (uint32_t)(kk - sl * a.nb) : (uint32_t)(kk - sl * a.nb);
+      const size_t band = (size_t)b * a.m * a.n * EB;
+      char *base = data + sl * a.slice_bytes;
+      slice = FORM == HOLD_RAG_DST ? base : base + band;
+      from = FORM == HOLD_RAG_DST ? base + band : base;
+      s0 = b * (FORM == HOLD_RAG_DST ? a.n : a.m);
+    } else {
+      slice = from = data + kk * a.slice_bytes;
+      s0 = 0;
+    }
+  };
+  char *slice = nullptr, *from = nullptr;
+  uint32_t s0 = 0;
+  if (k < a.d3) {
+    item(k, slice, from, s0);
+    if (mine) hold_load<EB, FORM, kTmemThreads>(from, a, r0, c0, smem_raw, s0, &mb);
+    hold_loaded(&mb);
+  }
+  while (k < a.d3) {
+    if (!hold_landed(&mb, phase)) {  // as in k_hold
+      if (threadIdx.x == 0) atomicExch(status, 5 /* T213_ERR_TIMEOUT */);
+      break;
+    }
+    bool last = false;
+    if (threadIdx.x == 0) last = hold_grid_arrive(bar, a.ctas, gen);
+    if (mine) tmem_fill<EB, FORM>(slice, from, a, r0, c0, smem_raw, s0, taddr);
+    __syncthreads();  // every warp has read the tile: the next slice's may land
+    const int64_t next = k + a.teams;
+    char *nslice = slice, *nfrom = from;
+    uint32_t ns0 = s0;
+    if (next < a.d3) {
+      item(next, nslice, nfrom, ns0);
+      fence_proxy_async();
+      if (mine) hold_load<EB, FORM, kTmemThreads>(nfrom, a, r0, c0, smem_raw, ns0, &mb);
+      hold_loaded(&mb);
+    }
+    if (threadIdx.x == 0) {
+      ok_s = last || hold_grid_wait(bar, a.ctas, gen);
+      gen++;
+    }
+    __syncthreads();
+    if (!ok_s) {
+      if (next < a.d3) hold_landed(&mb, phase);  // nothing may land after the CTA has gone
+      if (threadIdx.x == 0) atomicExch(status, 5 /* T213_ERR_TIMEOUT */);
+      break;
+    }
+    if (mine) tmem_drain<EB, FORM>(slice, a, r0, c0, s0, taddr);
+    k = next;
+    slice = nslice;
+    from = nfrom;
+    s0 = ns0;
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "n"(kTmemCols) : "memory");
 }
 
 // ---- many tensors in rounds -------------------------------------------------------
@@ -435,11 +758,11 @@ struct RoundTile {
 };
 
 template <int EB, int FORM>
-__device__ __noinline__ void round_load(const RoundTensor &t, const RoundTile &ti, unsigned char *buf) {
+__device__ __noinline__ void round_load(const RoundTensor &t, const RoundTile &ti, unsigned char *buf, uint64_t *mb) {
   const HoldArgs a = t.a;  // a copy: the tile's stores must not make the compiler read it again
   const uint32_t tr = a.tcdiv.div(ti.tile);
   hold_load<EB, FORM>(t.data + (int64_t)ti.slice * a.slice_bytes, a, tr * a.tm, (ti.tile - tr * a.TC) * a.tn,
-                      buf + ti.off, 0);
+                      buf + ti.off, 0, mb);
 }
 template <int EB, int FORM>
 __device__ __noinline__ void round_store(const RoundTensor &t, const RoundTile &ti, const unsigned char *buf) {
@@ -455,6 +778,13 @@ __global__ void __launch_bounds__(kHoldThreads, 2)
                   int *status) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ int ok_s;
+  __shared__ uint64_t mb;
+  if (threadIdx.x == 0) {
+    mbar_init(&mb, kHoldThreads / 32);
+    fence_barrier_init();
+  }
+  __syncthreads();
+  uint32_t phase = 0;
   const uint32_t G = gridDim.x;
   auto load = [&](uint32_t r) {
     unsigned char *buf = smem_raw + (size_t)(r & 1) * buf_bytes;
@@ -463,20 +793,25 @@ __global__ void __launch_bounds__(kHoldThreads, 2)
       const RoundTile ti = tiles[q];
       const RoundTensor &t = tensors[ti.tensor];
       switch (t.kind) {
-        case 1: round_load<1, HOLD_SCALAR>(t, ti, buf); break;
-        case 2: round_load<2, HOLD_SCALAR>(t, ti, buf); break;
-        case 4: round_load<4, HOLD_SCALAR>(t, ti, buf); break;
-        case 8: round_load<8, HOLD_SCALAR>(t, ti, buf); break;
-        case 16: round_load<16, HOLD_SCALAR>(t, ti, buf); break;
-        case -2: round_load<2, HOLD_VEC>(t, ti, buf); break;
-        default: round_load<4, HOLD_VEC>(t, ti, buf); break;
+        case 1: round_load<1, HOLD_SCALAR>(t, ti, buf, &mb); break;
+        case 2: round_load<2, HOLD_SCALAR>(t, ti, buf, &mb); break;
+        case 4: round_load<4, HOLD_SCALAR>(t, ti, buf, &mb); break;
+        case 8: round_load<8, HOLD_SCALAR>(t, ti, buf, &mb); break;
+        case 16: round_load<16, HOLD_SCALAR>(t, ti, buf, &mb); break;
+        case -2: round_load<2, HOLD_VEC>(t, ti, buf, &mb); break;
+        default: round_load<4, HOLD_VEC>(t, ti, buf, &mb); break;
       }
     }
+    hold_loaded(&mb);
   };
   load(0);
   for (uint32_t r = 0; r < rounds; r++) {
-    cp_async_wait_all();
-    __syncthreads();  // this CTA's loads of round r have landed, its stores of round r - 1 are issued
+    // this CTA's loads of round r have landed, its stores of round r - 1 are issued
+    if (!hold_landed(&mb, phase)) {
+      if (threadIdx.x == 0) atomicExch(status, 5 /* T213_ERR_TIMEOUT */);
+      return;
+    }
+    fence_proxy_async();
     if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
     if (r + 1 < rounds) load(r + 1);
     if (threadIdx.x == 0) {
@@ -494,7 +829,7 @@ __global__ void __launch_bounds__(kHoldThreads, 2)
     }
     __syncthreads();
     if (!ok_s) {
-      cp_async_wait_all();
+      if (r + 1 < rounds) hold_landed(&mb, phase);  // nothing may land after the CTA has gone
       if (threadIdx.x == 0) atomicExch(status, 5 /* T213_ERR_TIMEOUT */);
       return;
     }

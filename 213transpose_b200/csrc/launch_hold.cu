@@ -88,11 +88,15 @@ int lanes_log2(int64_t x) {
 // 1 us each and a barrier with its costlier launch (cluster 1.2 us, grid 2.5 us);
 // a slice of one CTA waits for no other; short row pieces cost
 // a 32-byte sector more per piece.
-bool hold_search(HoldGeom &g, int64_t m, int64_t n, int eb, int64_t we, int64_t d3, int form) {
+// `tmem`: tilings of the form that keeps a team's next slice in flight
+// (k_hold_tmem): one tile per CTA, its words in the SM's tensor
+// memory; the barrier and the latencies are then hidden from the second slice
+// on, and 1 us a slice is left.
+bool hold_search(HoldGeom &g, int64_t m, int64_t n, int eb, int64_t we, int64_t d3, int form, bool tmem = false) {
   const DevInfo &d = dev_info();
   const int64_t E = eb * we;
-  const int64_t budget = hold_budget();
-  const int64_t slots = 2ll * d.sms;
+  const int64_t budget = tmem ? (d.smem_optin - 128) / 128 * 128 : hold_budget();
+  const int64_t slots = tmem ? d.sms : 2ll * d.sms;
   const int64_t Q = form == HOLD_VEC ? 16 / eb : 1;
   // tile sides in whole 32-byte sectors where the rows are
   const int64_t un = std::max<int64_t>(Q, (n * E) % 32 == 0 && E < 32 ? 32 / E : 1);
@@ -100,7 +104,14 @@ bool hold_search(HoldGeom &g, int64_t m, int64_t n, int eb, int64_t we, int64_t 
   const bool rag = form == HOLD_RAG_DST || form == HOLD_RAG_SRC;  // one team: a slice's bands in order
   double best = 1e30;
   g.ok = false;
-  for (int S = 1; S <= 2; S++) {
+  const int64_t N4 = eb < 4 ? 4 / eb : 1;
+  auto tmem_fits = [&](int64_t tm, int64_t tn) {
+    const int64_t words = N4 == 1 ? tm : (tm + 2 * N4 - 2) / N4, U = kTmemUnitCols / std::max(1, eb / 4);
+    const int lg = lanes_log2(words);
+    const int64_t step = U * (32 >> lg) * N4;
+    return ((words + (1 << lg) - 1) >> lg) * ((tn + step - 1) / step * N4) <= kTmemUnits * (kTmemThreads / 32);
+  };
+  for (int S = 1; S <= (tmem ? 1 : 2); S++) {
     const int64_t tile_cap = budget / S;
     const int64_t max_tiles = slots * S;
     for (int64_t TC = 1; TC <= std::min<int64_t>(max_tiles, n); TC = TC < 48 ? TC + 1 : TC + TC / 16) {
@@ -126,12 +137,13 @@ bool hold_search(HoldGeom &g, int64_t m, int64_t n, int eb, int64_t we, int64_t 
         const int64_t ctas = (T + S - 1) / S;
         const int mode = ctas == 1 ? HOLD_CTA : ctas <= 16 ? HOLD_CLUSTER : HOLD_GRID;
         if (S > 1 && mode != HOLD_GRID) continue;
-        if (rag && mode != HOLD_GRID) continue;
+        if ((rag || tmem) && mode != HOLD_GRID) continue;
+        if (tmem && !tmem_fits(tm, tn)) continue;
         const int64_t teams = rag ? 1 : std::min<int64_t>(d3, slots / ctas);
         if (mode == HOLD_GRID && teams > kHoldTeams) continue;
         const int64_t waves = (d3 + teams - 1) / teams;
         const int64_t conc = teams * ctas, per_sm = (conc + d.sms - 1) / d.sms;
-        const double bw = std::min(60e9, 6.4e12 / (double)std::min<int64_t>(conc, d.sms)) / (double)per_sm;
+        const double bw = std::min(tmem ? 40e9 : 60e9, 6.4e12 / (double)std::min<int64_t>(conc, d.sms)) / (double)per_sm;
         const double share = (double)S * tm * tn * E;
         // lanes left idle by tiles of a few rows more than a multiple of 32
         const int64_t N = eb < 4 ? 4 / eb : 1, wd = form != HOLD_VEC && form != HOLD_WIDE ? (tm + N - 1) / N : 32;
@@ -139,7 +151,7 @@ bool hold_search(HoldGeom &g, int64_t m, int64_t n, int eb, int64_t we, int64_t 
         const double ineff = idle + 2.0 + 32.0 / (double)(tn * E) + 32.0 / (double)(tm * E);
         const double bar = mode == HOLD_CTA ? 0.2e-6 : mode == HOLD_CLUSTER ? 1.2e-6 : 2.5e-6;
         const double lat = waves > 1 && S > 1 ? 1.5e-6 : 2e-6;
-        const double t = waves * (lat + bar + share * ineff / bw);
+        const double t = tmem ? 4e-6 + waves * (1e-6 + share * ineff / bw) : waves * (lat + bar + share * ineff / bw);
         if (t < best * 0.999) {
           best = t;
           g.ok = true;
@@ -154,6 +166,7 @@ bool hold_search(HoldGeom &g, int64_t m, int64_t n, int eb, int64_t we, int64_t 
           g.packed = packed;
           g.mode = mode;
           g.form = form;
+          g.tmem = tmem;
           g.est_us = t * 1e6;
         }
       }
@@ -261,6 +274,19 @@ uint32_t *hold_bars(int *status) {
 
 }  // namespace
 
+// Tensor memory as the second buffer, where one team takes slices that fill
+// more than half of the chip one after the other.  Measured on B200, with and
+// without, us: bf16 (4099, 2053, 8) 97.5 / 108.9, fp32 (3001, 2000, 4) 49.6 /
+// 51.1, fp64 (2408, 1432, 4) 52.9 / 55.8, ragged bands of fp32 (561, 62490, 2)
+// 267 / 288 and (7402, 10752, 1) 325 / 344.  Several teams beside each other
+// already overlap, and two CTAs per SM serve them better: fp32 (1500, 1301, 8)
+// 37.8 / 34.1.
+void hold_try_tmem(HoldGeom &g, int64_t m, int64_t n, int eb, int64_t d3, int form) {
+  if (!g.ok || g.mode != HOLD_GRID || g.teams > 1 || d3 <= 1) return;
+  HoldGeom t;
+  if (hold_search(t, m, n, eb, 1, d3, form, true) && t.tm * 4 >= std::min<uint32_t>(t.tn, 128)) g = t;
+}
+
 void hold_plan(HoldPlan &hp, int64_t m, int64_t n, int eb, int64_t we, int64_t d3) {
   hp.ready = std::make_shared<HoldReady>();
   if (we > 1) {
@@ -268,6 +294,7 @@ void hold_plan(HoldPlan &hp, int64_t m, int64_t n, int eb, int64_t we, int64_t d
     return;
   }
   hold_search(hp.any, m, n, eb, 1, d3, HOLD_SCALAR);
+  hold_try_tmem(hp.any, m, n, eb, d3, HOLD_SCALAR);
   if ((eb == 2 || eb == 4) && (n * eb) % 16 == 0 && (m * eb) % 16 == 0)
     hold_search(hp.vec, m, n, eb, 1, d3, HOLD_VEC);
 }
@@ -279,7 +306,7 @@ std::string describe_slice(const HoldPlan &hp) {
   char buf[160];
   snprintf(buf, sizeof buf, "slice(%s tiles=%u of %ux%u per cta=%u ctas=%u teams=%u%s)",
            g.mode == HOLD_CTA ? "cta" : g.mode == HOLD_CLUSTER ? "cluster" : "grid", g.T, g.tm, g.tn, g.S, g.ctas,
-           g.teams, g.form == HOLD_VEC ? " vec" : "");
+           g.teams, g.form == HOLD_VEC ? " vec" : g.tmem ? " tmem" : "");
   return buf;
 }
 
@@ -299,6 +326,11 @@ void hold_args(HoldArgs &a, const HoldGeom &g, int64_t m, int64_t n, int eb, int
   a.P = g.P;
   a.H = (uint32_t)hold_region(g.tm, g.P, eb, g.form);
   a.packed = g.packed;
+  // bulk copies from 256 bytes a row piece: one instruction a row instead of
+  // one a 512 bytes (ragged bands of fp32 (1000003, 37, 1) 142 -> 132 us, fp32
+  // (3001, 2000, 4) 51.9 -> 51.1); shorter pieces are many small copies
+  a.bulk = !g.packed && (g.form == HOLD_SCALAR || g.form == HOLD_RAG_DST || g.form == HOLD_RAG_SRC) &&
+           (int64_t)g.tn * eb >= 256;
   a.tile_bytes = (uint32_t)hold_tile_bytes(g.tm, g.tn, g.P, eb, g.form, g.packed);
   a.mode = g.mode;
   a.we = (uint32_t)we;
@@ -316,71 +348,51 @@ void hold_args(HoldArgs &a, const HoldGeom &g, int64_t m, int64_t n, int eb, int
   }
 }
 
+template <int EB>
+const void *hold_kernel_of(const HoldGeom &g) {
+  if constexpr (EB == 2 || EB == 4)
+    if (g.form == HOLD_VEC) return (const void *)k_hold<EB, HOLD_VEC>;
+  if constexpr (EB == 16)
+    if (g.form == HOLD_WIDE) return (const void *)k_hold<16, HOLD_WIDE>;
+  switch (g.form) {
+    case HOLD_SCALAR:
+      return g.tmem ? (const void *)k_hold_tmem<EB, HOLD_SCALAR> : (const void *)k_hold<EB, HOLD_SCALAR>;
+    case HOLD_RAG_SRC:
+      return g.tmem ? (const void *)k_hold_tmem<EB, HOLD_RAG_SRC> : (const void *)k_hold<EB, HOLD_RAG_SRC>;
+    case HOLD_RAG_DST:
+      if constexpr (EB >= 4)
+        if (g.tmem) return (const void *)k_hold_tmem<EB, HOLD_RAG_DST>;
+      return (const void *)k_hold<EB, HOLD_RAG_DST>;
+  }
+  return nullptr;
+}
+
+const void *hold_kernel(const HoldGeom &g, int eb) {
+  switch (eb) {
+    case 1:
+      return hold_kernel_of<1>(g);
+    case 2:
+      return hold_kernel_of<2>(g);
+    case 4:
+      return hold_kernel_of<4>(g);
+    case 8:
+      return hold_kernel_of<8>(g);
+    case 16:
+      return hold_kernel_of<16>(g);
+  }
+  return nullptr;
+}
+
 int hold_prepare(HoldReady::Form &f, const HoldGeom &g, int64_t m, int64_t n, int eb, int64_t we) {
   int status = T213_OK;
   f.status = device_status_word(&status);
   if (!f.status) return status;
   hold_args(f.args, g, m, n, eb, we);
   f.smem = (int64_t)g.S * f.args.tile_bytes;
-  switch (g.form == HOLD_WIDE ? 0 : g.form == HOLD_VEC ? -eb : g.form == HOLD_RAG_DST ? 100 + eb
-          : g.form == HOLD_RAG_SRC ? 200 + eb : eb) {
-    case 101:
-      f.kern = (const void *)k_hold<1, HOLD_RAG_DST>;
-      break;
-    case 102:
-      f.kern = (const void *)k_hold<2, HOLD_RAG_DST>;
-      break;
-    case 104:
-      f.kern = (const void *)k_hold<4, HOLD_RAG_DST>;
-      break;
-    case 108:
-      f.kern = (const void *)k_hold<8, HOLD_RAG_DST>;
-      break;
-    case 116:
-      f.kern = (const void *)k_hold<16, HOLD_RAG_DST>;
-      break;
-    case 201:
-      f.kern = (const void *)k_hold<1, HOLD_RAG_SRC>;
-      break;
-    case 202:
-      f.kern = (const void *)k_hold<2, HOLD_RAG_SRC>;
-      break;
-    case 204:
-      f.kern = (const void *)k_hold<4, HOLD_RAG_SRC>;
-      break;
-    case 208:
-      f.kern = (const void *)k_hold<8, HOLD_RAG_SRC>;
-      break;
-    case 216:
-      f.kern = (const void *)k_hold<16, HOLD_RAG_SRC>;
-      break;
-    case 0:
-      f.kern = (const void *)k_hold<16, HOLD_WIDE>;
-      break;
-    case -2:
-      f.kern = (const void *)k_hold<2, HOLD_VEC>;
-      break;
-    case -4:
-      f.kern = (const void *)k_hold<4, HOLD_VEC>;
-      break;
-    case 1:
-      f.kern = (const void *)k_hold<1, HOLD_SCALAR>;
-      break;
-    case 2:
-      f.kern = (const void *)k_hold<2, HOLD_SCALAR>;
-      break;
-    case 4:
-      f.kern = (const void *)k_hold<4, HOLD_SCALAR>;
-      break;
-    case 8:
-      f.kern = (const void *)k_hold<8, HOLD_SCALAR>;
-      break;
-    case 16:
-      f.kern = (const void *)k_hold<16, HOLD_SCALAR>;
-      break;
-    default:
-      set_error("unsupported element size");
-      return T213_ERR_UNSUPPORTED;
+  f.kern = hold_kernel(g, eb);
+  if (!f.kern) {
+    set_error("unsupported element size");
+    return T213_ERR_UNSUPPORTED;
   }
   if (!kernel_attr_once(f.kern, f.smem, g.mode == HOLD_CLUSTER ? (int)g.ctas : 1))
     return cuda_status(cudaGetLastError(), "cudaFuncSetAttribute(slice)");
@@ -388,7 +400,7 @@ int hold_prepare(HoldReady::Form &f, const HoldGeom &g, int64_t m, int64_t n, in
     f.bars = hold_bars(&status);
     if (!f.bars) return status;
     int per_sm = 1;
-    occupancy_cached(f.kern, kHoldThreads, f.smem, 1, &per_sm);
+    occupancy_cached(f.kern, g.tmem ? kTmemThreads : kHoldThreads, f.smem, 1, &per_sm);
     f.resident = (int64_t)per_sm * dev_info().sms >= (int64_t)g.teams * g.ctas ? (int)g.teams : 0;
   } else {
     occupancy_cached(f.kern, kHoldThreads, f.smem, (int)g.ctas, &f.resident);
@@ -401,7 +413,7 @@ int hold_prepare(HoldReady::Form &f, const HoldGeom &g, int64_t m, int64_t n, in
 int hold_enqueue(const HoldReady::Form &f, const HoldGeom &g, HoldArgs &a, char *data, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(a.teams * a.ctas, 1, 1);
-  cfg.blockDim = dim3(kHoldThreads, 1, 1);
+  cfg.blockDim = dim3(g.tmem ? kTmemThreads : kHoldThreads, 1, 1);
   cfg.dynamicSmemBytes = (size_t)f.smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
@@ -454,9 +466,9 @@ bool ragged_geometry(RaggedPlan &rp, int64_t m, int64_t n, int eb, int64_t d3) {
     const int64_t r = big - q * t;
     rp.hold = HoldPlan{};
     rp.hold.ready = std::make_shared<HoldReady>();
-    if (!hold_search(rp.hold.any, rp.cols ? m : t, rp.cols ? t : n, eb, 1, d3 * q,
-                     rp.cols ? HOLD_RAG_SRC : HOLD_RAG_DST))
-      continue;
+    const int form = rp.cols ? HOLD_RAG_SRC : HOLD_RAG_DST;
+    if (!hold_search(rp.hold.any, rp.cols ? m : t, rp.cols ? t : n, eb, 1, d3 * q, form)) continue;
+    if (rp.cols || eb >= 4) hold_try_tmem(rp.hold.any, rp.cols ? m : t, rp.cols ? t : n, eb, d3 * q, form);
     rp.t = t;
     rp.q = q;
     rp.r = r;
