@@ -51,17 +51,19 @@ struct HoldArgs {
   int32_t lgs;  // log2 of the lanes that share an output column
   uint32_t we;       // wide form: 16-byte words per element
   FastDiv<uint32_t> wediv, tcdiv, rbdiv;
-  // ragged bands: m x n is a band, nb bands per slice; segment s of a slice
-  // (seg_bytes long, q to a row of rag_pitch bytes) at
-  // (s / q) * rag_pitch + (s % q) * seg_bytes
+  // ragged bands: m x n is a band, nb bands per slice; segment s of a slice is
+  // seg_bytes long, and rest_bytes lie between the q-th segment of a row and
+  // the next row
   FastDiv<uint32_t> qdiv;
-  uint32_t nb, seg_bytes;
-  int64_t rag_pitch;
+  uint32_t nb, seg_bytes, rest_bytes;
   __device__ __forceinline__ uint64_t seg_at(uint32_t s) const {
-    const uint32_t r = qdiv.div(s);
-    return (uint64_t)r * (uint64_t)rag_pitch + (uint64_t)(s - r * qdiv.get()) * seg_bytes;
+    return (uint64_t)s * seg_bytes + (uint64_t)qdiv.div(s) * rest_bytes;
   }
 };
+
+// The warp's index, broadcast so that the compiler keeps what follows from it
+// (unit, column, output row) in uniform registers.
+__device__ __forceinline__ uint32_t warp_index() { return __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); }
 
 // ---- tiles -------------------------------------------------------------------
 // Shared-memory layout of a scalar tile: a row piece lies in the 16-byte
@@ -171,7 +173,8 @@ __device__ __forceinline__ void hold_store(char *slice, const char *from, const 
                                            const unsigned char *s, uint32_t s0) {
   using E = typename ElemT<EB>::type;
   const uint32_t rows = min(a.tm, a.m - r0), cols = min(a.tn, a.n - c0);
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const uint32_t lane = threadIdx.x & 31, warp = warp_index();
+  constexpr uint32_t nw = kHoldThreads / 32;
   if constexpr (FORM == HOLD_VEC) {
     // a warp takes 8 row blocks by 4 column chunks: its 8-lane phases read 8
     // different chunks of the swizzle, and it writes 4 x 128 bytes at a time
@@ -221,16 +224,20 @@ __device__ __forceinline__ void hold_store(char *slice, const char *from, const 
     // output rows of a unit start at the same byte of a 4-byte word.
     constexpr uint32_t N = EB < 4 ? 4 / EB : 1;
     constexpr uint32_t U = EB == 16 ? 4 : EB == 4 ? 16 : 8;
-    const uint32_t L = 1u << a.lgs, G = 32u >> a.lgs, li = lane & (L - 1), sub = lane >> a.lgs;
+    auto units = [&](auto whole) {
+    // `whole`: the 32 lanes share a column
+    constexpr bool W32 = decltype(whole)::value;
+    const uint32_t lgs = W32 ? 5u : (uint32_t)a.lgs;
+    const uint32_t L = 1u << lgs, G = W32 ? 1u : 32u >> lgs, li = W32 ? lane : lane & (L - 1), sub = W32 ? 0u : lane >> lgs;
     const uint32_t plo = a.n * EB;
     const uint32_t lo = (uint32_t)(uintptr_t)from + (FORM == HOLD_RAG_SRC ? c0 * EB : (r0 * a.n + c0) * EB);
     const uint32_t sr = s0 + r0;  // RAG_SRC: the segment of the tile's first row
     const uint32_t words = N == 1 ? rows : (rows + 2 * N - 2) / N;  // one more covers every offset
-    const uint32_t nrb = (words + L - 1) >> a.lgs, ncg = (cols + U * G * N - 1) / (U * G * N) * N;
+    const uint32_t nrb = (words + L - 1) >> lgs, ncg = (cols + U * G * N - 1) / (U * G * N) * N;
     const bool full = rows == a.tm;
     for (uint32_t u = warp; u < nrb * ncg; u += nw) {
       const uint32_t cg = full ? a.rbdiv.div(u) : u / nrb;
-      const uint32_t w = ((u - cg * nrb) << a.lgs) + li;
+      const uint32_t w = ((u - cg * nrb) << lgs) + li;
       const uint32_t j0 = cg / N * (U * G * N) + cg % N * G + sub;
       if (w >= words || j0 >= cols) continue;
       const uint32_t o = ((c0 + j0) * a.m + r0) * EB;
@@ -241,19 +248,28 @@ __device__ __forceinline__ void hold_store(char *slice, const char *from, const 
         const unsigned char *p = s + hold_row<EB, FORM>(a, w, lo, plo, sr) + j0 * EB;
         E v[U];
         if constexpr (FORM == HOLD_RAG_DST) {
-          char *g = slice + (size_t)((r0 + w) * EB);
           const uint32_t sj = s0 + c0 + j0;
+          char *g = slice + (size_t)((r0 + w) * EB) + a.seg_at(sj);
+          uint32_t col = sj - a.qdiv.div(sj) * a.qdiv.get();  // the segment's place in its row
 #pragma unroll
           for (uint32_t q = 0; q < U; q++)
             if (q < left) v[q] = *reinterpret_cast<const E *>(p + q * ps);
 #pragma unroll
-          for (uint32_t q = 0; q < U; q++)
-            if (q < left) *reinterpret_cast<E *>(g + a.seg_at(sj + q * G)) = v[q];
+          for (uint32_t q = 0; q < U; q++) {
+            if (q < left) *reinterpret_cast<E *>(g) = v[q];
+            if constexpr (W32) {
+              const bool wrap = ++col == a.qdiv.get();
+              g += (size_t)a.seg_bytes + (wrap ? a.rest_bytes : 0u);
+              if (wrap) col = 0;
+            } else {
+              g = slice + (size_t)((r0 + w) * EB) + a.seg_at(sj + (q + 1) * G);
+            }
+          }
           continue;
         }
         char *g = slice + (size_t)(o + w * EB);
         if (left >= U) {
-          if (a.lgs == 5) {  // consecutive columns: reads at constant offsets
+          if constexpr (W32) {  // consecutive columns: reads at constant offsets
 #pragma unroll
             for (uint32_t q = 0; q < U; q++) v[q] = *reinterpret_cast<const E *>(p + q * EB);
           } else {
@@ -336,6 +352,11 @@ __device__ __forceinline__ void hold_store(char *slice, const char *from, const 
         }
       }
     }
+    };
+    if (a.lgs == 5)
+      units(std::true_type{});
+    else
+      units(std::false_type{});
   }
 }
 
@@ -525,22 +546,27 @@ __device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
       : "memory");
 }
 
-// The units of hold_store's scalar form with 16 words per lane.
-template <int EB>
+// The units of hold_store's scalar form with 16 words per lane.  W32: the 32
+// lanes share a column, and all but the lane's word is uniform in the warp.
+template <int EB, bool W32>
 struct TmemUnit {
   static constexpr uint32_t N = EB < 4 ? 4 / EB : 1;
   static constexpr uint32_t W = EB < 4 ? 1 : EB / 4;  // words per element
   static constexpr uint32_t U = kTmemUnitCols / W;    // column steps
-  uint32_t w, j0, left, gn;  // word, first column, column steps left (0: idle lane), columns per step
+  uint32_t w, j0, left, gn;  // word, first column, column steps left, columns per step
+  bool in;                   // the lane has a word
   __device__ __forceinline__ TmemUnit(const HoldArgs &a, uint32_t u, uint32_t rows, uint32_t cols, uint32_t lane) {
-    const uint32_t L = 1u << a.lgs, G = 32u >> a.lgs, li = lane & (L - 1), sub = lane >> a.lgs;
+    const uint32_t lgs = W32 ? 5u : (uint32_t)a.lgs;
+    const uint32_t L = 1u << lgs, G = W32 ? 1u : 32u >> lgs;
+    const uint32_t li = W32 ? lane : lane & (L - 1), sub = W32 ? 0u : lane >> lgs;
     const uint32_t words = N == 1 ? rows : (rows + 2 * N - 2) / N;
-    const uint32_t nrb = (words + L - 1) >> a.lgs;
+    const uint32_t nrb = (words + L - 1) >> lgs;
     const uint32_t cg = rows == a.tm ? a.rbdiv.div(u) : u / nrb;
-    w = ((u - cg * nrb) << a.lgs) + li;
+    w = ((u - cg * nrb) << lgs) + li;
     gn = G * N;
     j0 = cg / N * (U * gn) + cg % N * G + sub;
-    left = w < words && j0 < cols ? min((cols - 1 - j0) / gn + 1, U) : 0;
+    left = j0 < cols ? min((cols - 1 - j0) / gn + 1, U) : 0;
+    in = w < words;
   }
   __device__ static __forceinline__ uint32_t count(const HoldArgs &a, uint32_t rows, uint32_t cols) {
     const uint32_t L = 1u << a.lgs, G = 32u >> a.lgs;
@@ -549,44 +575,53 @@ struct TmemUnit {
   }
 };
 
-template <int EB, int FORM>
+template <int EB, int FORM, bool W32>
 __device__ __forceinline__ void tmem_fill(const char *slice, const char *from, const HoldArgs &a, uint32_t r0,
                                           uint32_t c0, const unsigned char *s, uint32_t s0, uint32_t taddr) {
   using E = typename ElemT<EB>::type;
-  using TU = TmemUnit<EB>;
+  using TU = TmemUnit<EB, W32>;
+  constexpr uint32_t N = TU::N;
   const uint32_t rows = min(a.tm, a.m - r0), cols = min(a.tn, a.n - c0);
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t lane = threadIdx.x & 31, warp = warp_index();
   const uint32_t plo = a.n * EB;
   const uint32_t lo = (uint32_t)(uintptr_t)from + (FORM == HOLD_RAG_SRC ? c0 * EB : (r0 * a.n + c0) * EB);
   const uint32_t sr = s0 + r0;
   const uint32_t units = TU::count(a, rows, cols);
   for (uint32_t u = warp; u < units; u += kTmemThreads / 32, taddr += kTmemUnitCols) {
     const TU t(a, u, rows, cols, lane);
+    const uint32_t j0 = min(t.j0, cols - 1);
     union {
       uint32_t w[16];
       E e[TU::U];
     } v;
-    if constexpr (TU::N == 1) {
-      const unsigned char *p = s + hold_row<EB, FORM>(a, min(t.w, rows - 1), lo, plo, sr) + t.j0 * EB;
-#pragma unroll
-      for (uint32_t q = 0; q < TU::U; q++)
-        if (q < t.left) v.e[q] = *reinterpret_cast<const E *>(p + q * t.gn * EB);
+    const unsigned char *p[N];
+    if constexpr (N == 1) {
+      // lanes without a word read the last row's, and write nothing later
+      p[0] = s + hold_row<EB, FORM>(a, min(t.w, rows - 1), lo, plo, sr) + j0 * EB;
     } else {
       const uint32_t h = (((uint32_t)(uintptr_t)slice + ((c0 + t.j0) * a.m + r0) * EB) & 3u) / EB;
-      const int32_t e0 = (int32_t)(t.w * TU::N) - (int32_t)h;
-      const unsigned char *p[TU::N];
+      const int32_t e0 = (int32_t)(t.w * N) - (int32_t)h;
 #pragma unroll
-      for (uint32_t b = 0; b < TU::N; b++)
-        p[b] = s + hold_row<EB, FORM>(a, min((uint32_t)max(e0 + (int32_t)b, 0), rows - 1), lo, plo, sr) + t.j0 * EB;
-#pragma unroll
-      for (uint32_t q = 0; q < 16; q++) {
+      for (uint32_t b = 0; b < N; b++)
+        p[b] = s + hold_row<EB, FORM>(a, min((uint32_t)max(e0 + (int32_t)b, 0), rows - 1), lo, plo, sr) + j0 * EB;
+    }
+    auto read = [&](uint32_t q, uint32_t off) {
+      if constexpr (N == 1) {
+        v.e[q] = *reinterpret_cast<const E *>(p[0] + off);
+      } else {
         v.w[q] = 0;
-        if (q < t.left) {
 #pragma unroll
-          for (uint32_t b = 0; b < TU::N; b++)
-            v.w[q] |= (uint32_t) * reinterpret_cast<const E *>(p[b] + q * t.gn * EB) << (8 * EB * b);
-        }
+        for (uint32_t b = 0; b < N; b++)
+          v.w[q] |= (uint32_t) * reinterpret_cast<const E *>(p[b] + off) << (8 * EB * b);
       }
+    };
+    if (W32 && t.left == TU::U) {
+#pragma unroll
+      for (uint32_t q = 0; q < TU::U; q++) read(q, q * N * EB);
+    } else {
+#pragma unroll
+      for (uint32_t q = 0; q < TU::U; q++)
+        if (q < t.left) read(q, q * t.gn * EB);
     }
     __syncwarp();
     tmem_st16(taddr, v.w);
@@ -594,13 +629,14 @@ __device__ __forceinline__ void tmem_fill(const char *slice, const char *from, c
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
-template <int EB, int FORM>
+template <int EB, int FORM, bool W32>
 __device__ __forceinline__ void tmem_drain(char *slice, const HoldArgs &a, uint32_t r0, uint32_t c0, uint32_t s0,
                                            uint32_t taddr) {
   using E = typename ElemT<EB>::type;
-  using TU = TmemUnit<EB>;
+  using TU = TmemUnit<EB, W32>;
+  constexpr uint32_t N = TU::N;
   const uint32_t rows = min(a.tm, a.m - r0), cols = min(a.tn, a.n - c0);
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t lane = threadIdx.x & 31, warp = warp_index();
   const uint32_t units = TU::count(a, rows, cols);
   for (uint32_t u = warp; u < units; u += kTmemThreads / 32, taddr += kTmemUnitCols) {
     const TU t(a, u, rows, cols, lane);
@@ -610,31 +646,51 @@ __device__ __forceinline__ void tmem_drain(char *slice, const HoldArgs &a, uint3
     } v;
     __syncwarp();
     tmem_ld16(taddr, v.w);
+    if (!t.in) continue;
     if constexpr (FORM == HOLD_RAG_DST) {
-      static_assert(TU::N == 1, "the byte offset of an output row is its own");
-      char *g = slice + (size_t)((r0 + t.w) * EB);
+      static_assert(N == 1, "the byte offset of an output row is its own");
       const uint32_t sj = s0 + c0 + t.j0;
+      char *g = slice + (size_t)((r0 + t.w) * EB) + a.seg_at(sj);
+      uint32_t col = sj - a.qdiv.div(sj) * a.qdiv.get();  // the segment's place in its row
 #pragma unroll
-      for (uint32_t q = 0; q < TU::U; q++)
-        if (q < t.left) *reinterpret_cast<E *>(g + a.seg_at(sj + q * t.gn)) = v.e[q];
+      for (uint32_t q = 0; q < TU::U; q++) {
+        if (q < t.left) *reinterpret_cast<E *>(g) = v.e[q];
+        if constexpr (W32) {
+          const bool wrap = ++col == a.qdiv.get();
+          g += (size_t)a.seg_bytes + (wrap ? a.rest_bytes : 0u);
+          if (wrap) col = 0;
+        } else {
+          g = slice + (size_t)((r0 + t.w) * EB) + a.seg_at(sj + (q + 1) * t.gn);
+        }
+      }
     } else {
       const uint32_t o = ((c0 + t.j0) * a.m + r0) * EB, gs = t.gn * a.m * EB;
-      if constexpr (TU::N == 1) {
+      if constexpr (N == 1) {
         char *g = slice + (size_t)(o + t.w * EB);
+        if (W32 && t.left == TU::U) {
 #pragma unroll
-        for (uint32_t q = 0; q < TU::U; q++, g += gs)
-          if (q < t.left) *reinterpret_cast<E *>(g) = v.e[q];
-      } else {
-        const uint32_t h = (((uint32_t)(uintptr_t)slice + o) & 3u) / EB;
-        const int32_t e0 = (int32_t)(t.w * TU::N) - (int32_t)h;
-        char *g = slice + (size_t)o + (int64_t)e0 * EB;
-        if (e0 >= 0 && e0 + (int32_t)TU::N <= (int32_t)rows) {
-#pragma unroll
-          for (uint32_t q = 0; q < 16; q++, g += gs)
-            if (q < t.left) *reinterpret_cast<uint32_t *>(g) = v.w[q];
+          for (uint32_t q = 0; q < TU::U; q++, g += gs) *reinterpret_cast<E *>(g) = v.e[q];
         } else {
 #pragma unroll
-          for (uint32_t b = 0; b < TU::N; b++)
+          for (uint32_t q = 0; q < TU::U; q++, g += gs)
+            if (q < t.left) *reinterpret_cast<E *>(g) = v.e[q];
+        }
+      } else {
+        const uint32_t h = (((uint32_t)(uintptr_t)slice + o) & 3u) / EB;
+        const int32_t e0 = (int32_t)(t.w * N) - (int32_t)h;
+        char *g = slice + (size_t)o + (int64_t)e0 * EB;
+        if (e0 >= 0 && e0 + (int32_t)N <= (int32_t)rows) {
+          if (W32 && t.left == TU::U) {
+#pragma unroll
+            for (uint32_t q = 0; q < 16; q++, g += gs) *reinterpret_cast<uint32_t *>(g) = v.w[q];
+          } else {
+#pragma unroll
+            for (uint32_t q = 0; q < 16; q++, g += gs)
+              if (q < t.left) *reinterpret_cast<uint32_t *>(g) = v.w[q];
+          }
+        } else {
+#pragma unroll
+          for (uint32_t b = 0; b < N; b++)
             if ((uint32_t)(e0 + (int32_t)b) < rows) {
 #pragma unroll
               for (uint32_t q = 0; q < 16; q++)
@@ -707,7 +763,12 @@ __global__ void __launch_bounds__(kTmemThreads, 1)
     }
     bool last = false;
     if (threadIdx.x == 0) last = hold_grid_arrive(bar, a.ctas, gen);
-    if (mine) tmem_fill<EB, FORM>(slice, from, a, r0, c0, smem_raw, s0, taddr);
+    if (mine) {
+      if (a.lgs == 5)
+        tmem_fill<EB, FORM, true>(slice, from, a, r0, c0, smem_raw, s0, taddr);
+      else
+        tmem_fill<EB, FORM, false>(slice, from, a, r0, c0, smem_raw, s0, taddr);
+    }
     __syncthreads();  // every warp has read the tile: the next slice's may land
     const int64_t next = k + a.teams;
     char *nslice = slice, *nfrom = from;
@@ -728,7 +789,12 @@ __global__ void __launch_bounds__(kTmemThreads, 1)
       if (threadIdx.x == 0) atomicExch(status, 5 /* T213_ERR_TIMEOUT */);
       break;
     }
-    if (mine) tmem_drain<EB, FORM>(slice, a, r0, c0, s0, taddr);
+    if (mine) {
+      if (a.lgs == 5)
+        tmem_drain<EB, FORM, true>(slice, a, r0, c0, s0, taddr);
+      else
+        tmem_drain<EB, FORM, false>(slice, a, r0, c0, s0, taddr);
+    }
     k = next;
     slice = nslice;
     from = nfrom;

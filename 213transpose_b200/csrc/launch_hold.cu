@@ -454,11 +454,15 @@ int hold_form_ready(HoldReady &r, HoldReady::Form &f, const HoldGeom &g, int64_t
 
 bool ragged_geometry(RaggedPlan &rp, int64_t m, int64_t n, int eb, int64_t d3) {
   rp.ok = false;
-  rp.cols = n >= m;
-  const int64_t big = std::max(m, n), small = std::min(m, n);
   const int64_t u = std::max(1, 16 / eb);
   const double chip = 2.0 * dev_info().sms * (double)hold_budget();
   const int64_t q0 = std::max<int64_t>(2, (int64_t)std::ceil((double)m * (double)n * eb / chip));
+  // The longer side is cut; 1- and 2-byte elements, whose output words are
+  // put together column by column in the row form, prefer the column form
+  // while its segments are long enough for the walker (f16 (3712, 5208, 8) 391
+  // us by columns, 411 by rows).
+  rp.cols = n >= m || (eb < 4 && n / q0 * eb >= 3000);
+  const int64_t big = rp.cols ? n : m, small = rp.cols ? m : n;
   for (int64_t q = q0; q <= q0 + q0 / 4 + 4; q++) {
     int64_t t = big / q;
     if (t >= 4 * u) t = t / u * u;  // segments of whole 16-byte blocks
@@ -507,7 +511,7 @@ int launch_hold_rag(const RaggedPlan &rp, char *data, int64_t d3, int64_t slice_
   a.nb = (uint32_t)rp.q;
   a.qdiv = FastDiv<uint32_t>((uint64_t)rp.q);
   a.seg_bytes = (uint32_t)(rp.t * eb);
-  a.rag_pitch = (rp.q * rp.t + rp.r) * eb;
+  a.rest_bytes = (uint32_t)(rp.r * eb);
   return hold_enqueue(f, rp.hold.any, a, data, st);
 }
 
