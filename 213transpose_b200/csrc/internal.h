@@ -199,11 +199,6 @@ int hold_rounds_count(const HoldRounds *r);
 int hold_rounds_launch(HoldRounds *r, int *status_word, cudaStream_t st);
 int64_t hold_cluster_bytes();  // shared memory of the largest team that needs no cooperative launch
 std::string describe_slice(const HoldPlan &hp);
-// Grouped one-pass slices (the batched form): the rows per CTA H and padded
-// pitch P of a slice split over an 8-CTA cluster (false if it does not fit),
-// and one launch of the grouped kernel over device SliceEntry records.
-bool slice_group_params(int64_t m, int64_t n, int eb, const void *data, uint32_t *H, uint32_t *P, bool *vec);
-int launch_slice_group(const void *entries, int32_t n_entries, int64_t n_items, int64_t smem, cudaStream_t st);
 int64_t band_smem_limit();
 bool band_fits(int64_t R, int64_t C, int eb);
 

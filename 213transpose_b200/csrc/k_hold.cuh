@@ -240,8 +240,8 @@ __device__ __forceinline__ void hold_store(char *slice, const char *from, const 
       const uint32_t w = ((u - cg * nrb) << lgs) + li;
       const uint32_t j0 = cg / N * (U * G * N) + cg % N * G + sub;
       if (w >= words || j0 >= cols) continue;
-      const uint32_t o = ((c0 + j0) * a.m + r0) * EB;
-      const uint32_t gs = G * N * a.m * EB;
+      [[maybe_unused]] const uint32_t o = ((c0 + j0) * a.m + r0) * EB;
+      [[maybe_unused]] const uint32_t gs = G * N * a.m * EB;
       const uint32_t ps = G * N * EB;
       const uint32_t left = (cols - 1 - j0) / (G * N) + 1;  // column steps of this lane
       if constexpr (N == 1) {

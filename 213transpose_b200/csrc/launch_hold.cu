@@ -4,6 +4,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
+#include <deque>
 #include <map>
 #include <thread>
 #include <tuple>
@@ -181,16 +182,25 @@ bool hold_search(HoldGeom &g, int64_t m, int64_t n, int eb, int64_t we, int64_t 
 // instantiated from it are gone.
 struct HoldSlots {
   std::mutex mu;
-  std::map<std::tuple<cudaStream_t, std::thread::id>, int> of_stream;
-  std::vector<int> free_list;
+  // by handle, with the stream's own id: a handle comes back for another
+  // stream after its first one was destroyed, whose last launch may still run
+  std::map<std::tuple<cudaStream_t, std::thread::id>, std::pair<unsigned long long, int>> of_stream;
+  std::deque<int> free_list;     // of captured launches whose graph is gone
+  std::deque<int> retired_list;  // of destroyed streams, the oldest first
   int next = 0;
   int take() {
     if (!free_list.empty()) {
-      const int s = free_list.back();
-      free_list.pop_back();
+      const int s = free_list.front();
+      free_list.pop_front();
       return s;
     }
-    return next < kHoldSlots ? next++ : -1;
+    if (next < kHoldSlots) return next++;
+    if (retired_list.size() > kHoldSlots / 4) {  // a thousand streams have come and gone since
+      const int s = retired_list.front();
+      retired_list.pop_front();
+      return s;
+    }
+    return -1;
   }
 };
 
@@ -246,13 +256,20 @@ int hold_slot(cudaStream_t st) {
     }
     return slot;
   }
+  unsigned long long id = 0;
+  if (cudaStreamGetId(st, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return -1;
+  }
   std::lock_guard<std::mutex> lk(hs.mu);
   // the per-thread default stream is one handle for a stream of every thread
   const auto key = std::make_tuple(st, st == cudaStreamPerThread ? std::this_thread::get_id() : std::thread::id());
   auto it = hs.of_stream.find(key);
-  if (it != hs.of_stream.end()) return it->second;
+  if (it != hs.of_stream.end() && it->second.first == id) return it->second.second;
   const int slot = hs.take();
-  if (slot >= 0) hs.of_stream[key] = slot;
+  if (slot < 0) return -1;
+  if (it != hs.of_stream.end()) hs.retired_list.push_back(it->second.second);
+  hs.of_stream[key] = {id, slot};
   return slot;
 }
 

@@ -952,6 +952,8 @@ const Variant &current_variant() { return t_variant; }
 VariantScope::VariantScope(const Variant &v) : saved(t_variant) { t_variant = v; }
 VariantScope::~VariantScope() { t_variant = saved; }
 
+static std::recursive_mutex &g_enqueue_mu = *new std::recursive_mutex;
+
 // Slices per group when a plan runs its passes group by group
 // (T213_SLICE_GROUP_MB: the group's size in MB; unset or 0: all slices in
 // one group).  Every pass of a group runs before the next group starts, so a
@@ -970,6 +972,15 @@ int run_plan(const Plan &P, char *data, cudaStream_t st, LaunchStats *ls) {
   const int64_t slice_bytes = P.d1 * P.d2 * P.eb;
   VariantScope vs(P.var);
   const int64_t group = slice_group(P);
+  // The launches of a call that keeps something in the stream's workspace from
+  // one to the next are enqueued together: another thread's call on the same
+  // stream would use the same bytes in between.
+  std::unique_lock<std::recursive_mutex> together(g_enqueue_mu, std::defer_lock);
+  for (const PassDesc &p : P.passes)
+    if (p.type == PT_RAGGED || (p.type == PT_SEG && p.table && p.table->n_carry > 0)) {
+      together.lock();
+      break;
+    }
   for (int64_t k0 = 0; k0 < P.d3; k0 += group) {
     const int64_t g = std::min<int64_t>(group, P.d3 - k0);
     char *gd = data + k0 * slice_bytes;
