@@ -726,6 +726,10 @@ static int batch_enqueue(t213_batch B, cudaStream_t st) {
     int rc = hold_rounds_launch(B->rounds, B->d_status, st);
     if (rc) return rc;
   }
+  if (B->spill_ws) {  // the largest at once: the plans, captured one after the other, share it
+    int rc = T213_OK;
+    if (!workspace(fork ? B->side : st, B->spill_ws, &rc)) return rc;
+  }
   for (int i : B->spill) {
     int rc = run_plan(*B->plans[i], (char *)B->tensors[i].data, fork ? B->side : st, nullptr);
     if (rc) return rc;
@@ -748,7 +752,6 @@ int t213_batch_execute(t213_batch B, t213_stream_t stream) {
   if (!B->spill.empty()) {
     int rc = T213_OK;
     const cudaStream_t ws_stream = B->serial ? st : B->side;
-    if (B->spill_ws && !workspace(ws_stream, B->spill_ws, &rc)) return rc;
     for (int i : B->spill)
       for (const PassDesc &q : B->plans[i]->passes) {
         CycleTable *ct = q.table ? q.table.get() : q.ragged.table.get();
@@ -882,6 +885,7 @@ int t213_batch_destroy(t213_batch B) {
   if (B->fork) cudaEventDestroy(B->fork);
   if (B->join) cudaEventDestroy(B->join);
   delete B;
+  release_kept();  // the graph's scratch
   return T213_OK;
 }
 

@@ -39,11 +39,31 @@ int *device_status_word(int *status);
 // ------------------------------------------------------------- workspace --
 // Grow-only scratch buffer per (device, stream).  Calls on one stream run in
 // order, so they can share it; calls on different streams never do.
+// While a stream captures, the buffer belongs to the graph and what is
+// instantiated from it.
 char *workspace(cudaStream_t st, size_t bytes, int *status);
-// Whether the stream's workspace already holds this many bytes.
-bool workspace_ready(cudaStream_t st, size_t bytes);
 // Frees the workspace of one stream (before the stream is destroyed).
 void release_stream_workspace(cudaStream_t st);
+
+// Whether st is capturing, and into which graph; its capture's id (optional).
+bool capturing(cudaStream_t st, cudaGraph_t *graph, unsigned long long *id);
+// Keeps `what` as long as a graph, its instantiations and their launches last.
+int keep_with_graph(cudaGraph_t graph, std::shared_ptr<void> what);
+// Lets go of what graphs that are gone have kept (outside captures).
+void release_kept();
+// In its scope the thread may allocate and query events although a stream
+// captures; neither touches the capturing stream.
+struct CaptureRelaxed {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  CaptureRelaxed();
+  ~CaptureRelaxed();
+};
+struct GraphBuffer {
+  int dev = 0;
+  char *p = nullptr;
+  size_t bytes = 0;
+  ~GraphBuffer();
+};
 
 // Device memory that kernels in flight on any stream may still read (cycle
 // tables of evicted plans) is not freed at once: cudaFree does not promise to

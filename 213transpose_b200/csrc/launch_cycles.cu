@@ -238,6 +238,16 @@ int CycleTable::ensure_uploaded(cudaStream_t st) {
   if (n_chunks == 0) return T213_OK;
   if (d_chunks) {
     if (ready_seen) return T213_OK;
+    cudaGraph_t graph = nullptr;
+    if (capturing(st, &graph, nullptr)) {
+      // a capture may hold no wait for an event from outside it: see the
+      // upload land here
+      CaptureRelaxed relaxed;
+      const cudaError_t w = cudaEventSynchronize(ready);
+      if (w != cudaSuccess) return cuda_status(w, "cycle table upload");
+      ready_seen = true;
+      return T213_OK;
+    }
     cudaError_t q = cudaEventQuery(ready);
     if (q == cudaSuccess) {
       ready_seen = true;

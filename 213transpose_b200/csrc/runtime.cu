@@ -59,8 +59,137 @@ std::mutex g_ws_mu;
 std::map<std::pair<int, cudaStream_t>, std::pair<char *, size_t>> g_ws;
 }  // namespace
 
+CaptureRelaxed::CaptureRelaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+CaptureRelaxed::~CaptureRelaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+
+bool capturing(cudaStream_t st, cudaGraph_t *graph, unsigned long long *id) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamGetCaptureInfo_v2(st, &cs, id, graph, nullptr, nullptr) != cudaSuccess) {
+    cudaGetLastError();  // the legacy stream while another one captures
+    return false;
+  }
+  return cs == cudaStreamCaptureStatusActive;
+}
+
+namespace {
+// What graphs that are gone have kept.  Their callbacks may make no CUDA call,
+// so it is let go by a later call outside a capture, or a buffer is taken by
+// a later capture.
+struct Graveyard {
+  std::mutex mu;
+  std::vector<std::shared_ptr<void>> kept;
+  std::vector<std::shared_ptr<GraphBuffer>> buffers;
+  std::atomic<bool> any{false};
+};
+Graveyard &graveyard() {
+  static auto &g = *new Graveyard;  // never destroyed: graphs may outlive statics
+  return g;
+}
+
+struct Kept {
+  std::shared_ptr<void> what;
+  std::shared_ptr<GraphBuffer> buffer;
+};
+
+void CUDART_CB graph_gone(void *p) {
+  auto *k = (Kept *)p;
+  Graveyard &g = graveyard();
+  {
+    std::lock_guard<std::mutex> lk(g.mu);
+    if (k->what) g.kept.push_back(std::move(k->what));
+    if (k->buffer) g.buffers.push_back(std::move(k->buffer));
+    g.any.store(true, std::memory_order_release);
+  }
+  delete k;
+}
+
+int keep(cudaGraph_t graph, Kept what) {
+  auto *k = new Kept(std::move(what));
+  cudaUserObject_t obj = nullptr;
+  cudaError_t e = cudaUserObjectCreate(&obj, k, graph_gone, 1, cudaUserObjectNoDestructorSync);
+  if (e != cudaSuccess) {
+    graph_gone(k);
+    return cuda_status(e, "cudaUserObjectCreate");
+  }
+  e = cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove);
+  if (e != cudaSuccess) {
+    cudaUserObjectRelease(obj, 1);  // runs graph_gone
+    return cuda_status(e, "cudaGraphRetainUserObject");
+  }
+  return T213_OK;
+}
+
+// Buffers of captures in progress: of a stream's newest capture, by its id.
+struct CapturedBuffer {
+  unsigned long long id;
+  char *p;
+  size_t bytes;
+};
+std::map<std::pair<int, cudaStream_t>, CapturedBuffer> g_captured;
+
+// A captured call's scratch belongs to the graph: a replay may run beside the
+// stream's own calls, and long after the stream's workspace has moved.  The
+// calls captured on one stream run in order and share one.
+char *captured_workspace(cudaStream_t st, cudaGraph_t graph, unsigned long long id, size_t bytes, int *status) {
+  const int dev = dev_info().id;
+  std::lock_guard<std::mutex> lk(g_ws_mu);
+  auto it = g_captured.find({dev, st});
+  if (it != g_captured.end() && it->second.id == id && it->second.bytes >= bytes) return it->second.p;
+  std::shared_ptr<GraphBuffer> b;
+  {
+    Graveyard &g = graveyard();
+    std::lock_guard<std::mutex> lk2(g.mu);
+    for (auto &old : g.buffers)
+      if (old->dev == dev && old->bytes >= bytes) {
+        b = std::move(old);
+        old = std::move(g.buffers.back());
+        g.buffers.pop_back();
+        break;
+      }
+  }
+  if (!b) {
+    b = std::make_shared<GraphBuffer>();
+    b->dev = dev;
+    b->bytes = (bytes + 255) & ~(size_t)255;
+    CaptureRelaxed relaxed;
+    cudaError_t e = cudaMalloc(&b->p, b->bytes);
+    if (e != cudaSuccess) {
+      *status = cuda_status(e, "workspace cudaMalloc");
+      return nullptr;
+    }
+  }
+  const CapturedBuffer c{id, b->p, b->bytes};
+  if ((*status = keep(graph, Kept{nullptr, std::move(b)}))) return nullptr;
+  g_captured[{dev, st}] = c;
+  return c.p;
+}
+}  // namespace
+
+GraphBuffer::~GraphBuffer() {
+  if (p) cudaFree(p);  // its graph and every launch of it are gone
+}
+
+int keep_with_graph(cudaGraph_t graph, std::shared_ptr<void> what) { return keep(graph, Kept{std::move(what), nullptr}); }
+
+void release_kept() {
+  Graveyard &g = graveyard();
+  if (!g.any.load(std::memory_order_acquire)) return;
+  std::vector<std::shared_ptr<void>> kept;
+  std::vector<std::shared_ptr<GraphBuffer>> buffers;
+  {
+    std::lock_guard<std::mutex> lk(g.mu);
+    kept.swap(g.kept);
+    buffers.swap(g.buffers);
+    g.any.store(false, std::memory_order_release);
+  }
+}
+
 char *workspace(cudaStream_t st, size_t bytes, int *status) {
   const int dev = dev_info().id;
+  cudaGraph_t graph = nullptr;
+  unsigned long long id = 0;
+  if (capturing(st, &graph, &id)) return captured_workspace(st, graph, id, bytes, status);
+  release_kept();
   std::lock_guard<std::mutex> lk(g_ws_mu);
   auto &w = g_ws[{dev, st}];
   if (w.first && w.second >= bytes) return w.first;
@@ -83,13 +212,6 @@ char *workspace(cudaStream_t st, size_t bytes, int *status) {
   w.first = p;
   w.second = want;
   return p;
-}
-
-bool workspace_ready(cudaStream_t st, size_t bytes) {
-  const int dev = dev_info().id;
-  std::lock_guard<std::mutex> lk(g_ws_mu);
-  auto it = g_ws.find({dev, st});
-  return bytes == 0 || (it != g_ws.end() && it->second.first && it->second.second >= bytes);
 }
 
 // A variable of the module rather than an allocation: it is zero from the
@@ -115,6 +237,7 @@ int *device_status_word(int *status) {
 void release_stream_workspace(cudaStream_t st) {
   const int dev = dev_info().id;
   std::lock_guard<std::mutex> lk(g_ws_mu);
+  g_captured.erase({dev, st});
   auto it = g_ws.find({dev, st});
   if (it == g_ws.end()) return;
   cudaStreamSynchronize(st);
@@ -981,6 +1104,15 @@ int run_plan(const Plan &P, char *data, cudaStream_t st, LaunchStats *ls) {
       together.lock();
       break;
     }
+  // a captured launch reads its cycle table as long as the graph lives, which
+  // may be longer than the plan stays cached
+  for (const PassDesc &p : P.passes) {
+    const std::shared_ptr<CycleTable> &ct = p.type == PT_RAGGED ? p.ragged.table : p.table;
+    cudaGraph_t graph = nullptr;
+    if (!ct || !capturing(st, &graph, nullptr)) continue;
+    const int rc = keep_with_graph(graph, ct);
+    if (rc) return rc;
+  }
   for (int64_t k0 = 0; k0 < P.d3; k0 += group) {
     const int64_t g = std::min<int64_t>(group, P.d3 - k0);
     char *gd = data + k0 * slice_bytes;
@@ -1493,6 +1625,7 @@ int t213_release_cache(void) {
     g_plan_lru.clear();
   }
   release_workspaces();
+  release_kept();
   flush_deferred_frees();
   return T213_OK;
 }
