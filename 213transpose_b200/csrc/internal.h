@@ -202,11 +202,14 @@ struct HoldPlan {
 };
 // we: 16-byte words per element (wide elements, eb == 16), else 1.
 void hold_plan(HoldPlan &hp, int64_t m, int64_t n, int eb, int64_t we, int64_t d3);
+// Slices whose rows, h1 x h2 of them with h1 the faster index, come in the
+// order h2 x h1: launch_slice with this h2.
+void hold_plan_swapped(HoldPlan &hp, int64_t m, int64_t n, int eb, int64_t d3);
 // launch_slice could not have all its CTAs resident, or no barrier slot is
 // left: nothing was launched, the caller takes another plan.
 constexpr int kHoldNoSlot = -2;
 int launch_slice(const HoldPlan &hp, char *data, int64_t d3, int64_t m, int64_t n, int eb, int64_t we,
-                 cudaStream_t st, LaunchStats *ls);
+                 cudaStream_t st, LaunchStats *ls, int64_t h2 = 0);
 // Slices of many tensors in rounds of one cooperative launch (the batched
 // form).  create() takes those of `which` whose slices fit a round and lists
 // them in `taken`; null without an error when there is none, or when the CTAs

@@ -37,6 +37,10 @@ constexpr int kHoldTeams = 20;    // grid teams of a launch (17 CTAs or more eac
 
 // RAG_DST / RAG_SRC: scalar tiles of one band of a ragged band plan, whose
 // output columns / source rows lie as the segments of rows with a remainder.
+// RAG_SRC also takes slices whose rows come in swapped order (two steps of a
+// rank-N permutation in one pass): row b * q + a of the output order is row
+// a * h + b of the slice, which the same two constants say, with a negative
+// remainder.
 enum HoldForm { HOLD_SCALAR = 0, HOLD_VEC = 1, HOLD_WIDE = 2, HOLD_RAG_DST = 3, HOLD_RAG_SRC = 4 };
 
 struct HoldArgs {
@@ -55,9 +59,10 @@ struct HoldArgs {
   // seg_bytes long, and rest_bytes lie between the q-th segment of a row and
   // the next row
   FastDiv<uint32_t> qdiv;
-  uint32_t nb, seg_bytes, rest_bytes;
+  uint32_t nb, seg_bytes;
+  int32_t rest_bytes;
   __device__ __forceinline__ uint64_t seg_at(uint32_t s) const {
-    return (uint64_t)s * seg_bytes + (uint64_t)qdiv.div(s) * rest_bytes;
+    return (uint64_t)((int64_t)s * seg_bytes + (int64_t)qdiv.div(s) * rest_bytes);
   }
 };
 
@@ -259,7 +264,7 @@ __device__ __forceinline__ void hold_store(char *slice, const char *from, const 
             if (q < left) *reinterpret_cast<E *>(g) = v[q];
             if constexpr (W32) {
               const bool wrap = ++col == a.qdiv.get();
-              g += (size_t)a.seg_bytes + (wrap ? a.rest_bytes : 0u);
+              g += (size_t)a.seg_bytes + (wrap ? (uint32_t)a.rest_bytes : 0u);
               if (wrap) col = 0;
             } else {
               g = slice + (size_t)((r0 + w) * EB) + a.seg_at(sj + (q + 1) * G);
@@ -657,7 +662,7 @@ __device__ __forceinline__ void tmem_drain(char *slice, const HoldArgs &a, uint3
         if (q < t.left) *reinterpret_cast<E *>(g) = v.e[q];
         if constexpr (W32) {
           const bool wrap = ++col == a.qdiv.get();
-          g += (size_t)a.seg_bytes + (wrap ? a.rest_bytes : 0u);
+          g += (size_t)a.seg_bytes + (wrap ? (uint32_t)a.rest_bytes : 0u);
           if (wrap) col = 0;
         } else {
           g = slice + (size_t)((r0 + t.w) * EB) + a.seg_at(sj + (q + 1) * t.gn);

@@ -93,7 +93,9 @@ int lanes_log2(int64_t x) {
 // (k_hold_tmem): one tile per CTA, its words in the SM's tensor
 // memory; the barrier and the latencies are then hidden from the second slice
 // on, and 1 us a slice is left.
-bool hold_search(HoldGeom &g, int64_t m, int64_t n, int eb, int64_t we, int64_t d3, int form, bool tmem = false) {
+// `bands`: the items of a slice are its bands, taken in order by one team.
+bool hold_search(HoldGeom &g, int64_t m, int64_t n, int eb, int64_t we, int64_t d3, int form, bool tmem = false,
+                 bool bands = true) {
   const DevInfo &d = dev_info();
   const int64_t E = eb * we;
   const int64_t budget = tmem ? (d.smem_optin - 128) / 128 * 128 : hold_budget();
@@ -102,7 +104,7 @@ bool hold_search(HoldGeom &g, int64_t m, int64_t n, int eb, int64_t we, int64_t 
   // tile sides in whole 32-byte sectors where the rows are
   const int64_t un = std::max<int64_t>(Q, (n * E) % 32 == 0 && E < 32 ? 32 / E : 1);
   const int64_t um = std::max<int64_t>(Q, (m * E) % 32 == 0 && E < 32 ? 32 / E : 1);
-  const bool rag = form == HOLD_RAG_DST || form == HOLD_RAG_SRC;  // one team: a slice's bands in order
+  const bool rag = bands && (form == HOLD_RAG_DST || form == HOLD_RAG_SRC);
   double best = 1e30;
   g.ok = false;
   const int64_t N4 = eb < 4 ? 4 / eb : 1;
@@ -298,10 +300,10 @@ uint32_t *hold_bars(int *status) {
 // 267 / 288 and (7402, 10752, 1) 325 / 344.  Several teams beside each other
 // already overlap, and two CTAs per SM serve them better: fp32 (1500, 1301, 8)
 // 37.8 / 34.1.
-void hold_try_tmem(HoldGeom &g, int64_t m, int64_t n, int eb, int64_t d3, int form) {
+void hold_try_tmem(HoldGeom &g, int64_t m, int64_t n, int eb, int64_t d3, int form, bool bands = true) {
   if (!g.ok || g.mode != HOLD_GRID || g.teams > 1 || d3 <= 1) return;
   HoldGeom t;
-  if (hold_search(t, m, n, eb, 1, d3, form, true) && t.tm * 4 >= std::min<uint32_t>(t.tn, 128)) g = t;
+  if (hold_search(t, m, n, eb, 1, d3, form, true, bands) && t.tm * 4 >= std::min<uint32_t>(t.tn, 128)) g = t;
 }
 
 void hold_plan(HoldPlan &hp, int64_t m, int64_t n, int eb, int64_t we, int64_t d3) {
@@ -314,6 +316,12 @@ void hold_plan(HoldPlan &hp, int64_t m, int64_t n, int eb, int64_t we, int64_t d
   hold_try_tmem(hp.any, m, n, eb, d3, HOLD_SCALAR);
   if ((eb == 2 || eb == 4) && (n * eb) % 16 == 0 && (m * eb) % 16 == 0)
     hold_search(hp.vec, m, n, eb, 1, d3, HOLD_VEC);
+}
+
+void hold_plan_swapped(HoldPlan &hp, int64_t m, int64_t n, int eb, int64_t d3) {
+  hp.ready = std::make_shared<HoldReady>();
+  hold_search(hp.any, m, n, eb, 1, d3, HOLD_RAG_SRC, false, false);
+  hold_try_tmem(hp.any, m, n, eb, d3, HOLD_RAG_SRC, false);
 }
 
 int64_t hold_cluster_bytes() { return 16 * hold_budget(); }
@@ -528,12 +536,12 @@ int launch_hold_rag(const RaggedPlan &rp, char *data, int64_t d3, int64_t slice_
   a.nb = (uint32_t)rp.q;
   a.qdiv = FastDiv<uint32_t>((uint64_t)rp.q);
   a.seg_bytes = (uint32_t)(rp.t * eb);
-  a.rest_bytes = (uint32_t)(rp.r * eb);
+  a.rest_bytes = (int32_t)(rp.r * eb);
   return hold_enqueue(f, rp.hold.any, a, data, st);
 }
 
 int launch_slice(const HoldPlan &hp, char *data, int64_t d3, int64_t m, int64_t n, int eb, int64_t we,
-                 cudaStream_t st, LaunchStats *ls) {
+                 cudaStream_t st, LaunchStats *ls, int64_t h2) {
   if (d3 <= 0 || m <= 0 || n <= 0) return T213_OK;
   const bool vec = hp.vec.ok && (uintptr_t)data % 16 == 0;
   const HoldGeom &g = vec ? hp.vec : hp.any;
@@ -548,6 +556,12 @@ int launch_slice(const HoldPlan &hp, char *data, int64_t d3, int64_t m, int64_t 
   }
   HoldArgs a = f.args;
   a.d3 = d3;
+  if (h2) {  // row b * h2 + a of the output order is row a * (m / h2) + b
+    a.nb = 1;
+    a.qdiv = FastDiv<uint32_t>((uint64_t)h2);
+    a.seg_bytes = (uint32_t)(m / h2 * n * eb);
+    a.rest_bytes = (int32_t)(n * eb - m * n * eb);
+  }
   if (f.resident == 0) return kHoldNoSlot;  // fewer SMs than the device reports (a partitioned GPU)
   // persistent: as many teams as are resident at once
   a.teams = (uint32_t)std::min<int64_t>(f.resident, d3);

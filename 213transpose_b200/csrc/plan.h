@@ -44,6 +44,8 @@ constexpr int kPlanSweeps = -1;
 constexpr int kPlanOnePassOr = -16;
 // Internal kind: the one-pass plan of elements of eb = a multiple of 16 bytes.
 constexpr int kPlanWideSlice = -2;
+// Internal kind: the one-pass plan with the rows in swapped order.
+constexpr int kPlanSwappedSlice = -4;
 // Internal kind: the automatic choice without the tuner's entries.
 constexpr int kPlanUntuned = -3;
 // Internal kind: the two-sweep plan of slices larger than the chip (PT_RAGGED).

@@ -898,7 +898,7 @@ std::shared_ptr<Plan> get_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int k
     }
   }
   std::shared_ptr<Plan> best;
-  if (kind == kPlanWideSlice) {
+  if (kind == kPlanWideSlice || kind == kPlanSwappedSlice) {
     // no passes: a slice of these elements does not fit the chip
     best = new_plan(d1, d2, d3, eb);
     best->kind = T213_PLAN_SLICE;
@@ -906,7 +906,12 @@ std::shared_ptr<Plan> get_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int k
     sp.type = PT_SLICE;
     sp.m = d2;
     sp.n = d1;
-    if (d1 * d2 * eb < (64 << 20)) hold_plan(sp.hold, d2, d1, 16, eb / 16, d3);
+    if (d1 * d2 * eb < (64 << 20)) {
+      if (kind == kPlanWideSlice)
+        hold_plan(sp.hold, d2, d1, 16, eb / 16, d3);
+      else
+        hold_plan_swapped(sp.hold, d2, d1, eb, d3);
+    }
     if (sp.hold.any.ok) best->passes.push_back(sp);
   } else if (kind != T213_PLAN_AUTO && kind != kPlanSweeps) {
     best = new_plan(d1, d2, d3, eb);
@@ -1372,6 +1377,20 @@ int t213_transpose_with_plan(void *data, int64_t d1, int64_t d2, int64_t d3, int
   return run_shape(data, d1, d2, d3, elem_bytes, plan_kind, t, (cudaStream_t)stream, 0);
 }
 
+// Two permutation steps in one pass with the rows loaded in swapped order:
+// bound by memory where the slices fill the chip, like the transposes that it
+// joins, at one sweep for two.  Over 130 random (g1, h1, h2, slices) of 0.2 to
+// 300 MB one pass took less than the two in all but a few that are kept out
+// here: many slices whose rows are below 24 bytes, a copy instruction each
+// (fp32 (4, 31, 34, 1727) 29.8 us against 27.0), or which are below 4 KB, a
+// CTA's round trip each (16-byte (3, 11, 6, 3722) 27.0 against 18.8).  Ten
+// slices a CTA are many.  B200, us, one / two: fp32 (102, 30, 1134, 16) 112 /
+// 192, f16 (104, 8, 96, 1575) 134 / 343, fp64 (30, 5, 3, 299) 8.1 / 11.7; fp32
+// (48, 60, 100, 120) reversed, three steps of which two join, 228 -> 178.
+static bool swapped_in_one_pass(int64_t row_bytes, int64_t slice_bytes, int64_t slices) {
+  return slices <= 10ll * dev_info().sms || (row_bytes >= 24 && slice_bytes >= 4096);
+}
+
 int t213_permute(void *data, int32_t rank, const int64_t *dims, const int32_t *perm, int32_t elem_bytes,
                  t213_stream_t stream) {
   if (rank < 0 || rank > 32 || (rank > 0 && (!dims || !perm))) {
@@ -1427,6 +1446,42 @@ int t213_permute(void *data, int32_t rank, const int64_t *dims, const int32_t *p
     for (int q = k + 1; q < rank; q++) g3 *= dims[cur[q]];
     int rc;
     if (E <= 16) {
+      // The next step that moves anything, when it permutes just the g2
+      // elements that now come first: [h2][h1][g1] -> [g1][h2 x h1 swapped].
+      // Where a slice fits the chip both are one pass, its rows loaded in the
+      // order in which the columns are written.
+      std::vector<int> nxt = cur;
+      std::rotate(nxt.begin() + q0, nxt.begin() + p + 1, nxt.begin() + k + 1);
+      int k2 = k - 1, p2 = q0;
+      for (; k2 > q0; k2--) {
+        p2 = q0;
+        while (nxt[p2] != perm[k2]) p2++;
+        if (p2 != k2) break;
+      }
+      int64_t h1 = 1, h2 = 1;
+      if (k2 > q0) {
+        for (int q = q0; q <= p2; q++) h1 *= dims[nxt[q]];
+        for (int q = p2 + 1; q <= k2; q++) h2 *= dims[nxt[q]];
+      }
+      if (g1 > 1 && h1 > 1 && h2 > 1 && h1 * h2 == g2 && swapped_in_one_pass(g1 * E, g1 * g2 * E, g3)) {
+        rc = check_args(data, g1, g2, g3, (int32_t)E);
+        if (!rc) rc = prefetch_if_managed(data, (size_t)(g1 * g2 * g3 * E), (cudaStream_t)stream);
+        if (rc) return rc;
+        auto P = get_plan(g1, g2, g3, (int)E, kPlanSwappedSlice, 0, &rc);
+        if (!P) return rc;
+        rc = kHoldNoSlot;
+        if (!P->passes.empty()) {
+          PassTimer tm("slice", (cudaStream_t)stream);
+          rc = launch_slice(P->passes[0].hold, (char *)data, g3, g2, g1, (int)E, 1, (cudaStream_t)stream, nullptr, h2);
+        }
+        if (rc == T213_OK) {
+          cur = nxt;
+          std::rotate(cur.begin() + q0, cur.begin() + p2 + 1, cur.begin() + k2 + 1);
+          k = k2;
+          continue;
+        }
+        if (rc != kHoldNoSlot) return rc;
+      }
       rc = run_shape(data, g1, g2, g3, (int32_t)E, T213_PLAN_AUTO, 0, (cudaStream_t)stream, 0);
     } else if (g1 == 1 || g2 == 1) {
       rc = T213_OK;  // the memory layout does not change
