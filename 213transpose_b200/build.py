@@ -31,7 +31,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I" + INCLUDE, "-I" + CSRC,
                      "--expt-relaxed-constexpr"]
 
-LIB_SOURCES = ["runtime.cu", "launch_gather.cu", "launch_cycles.cu", "launch_tiles.cu", "launch_hold.cu", "launch_ragged.cu", "host_io.cu",
+LIB_SOURCES = ["runtime.cu", "launch_gather.cu", "launch_cycles.cu", "launch_tiles.cu", "launch_hold.cu", "launch_ragged.cu", "launch_crumbs.cu", "host_io.cu",
                "tuner.cu", "batch.cu", "serve.cu", "noalloc.cu"]
 CXX_API_SOURCES = ["cxx_api.cu"]
 

@@ -177,6 +177,7 @@ bool plan_fits_batch(const Plan &p) {
         break;
       case PT_SLICE:  // launches of their own; no executor in the persistent kernel
       case PT_RAGGED:
+      case PT_CRUMBS:
         return false;
       default:
         break;
@@ -408,7 +409,7 @@ namespace t213 {
 std::shared_ptr<Plan> group_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int *status, bool search_slice) {
   std::shared_ptr<Plan> P = get_plan(d1, d2, d3, eb, T213_PLAN_AUTO, 0, status);
   if (!P) return nullptr;
-  if (P->kind == T213_PLAN_SLICE || P->kind == kPlanRagged) {
+  if (P->kind == T213_PLAN_SLICE || P->kind == kPlanRagged || P->kind == kPlanCrumbs) {
     // A caller that plans as requests arrive leaves the tensors whose one-pass
     // form is the aligned one, which run best on their own launch; the others
     // take their best plan of two sweeps or more.

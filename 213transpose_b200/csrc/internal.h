@@ -210,6 +210,12 @@ void hold_plan_swapped(HoldPlan &hp, int64_t m, int64_t n, int eb, int64_t d3);
 constexpr int kHoldNoSlot = -2;
 int launch_slice(const HoldPlan &hp, char *data, int64_t d3, int64_t m, int64_t n, int eb, int64_t we,
                  cudaStream_t st, LaunchStats *ls, int64_t h2 = 0);
+// Many small slices (k_crumbs.cuh): whether this is the kernel for them, and
+// its launch.  h2 as in launch_slice.
+constexpr int64_t kCrumbMax = 4096;  // bytes of a slice, at most
+bool crumbs_fit(int64_t m, int64_t n, int eb, int64_t d3);
+int launch_crumbs(char *data, int64_t d3, int64_t m, int64_t n, int eb, cudaStream_t st, LaunchStats *ls,
+                  int64_t h2 = 0);
 // Slices of many tensors in rounds of one cooperative launch (the batched
 // form).  create() takes those of `which` whose slices fit a round and lists
 // them in `taken`; null without an error when there is none, or when the CTAs

@@ -673,6 +673,7 @@ HoldRounds *hold_rounds_create(const t213_tensor_desc *tensors, const std::vecto
     const bool vec = (eb == 2 || eb == 4) && (d.d1 * eb) % 16 == 0 && (d.d2 * eb) % 16 == 0 && (uintptr_t)d.data % 16 == 0;
     const int64_t sb = d.d1 * d.d2 * eb;
     HoldGeom g;
+    if (crumbs_fit(d.d2, d.d1, eb, d.d3)) continue;  // a tile each would be far too many
     // small slices take tiles of half a buffer, so that tiles of several fit
     if (d.d1 > (1 << 30) || d.d2 > (1 << 30) ||
         !round_tiling(g, d.d2, d.d1, eb, vec ? HOLD_VEC : HOLD_SCALAR, sb < (2 << 20) ? buf / 2 : buf))

@@ -9,7 +9,7 @@
 
 namespace t213 {
 
-enum PassType { PT_COL = 1, PT_ROW = 2, PT_SEG = 3, PT_TILE = 4, PT_BAND = 5, PT_SLICE = 6, PT_RAGGED = 7 };
+enum PassType { PT_COL = 1, PT_ROW = 2, PT_SEG = 3, PT_TILE = 4, PT_BAND = 5, PT_SLICE = 6, PT_RAGGED = 7, PT_CRUMBS = 8 };
 
 struct PassDesc {
   PassType type = PT_COL;
@@ -50,6 +50,8 @@ constexpr int kPlanSwappedSlice = -4;
 constexpr int kPlanUntuned = -3;
 // Internal kind: the two-sweep plan of slices larger than the chip (PT_RAGGED).
 constexpr int kPlanRagged = 9;
+// Internal kind: the one-sweep plan of many small slices (PT_CRUMBS).
+constexpr int kPlanCrumbs = 10;
 // Builds the plan of a family (T213_PLAN_*; AUTO picks).  t = 0 lets the
 // planner choose the block/band size.  Cached per device.
 std::shared_ptr<Plan> get_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int kind, int64_t t, int *status);

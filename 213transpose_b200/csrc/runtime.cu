@@ -389,6 +389,8 @@ const char *PassDesc::name() const {
       return "slice";
     case PT_RAGGED:
       return "ragged";
+    case PT_CRUMBS:
+      return "crumbs";
   }
   return "?";
 }
@@ -447,8 +449,8 @@ double seg_eff(int64_t seg_bytes) {
 
 std::string fmt_plan(const Plan &P) {
   VariantScope vs(P.var);  // the pass descriptions show the kernels this plan's variant picks
-  static const char *kn[] = {"auto", "c2r", "r2c", "skinny", "blocks", "bands", "bands_t", "identity", "slice", "ragged"};
-  std::string s = kn[P.kind >= 0 && P.kind <= kPlanRagged ? P.kind : 0];
+  static const char *kn[] = {"auto", "c2r", "r2c", "skinny", "blocks", "bands", "bands_t", "identity", "slice", "ragged", "crumbs"};
+  std::string s = kn[P.kind >= 0 && P.kind <= kPlanCrumbs ? P.kind : 0];
   char buf[256];
   if (P.t) {
     snprintf(buf, sizeof buf, " t=%lld", (long long)P.t);
@@ -470,6 +472,9 @@ std::string fmt_plan(const Plan &P) {
         break;
       case PT_SLICE:
         snprintf(buf, sizeof buf, "%s", describe_slice(p.hold).c_str());
+        break;
+      case PT_CRUMBS:
+        snprintf(buf, sizeof buf, "crumbs(%lldB)", (long long)(p.m * p.n * P.eb));
         break;
       case PT_RAGGED:
         snprintf(buf, sizeof buf, "%s(q=%lld r=%lld seg=%lldB chunks=%lld carry=%lld) %s", p.ragged.cols ? "cols" : "rows",
@@ -679,6 +684,15 @@ int build_plan(Plan &P, int kind, int64_t t) {
       P.passes.push_back(sp);
       return T213_OK;
     }
+    case kPlanCrumbs: {
+      if (!crumbs_fit(m, n, eb, d3)) return T213_ERR_UNSUPPORTED;
+      PassDesc cp;
+      cp.type = PT_CRUMBS;
+      cp.m = m;
+      cp.n = n;
+      P.passes.push_back(cp);
+      return T213_OK;
+    }
     case kPlanRagged: {
       PassDesc rp;
       rp.type = PT_RAGGED;
@@ -763,6 +777,7 @@ double plan_cost(const Plan &P) {
         c += 1 / 0.5;
         break;
       case PT_SLICE:
+      case PT_CRUMBS:
         c += 1 / 0.6;
         break;
       case PT_RAGGED:
@@ -919,6 +934,8 @@ std::shared_ptr<Plan> get_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int k
     if (kind <= kPlanOnePassOr) {
       if (d1 == 1 || d2 == 1)
         st = build_plan(*best, T213_PLAN_IDENTITY, 0);
+      else if (crumbs_fit(d2, d1, eb, d3))
+        st = build_plan(*best, kPlanCrumbs, 0);
       else if (d1 * d2 * eb < (64 << 20))  // above the shared memory of any chip
         st = build_plan(*best, T213_PLAN_SLICE, 0);
     }
@@ -972,7 +989,11 @@ std::shared_ptr<Plan> get_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int k
       // to 4 MB: such a launch starts only when the whole chip is free of
       // other streams' kernels, for a gain of a few us.
       bool one_pass = false;  // a slice fits the chip
-      if (kind == T213_PLAN_AUTO) {
+      if (kind == T213_PLAN_AUTO && crumbs_fit(m, n, eb, d3)) {
+        best = new_plan(d1, d2, d3, eb);
+        build_plan(*best, kPlanCrumbs, 0);
+        best->est_cost = plan_cost(*best);
+      } else if (kind == T213_PLAN_AUTO) {
         auto P = new_plan(d1, d2, d3, eb);
         if (build_plan(*P, T213_PLAN_SLICE, 0) == T213_OK) {
           one_pass = true;
@@ -1146,6 +1167,9 @@ int run_plan(const Plan &P, char *data, cudaStream_t st, LaunchStats *ls) {
             auto alt = get_plan(P.d1, P.d2, g, P.eb, P.fallback, 0, &rc);
             if (alt) rc = run_plan(*alt, gd, st, ls);
           }
+          break;
+        case PT_CRUMBS:
+          rc = launch_crumbs(gd, g, p.m, p.n, P.eb, st, ls);
           break;
         case PT_SLICE:
           rc = launch_slice(p.hold, gd, g, p.m, p.n, P.eb, 1, st, ls);
@@ -1463,14 +1487,20 @@ int t213_permute(void *data, int32_t rank, const int64_t *dims, const int32_t *p
         for (int q = q0; q <= p2; q++) h1 *= dims[nxt[q]];
         for (int q = p2 + 1; q <= k2; q++) h2 *= dims[nxt[q]];
       }
-      if (g1 > 1 && h1 > 1 && h2 > 1 && h1 * h2 == g2 && swapped_in_one_pass(g1 * E, g1 * g2 * E, g3)) {
+      const bool joined = g1 > 1 && h1 > 1 && h2 > 1 && h1 * h2 == g2;
+      // the rows of a column lie h1 rows apart there
+      const bool crumbs = joined && crumbs_fit(h2, h1 * g1, (int)E, g3);
+      if (crumbs || (joined && swapped_in_one_pass(g1 * E, g1 * g2 * E, g3))) {
         rc = check_args(data, g1, g2, g3, (int32_t)E);
         if (!rc) rc = prefetch_if_managed(data, (size_t)(g1 * g2 * g3 * E), (cudaStream_t)stream);
         if (rc) return rc;
-        auto P = get_plan(g1, g2, g3, (int)E, kPlanSwappedSlice, 0, &rc);
-        if (!P) return rc;
+        std::shared_ptr<Plan> P;
+        if (!crumbs && !(P = get_plan(g1, g2, g3, (int)E, kPlanSwappedSlice, 0, &rc))) return rc;
         rc = kHoldNoSlot;
-        if (!P->passes.empty()) {
+        if (crumbs) {
+          PassTimer tm("crumbs", (cudaStream_t)stream);
+          rc = launch_crumbs((char *)data, g3, g2, g1, (int)E, (cudaStream_t)stream, nullptr, h2);
+        } else if (!P->passes.empty()) {
           PassTimer tm("slice", (cudaStream_t)stream);
           rc = launch_slice(P->passes[0].hold, (char *)data, g3, g2, g1, (int)E, 1, (cudaStream_t)stream, nullptr, h2);
         }

@@ -195,7 +195,7 @@ int t213_tune_shape(void *scratch_data, int64_t d1, int64_t d2, int64_t d3, int3
   {
     int rc = T213_OK;
     auto P = get_plan(d1, d2, d3, elem_bytes, kPlanUntuned, 0, &rc);
-    if (P && P->kind == kPlanRagged && time_plan(kPlanUntuned, 0, Variant{}, nullptr) < best_ms) {
+    if (P && (P->kind == kPlanRagged || P->kind == kPlanCrumbs) && time_plan(kPlanUntuned, 0, Variant{}, nullptr) < best_ms) {
       best = Entry{T213_PLAN_AUTO, 0, 0};
       found = true;
     }
