@@ -1406,13 +1406,15 @@ int t213_transpose_with_plan(void *data, int64_t d1, int64_t d2, int64_t d3, int
 // joins, at one sweep for two.  Over 130 random (g1, h1, h2, slices) of 0.2 to
 // 300 MB one pass took less than the two in all but a few that are kept out
 // here: many slices whose rows are below 24 bytes, a copy instruction each
-// (fp32 (4, 31, 34, 1727) 29.8 us against 27.0), or which are below 4 KB, a
-// CTA's round trip each (16-byte (3, 11, 6, 3722) 27.0 against 18.8).  Ten
-// slices a CTA are many.  B200, us, one / two: fp32 (102, 30, 1134, 16) 112 /
-// 192, f16 (104, 8, 96, 1575) 134 / 343, fp64 (30, 5, 3, 299) 8.1 / 11.7; fp32
-// (48, 60, 100, 120) reversed, three steps of which two join, 228 -> 178.
-static bool swapped_in_one_pass(int64_t row_bytes, int64_t slice_bytes, int64_t slices) {
-  return slices <= 10ll * dev_info().sms || (row_bytes >= 24 && slice_bytes >= 4096);
+// (fp32 (4, 31, 34, 1727) 29.8 us against 27.0), or which are small, a CTA's
+// round trip each: below 4 KB (16-byte (3, 11, 6, 3722) 27.0 against 18.8),
+// below 12 KB where the second step is k_crumbs's (fp32 (40, 24, 2, 14855) 134
+// against 80).  Ten slices an SM are many.  B200, us, one / two: fp32 (102, 30,
+// 1134, 16) 112 / 192, f16 (104, 8, 96, 1575) 134 / 343, fp64 (30, 5, 3, 299)
+// 8.1 / 11.7; fp32 (48, 60, 100, 120) reversed, three steps of which two join,
+// 228 -> 178.
+static bool swapped_in_one_pass(int64_t row_bytes, int64_t slice_bytes, int64_t slices, bool second_crumbs) {
+  return slices <= 10ll * dev_info().sms || (row_bytes >= 24 && slice_bytes >= (second_crumbs ? 12 << 10 : 4 << 10));
 }
 
 int t213_permute(void *data, int32_t rank, const int64_t *dims, const int32_t *perm, int32_t elem_bytes,
@@ -1490,7 +1492,7 @@ int t213_permute(void *data, int32_t rank, const int64_t *dims, const int32_t *p
       const bool joined = g1 > 1 && h1 > 1 && h2 > 1 && h1 * h2 == g2;
       // the rows of a column lie h1 rows apart there
       const bool crumbs = joined && crumbs_fit(h2, h1 * g1, (int)E, g3);
-      if (crumbs || (joined && swapped_in_one_pass(g1 * E, g1 * g2 * E, g3))) {
+      if (crumbs || (joined && swapped_in_one_pass(g1 * E, g1 * g2 * E, g3, crumbs_fit(h2, h1, (int)E, g3 * g1)))) {
         rc = check_args(data, g1, g2, g3, (int32_t)E);
         if (!rc) rc = prefetch_if_managed(data, (size_t)(g1 * g2 * g3 * E), (cudaStream_t)stream);
         if (rc) return rc;
