@@ -173,7 +173,7 @@ __device__ __forceinline__ void hold_load(const char *slice, const HoldArgs &a, 
 
 // `slice` is where the columns go, `from` where the rows came from (hold_load's
 // `slice`), s0 the band's first segment.
-template <int EB, int FORM>
+template <int EB, int FORM, bool ROUNDS = false>
 __device__ __forceinline__ void hold_store(char *slice, const char *from, const HoldArgs &a, uint32_t r0, uint32_t c0,
                                            const unsigned char *s, uint32_t s0) {
   using E = typename ElemT<EB>::type;
@@ -228,7 +228,9 @@ __device__ __forceinline__ void hold_store(char *slice, const char *from, const 
     // at fixed offsets, then U stores.  Steps are N columns apart, so that the
     // output rows of a unit start at the same byte of a 4-byte word.
     constexpr uint32_t N = EB < 4 ? 4 / EB : 1;
-    constexpr uint32_t U = EB == 16 ? 4 : EB == 4 ? 16 : 8;
+    // ROUNDS: the arguments take registers there, and 16 reads spill (a batch of
+    // 64 tensors, 630 MB, 431 us with 16, 426 with 8)
+    constexpr uint32_t U = EB == 16 ? 4 : EB == 4 && !ROUNDS ? 16 : 8;
     auto units = [&](auto whole) {
     // `whole`: the 32 lanes share a column
     constexpr bool W32 = decltype(whole)::value;
@@ -840,7 +842,7 @@ __device__ __noinline__ void round_store(const RoundTensor &t, const RoundTile &
   const HoldArgs a = t.a;
   const uint32_t tr = a.tcdiv.div(ti.tile);
   char *slice = t.data + (int64_t)ti.slice * a.slice_bytes;
-  hold_store<EB, FORM>(slice, slice, a, tr * a.tm, (ti.tile - tr * a.TC) * a.tn, buf + ti.off, 0);
+  hold_store<EB, FORM, true>(slice, slice, a, tr * a.tm, (ti.tile - tr * a.TC) * a.tn, buf + ti.off, 0);
 }
 
 __global__ void __launch_bounds__(kHoldThreads, 2)
