@@ -20,6 +20,10 @@ const std::string &last_error();
 // Turns a CUDA error into T213_ERR_CUDA with a message.
 int cuda_status(cudaError_t e, const char *where);
 
+// What every entry point asks of a tensor: sizes, element size, a pointer
+// aligned to it, a volume within 64 bits.  T213_OK, or a status with a message.
+int check_args(const void *data, int64_t d1, int64_t d2, int64_t d3, int32_t eb);
+
 // ---------------------------------------------------------------- device --
 struct DevInfo {
   int id = 0;

@@ -1186,15 +1186,6 @@ int run_plan(const Plan &P, char *data, cudaStream_t st, LaunchStats *ls) {
   return T213_OK;
 }
 
-}  // namespace t213
-
-// =========================================================================
-// C ABI
-// =========================================================================
-using namespace t213;
-
-namespace {
-
 int check_args(const void *data, int64_t d1, int64_t d2, int64_t d3, int32_t eb) {
   if (d1 < 0 || d2 < 0 || d3 < 0) {
     set_error("negative dimension");
@@ -1219,6 +1210,15 @@ int check_args(const void *data, int64_t d1, int64_t d2, int64_t d3, int32_t eb)
   }
   return T213_OK;
 }
+
+}  // namespace t213
+
+// =========================================================================
+// C ABI
+// =========================================================================
+using namespace t213;
+
+namespace {
 
 int prefetch_if_managed(void *data, size_t bytes, cudaStream_t st) {
   cudaPointerAttributes at;

@@ -1,0 +1,28 @@
+"""Descriptors that t213_batch_create refuses, on the host, before it plans or
+allocates anything: data that is not aligned to its element size, NULL data and
+volumes past 64 bits, as the plain call refuses them.  The kernels access whole
+elements, so such a tensor must never reach one."""
+import ctypes
+
+import pytest
+
+BASE = 1 << 20
+
+
+def _create(t213, *descs):
+    arr = (t213._lib.TensorDesc * len(descs))(*[t213._lib.TensorDesc(*d) for d in descs])
+    h = ctypes.c_void_p(0)
+    return t213.lib().t213_batch_create(arr, len(descs), ctypes.byref(h)), h.value
+
+
+@pytest.mark.parametrize("eb", (2, 4, 8, 16))
+def test_misaligned_data_is_refused(t213, eb):
+    status, handle = _create(t213, (BASE + eb // 2, 33, 17, 3, eb, 0))
+    assert status == 1 and not handle
+    assert b"aligned" in t213.lib().t213_last_error()
+
+
+def test_one_bad_descriptor_refuses_the_batch(t213):
+    ok = [(BASE + (i << 20), 64, 48, 2, 4, 0) for i in range(4)]
+    for bad in ((BASE + 2, 64, 48, 2, 4, 0), (0, 64, 48, 2, 4, 0), (BASE, 1 << 31, 1 << 31, 4, 8, 0)):
+        assert _create(t213, *ok, bad) == (1, None)
