@@ -45,7 +45,17 @@ int *device_status_word(int *status);
 // order, so they can share it; calls on different streams never do.
 // While a stream captures, the buffer belongs to the graph and what is
 // instantiated from it.
-char *workspace(cudaStream_t st, size_t bytes, int *status);
+//
+// A call keeps bytes there from one of its launches to the next, so its
+// launches are enqueued together: between them another thread's call on the
+// same stream would use the same bytes, or free the buffer for a larger one.
+// WorkspaceUse is held from workspace() to the last launch that uses the
+// buffer; it does not nest.
+struct WorkspaceUse {
+  std::unique_lock<std::mutex> lk;
+  WorkspaceUse();
+};
+char *workspace(const WorkspaceUse &use, cudaStream_t st, size_t bytes, int *status);
 // Frees the workspace of one stream (before the stream is destroyed).
 void release_stream_workspace(cudaStream_t st);
 

@@ -6,6 +6,7 @@
 // so the walk spreads over the whole GPU.  Tables are cached per permutation and device
 // and uploaded once; they are the "precomputed cycle leaders" of the pass.
 #include <algorithm>
+#include <optional>
 #include <cstdlib>
 #include <cstdio>
 #include <list>
@@ -319,6 +320,7 @@ int launch_seg_cycles(const CycleTable &ct, char *data, int64_t d3, int64_t slic
   const DevInfo &d = dev_info();
   int status = T213_OK;
   char *carry = nullptr;
+  std::optional<WorkspaceUse> use;  // to the end of the call: carries are saved, then walked
   const size_t cb = seg_cycles_carry_bytes(ct, d3, seg_bytes);
   if (ct.n_carry > 0) {
     if (carry_override) {
@@ -328,7 +330,7 @@ int launch_seg_cycles(const CycleTable &ct, char *data, int64_t d3, int64_t slic
       }
       carry = carry_override;
     } else {
-      carry = workspace(st, cb, &status);
+      carry = workspace(use.emplace(), st, cb, &status);
       if (!carry) return status;
     }
   }

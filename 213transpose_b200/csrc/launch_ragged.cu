@@ -1,6 +1,7 @@
 // Launches of the ragged band plan: the remainder, the segment cycles and the
 // bands (see RaggedPlan).
 #include <algorithm>
+#include <optional>
 
 #include "internal.h"
 #include "k_walk.cuh"
@@ -144,7 +145,8 @@ int launch_ragged(const RaggedPlan &rp, char *data, int64_t d3, int64_t m, int64
   if (rc) return rc;
   if (ct.n_chunks > 0 && (rc = ct.ensure_uploaded(st))) return rc;
   char *ws = nullptr;
-  if (need && !(ws = workspace(st, need, &rc))) return rc;
+  std::optional<WorkspaceUse> use;  // to the end of the call
+  if (need && !(ws = workspace(use.emplace(), st, need, &rc))) return rc;
   char *carry = ws + tail_bytes(rp, eb, d3);
   if (rp.r > 0 && (rc = tail(rp, true, data, ws, d3, m, n, eb, st, ls))) return rc;
   if (rp.cols && (rc = walk(rp, data, carry, d3, m, n, eb, st, ls))) return rc;

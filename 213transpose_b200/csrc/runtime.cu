@@ -184,7 +184,11 @@ void release_kept() {
   }
 }
 
-char *workspace(cudaStream_t st, size_t bytes, int *status) {
+static std::mutex &g_enqueue_mu = *new std::mutex;  // never destroyed: threads may outlive statics
+
+WorkspaceUse::WorkspaceUse() : lk(g_enqueue_mu) {}
+
+char *workspace(const WorkspaceUse &, cudaStream_t st, size_t bytes, int *status) {
   const int dev = dev_info().id;
   cudaGraph_t graph = nullptr;
   unsigned long long id = 0;
@@ -1101,8 +1105,6 @@ const Variant &current_variant() { return t_variant; }
 VariantScope::VariantScope(const Variant &v) : saved(t_variant) { t_variant = v; }
 VariantScope::~VariantScope() { t_variant = saved; }
 
-static std::recursive_mutex &g_enqueue_mu = *new std::recursive_mutex;
-
 // Slices per group when a plan runs its passes group by group
 // (T213_SLICE_GROUP_MB: the group's size in MB; unset or 0: all slices in
 // one group).  Every pass of a group runs before the next group starts, so a
@@ -1121,15 +1123,6 @@ int run_plan(const Plan &P, char *data, cudaStream_t st, LaunchStats *ls) {
   const int64_t slice_bytes = P.d1 * P.d2 * P.eb;
   VariantScope vs(P.var);
   const int64_t group = slice_group(P);
-  // The launches of a call that keeps something in the stream's workspace from
-  // one to the next are enqueued together: another thread's call on the same
-  // stream would use the same bytes in between.
-  std::unique_lock<std::recursive_mutex> together(g_enqueue_mu, std::defer_lock);
-  for (const PassDesc &p : P.passes)
-    if (p.type == PT_RAGGED || (p.type == PT_SEG && p.table && p.table->n_carry > 0)) {
-      together.lock();
-      break;
-    }
   // a captured launch reads its cycle table as long as the graph lives, which
   // may be longer than the plan stays cached
   for (const PassDesc &p : P.passes) {
