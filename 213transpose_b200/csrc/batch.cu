@@ -727,7 +727,8 @@ static int batch_enqueue(t213_batch B, cudaStream_t st) {
   }
   if (B->spill_ws) {  // the largest at once: the plans, captured one after the other, share it
     int rc = T213_OK;
-    if (!workspace(WorkspaceUse(), fork ? B->side : st, B->spill_ws, &rc)) return rc;
+    WorkspaceUse use;
+    if (!workspace(use, fork ? B->side : st, B->spill_ws, &rc)) return rc;
   }
   for (int i : B->spill) {
     int rc = run_plan(*B->plans[i], (char *)B->tensors[i].data, fork ? B->side : st, nullptr);

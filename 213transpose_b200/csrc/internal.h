@@ -42,7 +42,8 @@ int *device_status_word(int *status);
 
 // ------------------------------------------------------------- workspace --
 // Grow-only scratch buffer per (device, stream).  Calls on one stream run in
-// order, so they can share it; calls on different streams never do.
+// order, so they can share it; calls on different streams never do, and each
+// thread's per-thread default stream (one handle for all) is its own.
 // While a stream captures, the buffer belongs to the graph and what is
 // instantiated from it.
 //
@@ -51,11 +52,15 @@ int *device_status_word(int *status);
 // same stream would use the same bytes, or free the buffer for a larger one.
 // WorkspaceUse is held from workspace() to the last launch that uses the
 // buffer; it does not nest.
+struct Workspace;
 struct WorkspaceUse {
   std::unique_lock<std::mutex> lk;
+  Workspace *w = nullptr;  // the buffer in use (none of a capture)
+  cudaStream_t st = nullptr;
   WorkspaceUse();
+  ~WorkspaceUse();  // notes on st where its use of the buffer ends
 };
-char *workspace(const WorkspaceUse &use, cudaStream_t st, size_t bytes, int *status);
+char *workspace(WorkspaceUse &use, cudaStream_t st, size_t bytes, int *status);
 // Frees the workspace of one stream (before the stream is destroyed).
 void release_stream_workspace(cudaStream_t st);
 

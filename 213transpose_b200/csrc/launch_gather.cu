@@ -820,7 +820,7 @@ int launch_col_gather(const FnSpec &f, char *data, int64_t d3, int64_t m, int64_
         }
         // scratch fallback
         const int64_t gw_max = c.group_w;
-        const WorkspaceUse use;
+        WorkspaceUse use;
         char *scr = workspace(use, st, (size_t)(m * gw_max * eb), &status);
         if (!scr) return true;
         auto kern = k_col_gather_scratch<EB, AW, F, U>;
@@ -945,7 +945,7 @@ int launch_row_gather(const FnSpec &f, char *data, int64_t d3, int64_t m, int64_
         }
         // scratch fallback: groups of whole rows
         const int64_t row_bytes = n * EB;
-        const WorkspaceUse use;
+        WorkspaceUse use;
         char *scr = workspace(use, st, (size_t)(r.group_rows * row_bytes), &status);
         if (!scr) return true;
         auto kern = k_row_gather_scratch<EB, AW, F, U>;

@@ -8,6 +8,7 @@
 #include <cstring>
 #include <list>
 #include <map>
+#include <thread>
 #include <tuple>
 
 #include "plan.h"
@@ -56,7 +57,33 @@ const DevInfo &dev_info() {
 // --------------------------------------------------------------- workspace --
 namespace {
 std::mutex g_ws_mu;
-std::map<std::pair<int, cudaStream_t>, std::pair<char *, size_t>> g_ws;
+// Streams by device and handle, the per-thread default stream also by thread.
+using StreamKey = std::tuple<int, cudaStream_t, std::thread::id>;
+StreamKey stream_key(int dev, cudaStream_t st) {
+  return {dev, st, st == cudaStreamPerThread ? std::this_thread::get_id() : std::thread::id()};
+}
+}  // namespace
+
+struct Workspace {
+  char *p = nullptr;
+  size_t bytes = 0;
+  // A handle, or a thread's id, comes back for another stream after its first
+  // one was destroyed, whose last use of the buffer may still run: the new
+  // stream then waits for `last`.
+  unsigned long long id = 0;
+  cudaEvent_t last = nullptr;
+};
+
+namespace {
+std::map<StreamKey, Workspace> g_ws;
+
+void free_workspace(Workspace &w) {
+  if (w.last) {
+    cudaEventSynchronize(w.last);
+    cudaEventDestroy(w.last);
+  }
+  if (w.p) cudaFree(w.p);
+}
 }  // namespace
 
 CaptureRelaxed::CaptureRelaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
@@ -125,7 +152,7 @@ struct CapturedBuffer {
   char *p;
   size_t bytes;
 };
-std::map<std::pair<int, cudaStream_t>, CapturedBuffer> g_captured;
+std::map<StreamKey, CapturedBuffer> g_captured;
 
 // A captured call's scratch belongs to the graph: a replay may run beside the
 // stream's own calls, and long after the stream's workspace has moved.  The
@@ -133,7 +160,7 @@ std::map<std::pair<int, cudaStream_t>, CapturedBuffer> g_captured;
 char *captured_workspace(cudaStream_t st, cudaGraph_t graph, unsigned long long id, size_t bytes, int *status) {
   const int dev = dev_info().id;
   std::lock_guard<std::mutex> lk(g_ws_mu);
-  auto it = g_captured.find({dev, st});
+  auto it = g_captured.find(stream_key(dev, st));
   if (it != g_captured.end() && it->second.id == id && it->second.bytes >= bytes) return it->second.p;
   std::shared_ptr<GraphBuffer> b;
   {
@@ -160,7 +187,7 @@ char *captured_workspace(cudaStream_t st, cudaGraph_t graph, unsigned long long 
   }
   const CapturedBuffer c{id, b->p, b->bytes};
   if ((*status = keep(graph, Kept{nullptr, std::move(b)}))) return nullptr;
-  g_captured[{dev, st}] = c;
+  g_captured[stream_key(dev, st)] = c;
   return c.p;
 }
 }  // namespace
@@ -188,34 +215,47 @@ static std::mutex &g_enqueue_mu = *new std::mutex;  // never destroyed: threads 
 
 WorkspaceUse::WorkspaceUse() : lk(g_enqueue_mu) {}
 
-char *workspace(const WorkspaceUse &, cudaStream_t st, size_t bytes, int *status) {
+WorkspaceUse::~WorkspaceUse() {
+  if (w && cudaEventRecord(w->last, st) != cudaSuccess) cudaGetLastError();  // the launches before it report
+}
+
+char *workspace(WorkspaceUse &use, cudaStream_t st, size_t bytes, int *status) {
   const int dev = dev_info().id;
   cudaGraph_t graph = nullptr;
   unsigned long long id = 0;
   if (capturing(st, &graph, &id)) return captured_workspace(st, graph, id, bytes, status);
   release_kept();
   std::lock_guard<std::mutex> lk(g_ws_mu);
-  auto &w = g_ws[{dev, st}];
-  if (w.first && w.second >= bytes) return w.first;
-  if (w.first) {
+  auto &w = g_ws[stream_key(dev, st)];
+  cudaError_t e = cudaStreamGetId(st, &id);
+  if (e == cudaSuccess && !w.last) e = cudaEventCreateWithFlags(&w.last, cudaEventDisableTiming);
+  if (e == cudaSuccess && w.p && w.id != id) e = cudaStreamWaitEvent(st, w.last, 0);
+  if (e != cudaSuccess) {
+    *status = cuda_status(e, "workspace");
+    return nullptr;
+  }
+  w.id = id;
+  use.w = &w;
+  use.st = st;
+  if (w.p && w.bytes >= bytes) return w.p;
+  if (w.p) {
     // cudaFree does not promise to wait for kernels in flight: finish the
-    // stream's earlier work (the only user of this buffer) first
-    cudaStreamSynchronize(st);
-    cudaFree(w.first);
-    w.first = nullptr;
-    w.second = 0;
+    // buffer's last use first
+    cudaEventSynchronize(w.last);
+    cudaFree(w.p);
+    w.p = nullptr;
+    w.bytes = 0;
   }
   size_t want = std::max<size_t>(bytes, (size_t)1 << 20);
   want = (want + ((size_t)1 << 20) - 1) & ~(((size_t)1 << 20) - 1);
-  char *p = nullptr;
-  cudaError_t e = cudaMalloc(&p, want);
+  e = cudaMalloc(&w.p, want);
   if (e != cudaSuccess) {
+    w.p = nullptr;
     *status = cuda_status(e, "workspace cudaMalloc");
     return nullptr;
   }
-  w.first = p;
-  w.second = want;
-  return p;
+  w.bytes = want;
+  return w.p;
 }
 
 // A variable of the module rather than an allocation: it is zero from the
@@ -240,21 +280,20 @@ int *device_status_word(int *status) {
 
 void release_stream_workspace(cudaStream_t st) {
   const int dev = dev_info().id;
-  std::lock_guard<std::mutex> lk(g_ws_mu);
-  g_captured.erase({dev, st});
-  auto it = g_ws.find({dev, st});
+  std::lock_guard<std::mutex> users(g_enqueue_mu), lk(g_ws_mu);
+  g_captured.erase(stream_key(dev, st));
+  auto it = g_ws.find(stream_key(dev, st));
   if (it == g_ws.end()) return;
-  cudaStreamSynchronize(st);
-  if (it->second.first) cudaFree(it->second.first);
+  free_workspace(it->second);
   g_ws.erase(it);
 }
 
 static void release_workspaces() {
   const int dev = dev_info().id;
-  std::lock_guard<std::mutex> lk(g_ws_mu);
+  std::lock_guard<std::mutex> users(g_enqueue_mu), lk(g_ws_mu);
   for (auto it = g_ws.begin(); it != g_ws.end();) {
-    if (it->first.first == dev) {
-      if (it->second.first) cudaFree(it->second.first);
+    if (std::get<0>(it->first) == dev) {
+      free_workspace(it->second);
       it = g_ws.erase(it);
     } else {
       ++it;

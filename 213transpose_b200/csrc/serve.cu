@@ -459,7 +459,11 @@ int t213_server_create(int64_t hbm_budget_bytes, int32_t max_inflight, int32_t n
     if ((e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking))) return fail(e, "stream");
     s->streams.push_back(st);
     int rc = T213_OK;
-    if (!workspace(WorkspaceUse(), st, (size_t)64 << 20, &rc)) {  // carries of the cycle passes
+    {
+      WorkspaceUse use;
+      workspace(use, st, (size_t)64 << 20, &rc);  // carries of the cycle passes
+    }
+    if (rc) {
       t213_server_destroy(s);
       return rc;
     }

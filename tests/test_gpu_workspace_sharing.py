@@ -1,7 +1,8 @@
 """Two host threads whose calls keep bytes in a stream's workspace between
 launches (a ragged transpose's remainder and carries, a row gather through
-scratch, a blocks plan's carries), on one stream.  Every result bit-exact
-against the oracle."""
+scratch, a blocks plan's carries), on one stream and on the threads' own
+per-thread default streams (one handle for all of them).  Every result
+bit-exact against the oracle."""
 import threading
 
 import numpy as np
@@ -10,6 +11,8 @@ import pytest
 from conftest import from_device, to_device
 
 pytestmark = pytest.mark.gpu
+
+PER_THREAD = 2  # cudaStreamPerThread
 
 # (d1, d2, element bytes, plan): remainder and carries; rows through scratch,
 # a larger workspace; carries of small segments
@@ -67,3 +70,29 @@ def _run(cuda, t213, jobs, stream_of):
 def test_threads_on_one_stream(cuda, oracle, t213):
     st = cuda.cuda.Stream()
     _run(cuda, t213, _jobs(cuda, oracle, t213), lambda i: st)
+
+
+def test_threads_on_their_per_thread_streams(cuda, oracle, t213):
+    _run(cuda, t213, _jobs(cuda, oracle, t213), lambda i: PER_THREAD)
+
+
+def test_a_new_stream_under_an_old_handle(cuda, oracle, t213):
+    """A destroyed stream's last call may still run when its handle, and with it
+    the workspace, comes back for a new stream."""
+    rt = pytest.importorskip("cuda.bindings.runtime")
+    jobs = _jobs(cuda, oracle, t213)
+    for rep in range(3):
+        (d1, d2, eb, plan), (src, bufs, want) = JOBS[0], jobs[0]
+        for b in bufs:
+            b.copy_(src)
+        cuda.cuda.synchronize()
+        handles = []
+        for b in bufs:
+            err, st = rt.cudaStreamCreateWithFlags(rt.cudaStreamNonBlocking)
+            assert int(err) == 0
+            handles.append(int(st))
+            t213.transpose(b, d1, d2, 1, elem_bytes=eb, stream=int(st))
+            assert int(rt.cudaStreamDestroy(st)[0]) == 0
+        cuda.cuda.synchronize()
+        for b in bufs:
+            assert np.array_equal(from_device(b), want), f"handles {handles}"
