@@ -259,7 +259,18 @@ int CycleTable::ensure_uploaded(cudaStream_t st) {
     q = cudaStreamWaitEvent(st, ready, 0);
     return q == cudaSuccess ? T213_OK : cuda_status(q, "cycle table upload wait");
   }
-  cudaError_t e = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming);
+  // A first call inside a capture uploads on a stream of its own and sees the
+  // upload land: the table must be there at the first replay, and a replay
+  // must not upload it again.
+  const bool captured = capturing(st, nullptr, nullptr);
+  std::optional<CaptureRelaxed> relaxed;
+  cudaError_t e = cudaSuccess;
+  if (captured) {
+    relaxed.emplace();
+    e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    if (e != cudaSuccess) return cuda_status(e, "cycle table upload stream");
+  }
+  e = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaMalloc(&d_chunks, h_chunks.size());
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(d_chunks, h_chunks.data(), h_chunks.size(), cudaMemcpyHostToDevice, st);
@@ -269,9 +280,16 @@ int CycleTable::ensure_uploaded(cudaStream_t st) {
       e = cudaMemcpyAsync(d_carry_items, h_carry_items.data(), h_carry_items.size(), cudaMemcpyHostToDevice, st);
   }
   if (e == cudaSuccess) e = cudaEventRecord(ready, st);
+  if (captured) {
+    const cudaError_t landed = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = landed;
+    cudaStreamDestroy(st);
+    ready_seen = e == cudaSuccess;
+    st = nullptr;
+  }
   if (e != cudaSuccess) {
     // nothing reads the tables yet; finish the stream before freeing them
-    cudaStreamSynchronize(st);
+    if (!captured) cudaStreamSynchronize(st);
     if (d_chunks) cudaFree(d_chunks);
     if (d_carry_items) cudaFree(d_carry_items);
     if (ready) cudaEventDestroy(ready);

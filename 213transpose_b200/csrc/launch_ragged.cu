@@ -133,13 +133,9 @@ int launch_ragged(const RaggedPlan &rp, char *data, int64_t d3, int64_t m, int64
                   LaunchStats *ls) {
   if (d3 <= 0) return T213_OK;
   // Everything that can fail is asked for before the first kernel touches the
-  // tensor.  A first call inside a capture cannot upload the table: it takes
-  // the plan that needs none.
-  cudaGraph_t graph = nullptr;
-  const bool captured = capturing(st, &graph, nullptr);
+  // tensor.
   const size_t need = ragged_workspace(rp, eb, d3);
   CycleTable &ct = *rp.table;
-  if (captured && ct.n_chunks > 0 && !ct.d_chunks) return kHoldNoSlot;
   int slot = -1;
   int rc = hold_rag_ready(rp, eb, st, &slot);
   if (rc) return rc;
