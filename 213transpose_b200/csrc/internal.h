@@ -265,7 +265,7 @@ struct PermSpec {
   }
 };
 
-struct CycleTable {
+struct CycleTable : std::enable_shared_from_this<CycleTable> {
   PermSpec spec;
   int64_t n_chunks = 0, n_carry = 0, moved = 0, n_cycles = 0, max_len = 0;
   std::vector<char> h_chunks, h_carry_items;  // host copies (Chunk[], CarryItem[])
@@ -282,6 +282,9 @@ struct CycleTable {
   cudaEvent_t ready = nullptr;
   cudaStream_t upload_stream = nullptr;
   bool ready_seen = false;
+  // Asked for before every launch that reads the table.  A captured launch
+  // reads it as long as the graph lives, which may be longer than any plan
+  // stays cached: the graph keeps the table.
   int ensure_uploaded(cudaStream_t st);
   // Blocks the host until the upload has landed (set-up paths that capture
   // graphs afterwards call this so captured work needs no event wait).

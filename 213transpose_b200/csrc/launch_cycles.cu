@@ -237,10 +237,15 @@ std::shared_ptr<CycleTable> get_cycle_table(const PermSpec &p, int64_t items_per
 int CycleTable::ensure_uploaded(cudaStream_t st) {
   std::lock_guard<std::mutex> lk(mu);
   if (n_chunks == 0) return T213_OK;
+  cudaGraph_t graph = nullptr;
+  const bool captured = capturing(st, &graph, nullptr);
+  if (captured) {
+    const int rc = keep_with_graph(graph, shared_from_this());
+    if (rc) return rc;
+  }
   if (d_chunks) {
     if (ready_seen) return T213_OK;
-    cudaGraph_t graph = nullptr;
-    if (capturing(st, &graph, nullptr)) {
+    if (captured) {
       // a capture may hold no wait for an event from outside it: see the
       // upload land here
       CaptureRelaxed relaxed;
@@ -262,7 +267,6 @@ int CycleTable::ensure_uploaded(cudaStream_t st) {
   // A first call inside a capture uploads on a stream of its own and sees the
   // upload land: the table must be there at the first replay, and a replay
   // must not upload it again.
-  const bool captured = capturing(st, nullptr, nullptr);
   std::optional<CaptureRelaxed> relaxed;
   cudaError_t e = cudaSuccess;
   if (captured) {

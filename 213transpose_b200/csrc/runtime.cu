@@ -1162,15 +1162,6 @@ int run_plan(const Plan &P, char *data, cudaStream_t st, LaunchStats *ls) {
   const int64_t slice_bytes = P.d1 * P.d2 * P.eb;
   VariantScope vs(P.var);
   const int64_t group = slice_group(P);
-  // a captured launch reads its cycle table as long as the graph lives, which
-  // may be longer than the plan stays cached
-  for (const PassDesc &p : P.passes) {
-    const std::shared_ptr<CycleTable> &ct = p.type == PT_RAGGED ? p.ragged.table : p.table;
-    cudaGraph_t graph = nullptr;
-    if (!ct || !capturing(st, &graph, nullptr)) continue;
-    const int rc = keep_with_graph(graph, ct);
-    if (rc) return rc;
-  }
   for (int64_t k0 = 0; k0 < P.d3; k0 += group) {
     const int64_t g = std::min<int64_t>(group, P.d3 - k0);
     char *gd = data + k0 * slice_bytes;

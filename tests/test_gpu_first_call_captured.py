@@ -37,3 +37,27 @@ def test_first_call_captured(cuda, oracle, t213, case):
         st.synchronize()
     assert np.array_equal(from_device(dev), want)
     assert t213.device_status() == 0
+
+
+def test_captured_permutation_keeps_its_table(cuda, oracle, t213):
+    """A permutation's segment step reads its cycle table at every replay: the
+    graph keeps it when 256 later tables have pushed it out of the cache."""
+    dims, perm = (128, 40, 60, 3), (0, 2, 1, 3)  # segments of 512 bytes
+    x = oracle.random_bits(int(np.prod(dims)), 4, 9)
+    want = oracle.seq_tt(x.view(np.dtype((np.void, 4))), list(dims), list(perm)).view(np.uint8)
+    dev = to_device(cuda, x)
+    st = cuda.cuda.Stream()
+    cuda.cuda.synchronize()
+    with cuda.cuda.stream(st):
+        g = cuda.cuda.CUDAGraph()
+        with cuda.cuda.graph(g, stream=st):
+            t213.permute(dev, dims, perm, elem_bytes=4)
+    for k in range(300):
+        assert "segment_cycles" in t213.describe(16, 8 * (k + 100), 1, 4, "bands", 8)
+    t213.release_cache()
+    filler = [cuda.full((1 << 18,), -1, dtype=cuda.int32, device="cuda") for _ in range(16)]
+    with cuda.cuda.stream(st):
+        g.replay()
+        st.synchronize()
+    assert np.array_equal(from_device(dev), want)
+    del filler
