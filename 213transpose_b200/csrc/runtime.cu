@@ -201,6 +201,9 @@ int keep_with_graph(cudaGraph_t graph, std::shared_ptr<void> what) { return keep
 void release_kept() {
   Graveyard &g = graveyard();
   if (!g.any.load(std::memory_order_acquire)) return;
+  // another thread may be capturing: a free in this one's default mode would
+  // invalidate its capture
+  CaptureRelaxed relaxed;
   std::vector<std::shared_ptr<void>> kept;
   std::vector<std::shared_ptr<GraphBuffer>> buffers;
   {
