@@ -35,6 +35,9 @@ struct DevInfo {
   int l2_bytes = 0;
 };
 const DevInfo &dev_info();  // the current device, cached
+// SMs that kernels on this stream may take: those of its green context where
+// it has one, else the device's; 0 where that cannot be told.
+int stream_sms(cudaStream_t st);
 
 // Per-device status word written by kernels whose bounded waits ran out
 // (T213_ERR_TIMEOUT); read and cleared by t213_device_status.
@@ -224,8 +227,9 @@ void hold_plan(HoldPlan &hp, int64_t m, int64_t n, int eb, int64_t we, int64_t d
 // Slices whose rows, h1 x h2 of them with h1 the faster index, come in the
 // order h2 x h1: launch_slice with this h2.
 void hold_plan_swapped(HoldPlan &hp, int64_t m, int64_t n, int eb, int64_t d3);
-// launch_slice could not have all its CTAs resident, or no barrier slot is
-// left: nothing was launched, the caller takes another plan.
+// launch_slice could not have all its CTAs resident on the stream's SMs, or no
+// barrier slot is left: the tensor was not touched, the caller takes another
+// plan.
 constexpr int kHoldNoSlot = -2;
 int launch_slice(const HoldPlan &hp, char *data, int64_t d3, int64_t m, int64_t n, int eb, int64_t we,
                  cudaStream_t st, LaunchStats *ls, int64_t h2 = 0);
@@ -322,7 +326,7 @@ bool ragged_geometry(RaggedPlan &rp, int64_t m, int64_t n, int eb, int64_t d3);
 int ragged_table(RaggedPlan &rp, int eb, int64_t d3);  // builds the cycle table
 size_t ragged_workspace(const RaggedPlan &rp, int eb, int64_t d3);
 int ragged_launches(const RaggedPlan &rp);
-// kHoldNoSlot: nothing was launched, the caller takes another plan.
+// kHoldNoSlot: the tensor was not touched, the caller takes another plan.
 int launch_ragged(const RaggedPlan &rp, char *data, int64_t d3, int64_t m, int64_t n, int eb, cudaStream_t st,
                   LaunchStats *ls);
 // The band pass of a ragged plan (launch_hold.cu), and whether it could run

@@ -22,7 +22,8 @@ struct HoldReady {
     HoldArgs args{};
     const void *kern = nullptr;
     int64_t smem = 0;
-    int resident = 1;  // teams resident at once
+    int resident = 1;  // teams resident at once (grid teams: on all SMs of the device)
+    int per_sm = 1;    // grid teams: CTAs resident on an SM
     uint32_t *bars = nullptr;
     int *status = nullptr;
   } any, vec;
@@ -424,15 +425,22 @@ int hold_prepare(HoldReady::Form &f, const HoldGeom &g, int64_t m, int64_t n, in
   if (g.mode == HOLD_GRID) {
     f.bars = hold_bars(&status);
     if (!f.bars) return status;
-    int per_sm = 1;
-    occupancy_cached(f.kern, g.tmem ? kTmemThreads : kHoldThreads, f.smem, 1, &per_sm);
-    f.resident = (int64_t)per_sm * dev_info().sms >= (int64_t)g.teams * g.ctas ? (int)g.teams : 0;
+    occupancy_cached(f.kern, g.tmem ? kTmemThreads : kHoldThreads, f.smem, 1, &f.per_sm);
+    f.resident = (int)g.teams;
   } else {
     occupancy_cached(f.kern, kHoldThreads, f.smem, (int)g.ctas, &f.resident);
     if (g.mode == HOLD_CTA) f.resident *= dev_info().sms;
     f.resident = std::max(1, f.resident);
   }
   return T213_OK;
+}
+
+// Teams resident at once on the SMs that the stream has.  Clusters of more
+// than the portable 8 CTAs are kept to streams that have them all.
+int hold_resident(const HoldReady::Form &f, const HoldGeom &g, cudaStream_t st) {
+  if (g.mode == HOLD_CLUSTER && g.ctas > 8 && stream_sms(st) < dev_info().sms) return 0;
+  if (g.mode != HOLD_GRID) return f.resident;
+  return (int)std::min<int64_t>(f.resident, (int64_t)f.per_sm * stream_sms(st) / g.ctas);
 }
 
 int hold_enqueue(const HoldReady::Form &f, const HoldGeom &g, HoldArgs &a, char *data, cudaStream_t st) {
@@ -520,7 +528,7 @@ int hold_rag_ready(const RaggedPlan &rp, int eb, cudaStream_t st, int *slot) {
   const int64_t m = rp.cols ? rp.small : rp.t, n = rp.cols ? rp.t : rp.small;
   const int rc = hold_form_ready(r, r.any, rp.hold.any, m, n, eb, 1);
   if (rc) return rc;
-  if (r.any.resident == 0) return kHoldNoSlot;
+  if (hold_resident(r.any, rp.hold.any, st) == 0) return kHoldNoSlot;
   *slot = hold_slot(st);
   return *slot < 0 ? kHoldNoSlot : T213_OK;
 }
@@ -562,9 +570,9 @@ int launch_slice(const HoldPlan &hp, char *data, int64_t d3, int64_t m, int64_t 
     a.seg_bytes = (uint32_t)(m / h2 * n * eb);
     a.rest_bytes = (int32_t)(n * eb - m * n * eb);
   }
-  if (f.resident == 0) return kHoldNoSlot;  // fewer SMs than the device reports (a partitioned GPU)
   // persistent: as many teams as are resident at once
-  a.teams = (uint32_t)std::min<int64_t>(f.resident, d3);
+  a.teams = (uint32_t)std::min<int64_t>(hold_resident(f, g, st), d3);
+  if (a.teams == 0) return kHoldNoSlot;  // a stream of a few of the device's SMs
   if (g.mode == HOLD_GRID) {
     a.slot = hold_slot(st);
     if (a.slot < 0) return kHoldNoSlot;

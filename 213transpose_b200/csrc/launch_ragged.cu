@@ -146,7 +146,12 @@ int launch_ragged(const RaggedPlan &rp, char *data, int64_t d3, int64_t m, int64
   char *carry = ws + tail_bytes(rp, eb, d3);
   if (rp.r > 0 && (rc = tail(rp, true, data, ws, d3, m, n, eb, st, ls))) return rc;
   if (rp.cols && (rc = walk(rp, data, carry, d3, m, n, eb, st, ls))) return rc;
-  if ((rc = launch_hold_rag(rp, data, d3, m * n * eb, eb, slot, st))) return rc;
+  rc = launch_hold_rag(rp, data, d3, m * n * eb, eb, slot, st);
+  if (rc == kHoldNoSlot && rp.cols) {  // no other plan may run on the walked segments
+    set_error("the bands' cooperative launch was refused after the segments had moved");
+    return T213_ERR_CUDA;
+  }
+  if (rc) return rc;
   if (ls) ls->launches++;
   if (!rp.cols && (rc = walk(rp, data, carry, d3, m, n, eb, st, ls))) return rc;
   if (rp.r > 0) return tail(rp, false, data, ws, d3, m, n, eb, st, ls);

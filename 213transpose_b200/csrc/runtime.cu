@@ -11,6 +11,8 @@
 #include <thread>
 #include <tuple>
 
+#include <cudaTypedefs.h>
+
 #include "plan.h"
 
 namespace t213 {
@@ -52,6 +54,35 @@ const DevInfo &dev_info() {
   if (cudaDeviceGetAttribute(&v, cudaDevAttrL2CacheSize, dev) == cudaSuccess) d.l2_bytes = v;
   cudaGetLastError();
   return cache.emplace(dev, d).first->second;
+}
+
+// Through the runtime's driver entry point (no link against libcuda).
+int stream_sms(cudaStream_t st) {
+  struct Entry {
+    PFN_cuStreamGetCtx_v12050 ctx = nullptr;
+    PFN_cuGreenCtxGetDevResource_v12040 resource = nullptr;
+  };
+  static const Entry fn = [] {
+    Entry e;
+    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+    void *p = nullptr, *r = nullptr;
+    if (cudaGetDriverEntryPointByVersion("cuStreamGetCtx", &p, 12050, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess &&
+        cudaGetDriverEntryPointByVersion("cuGreenCtxGetDevResource", &r, 12040, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess) {
+      e.ctx = (PFN_cuStreamGetCtx_v12050)p;
+      e.resource = (PFN_cuGreenCtxGetDevResource_v12040)r;
+    }
+    cudaGetLastError();
+    return e;
+  }();
+  if (!fn.ctx) return dev_info().sms;  // a driver without green contexts
+  CUcontext c = nullptr;
+  CUgreenCtx g = nullptr;
+  if (fn.ctx((CUstream)st, &c, &g) != CUDA_SUCCESS) return 0;
+  if (!g) return dev_info().sms;
+  CUdevResource r = {};
+  return fn.resource(g, &r, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS ? (int)r.sm.smCount : 0;
 }
 
 // --------------------------------------------------------------- workspace --
