@@ -579,8 +579,11 @@ int t213_batch_create(const t213_tensor_desc *tensors, int32_t count, t213_batch
       set_error("t213_batch_create: bad tensor descriptor");
       return fail(T213_ERR_INVALID_ARGUMENT);
     }
-    // NULL or misaligned data, too large a volume: refused as the plain call does
-    if (d.d1 > 0 && d.d2 > 0 && d.d3 > 0 && (rc = check_args(d.data, d.d1, d.d2, d.d3, d.elem_bytes))) return fail(rc);
+    // NULL or misaligned data, too large a volume, an unknown plan: refused as
+    // the plain call does
+    if (d.d1 > 0 && d.d2 > 0 && d.d3 > 0 &&
+        ((rc = check_args(d.data, d.d1, d.d2, d.d3, d.elem_bytes)) || (rc = check_plan_kind(d.plan_kind))))
+      return fail(rc);
     B->total_bytes += d.d1 * d.d2 * d.d3 * d.elem_bytes;
     if (d.plan_kind == T213_PLAN_AUTO && d.d1 > 1 && d.d2 > 1 && d.d3 > 0) {
       auto_tensors.push_back(i);

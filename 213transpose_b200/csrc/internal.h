@@ -23,6 +23,10 @@ int cuda_status(cudaError_t e, const char *where);
 // What every entry point asks of a tensor: sizes, element size, a pointer
 // aligned to it, a volume within 64 bits.  T213_OK, or a status with a message.
 int check_args(const void *data, int64_t d1, int64_t d2, int64_t d3, int32_t eb);
+// A plan kind that a caller may name.  The planner's internal kinds lie outside
+// that range, and some of their plans need launch arguments that only the
+// permutation has.
+int check_plan_kind(int32_t plan_kind);
 
 // ---------------------------------------------------------------- device --
 struct DevInfo {

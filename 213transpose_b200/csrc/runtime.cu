@@ -1243,6 +1243,12 @@ int run_plan(const Plan &P, char *data, cudaStream_t st, LaunchStats *ls) {
   return T213_OK;
 }
 
+int check_plan_kind(int32_t plan_kind) {
+  if (plan_kind >= T213_PLAN_AUTO && plan_kind <= T213_PLAN_SLICE) return T213_OK;
+  set_error("unknown plan kind");
+  return T213_ERR_INVALID_ARGUMENT;
+}
+
 int check_args(const void *data, int64_t d1, int64_t d2, int64_t d3, int32_t eb) {
   if (d1 < 0 || d2 < 0 || d3 < 0) {
     set_error("negative dimension");
@@ -1663,7 +1669,7 @@ int t213_scatter_permute(int32_t fn_kind, const int64_t *fn_params, int32_t n_pa
 int t213_plan_describe(int64_t d1, int64_t d2, int64_t d3, int32_t elem_bytes, int32_t plan_kind, int64_t t,
                        char *buf, size_t buflen) {
   int rc = check_args((void *)16, d1, d2, d3, elem_bytes);
-  if (rc) return rc;
+  if (rc || (rc = check_plan_kind(plan_kind))) return rc;
   if (!buf || buflen == 0) {
     set_error("buffer is NULL");
     return T213_ERR_INVALID_ARGUMENT;
@@ -1677,7 +1683,7 @@ int t213_plan_describe(int64_t d1, int64_t d2, int64_t d3, int32_t elem_bytes, i
 int t213_plan_launches(int64_t d1, int64_t d2, int64_t d3, int32_t elem_bytes, int32_t plan_kind, int64_t t,
                        int32_t *launches) {
   int rc = check_args((void *)16, d1, d2, d3, elem_bytes);
-  if (rc) return rc;
+  if (rc || (rc = check_plan_kind(plan_kind))) return rc;
   if (!launches) return T213_ERR_INVALID_ARGUMENT;
   std::shared_ptr<Plan> P = get_plan(d1, d2, d3, elem_bytes, plan_kind, t, &rc);
   if (!P) return rc;
