@@ -235,8 +235,10 @@ void hold_plan_swapped(HoldPlan &hp, int64_t m, int64_t n, int eb, int64_t d3);
 // barrier slot is left: the tensor was not touched, the caller takes another
 // plan.
 constexpr int kHoldNoSlot = -2;
+// stall_ns: a test of the bounded waits: the team barrier asks for one arrival
+// more than there are CTAs and gives up after stall_ns nanoseconds.
 int launch_slice(const HoldPlan &hp, char *data, int64_t d3, int64_t m, int64_t n, int eb, int64_t we,
-                 cudaStream_t st, LaunchStats *ls, int64_t h2 = 0);
+                 cudaStream_t st, LaunchStats *ls, int64_t h2 = 0, uint64_t stall_ns = 0);
 // Many small slices (k_crumbs.cuh): whether this is the kernel for them, and
 // its launch.  h2 as in launch_slice.
 constexpr int64_t kCrumbMax = 4096;  // bytes of a slice, at most
@@ -253,6 +255,8 @@ HoldRounds *hold_rounds_create(const t213_tensor_desc *tensors, const std::vecto
 void hold_rounds_destroy(HoldRounds *r);
 int hold_rounds_count(const HoldRounds *r);
 int hold_rounds_launch(HoldRounds *r, int *status_word, cudaStream_t st);
+// Later launches wait for an arrival that no CTA makes, at most wait_ns long.
+void hold_rounds_debug_stall(HoldRounds *r, uint64_t wait_ns);
 int64_t hold_cluster_bytes();  // shared memory of the largest team that needs no cooperative launch
 std::string describe_slice(const HoldPlan &hp);
 int64_t band_smem_limit();

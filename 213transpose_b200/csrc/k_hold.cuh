@@ -27,6 +27,7 @@
 
 #include "common.cuh"
 #include "internal.h"
+#include "team_barrier.cuh"
 #include "tma.cuh"
 
 namespace t213 {
@@ -52,6 +53,8 @@ struct HoldArgs {
   int32_t packed;             // narrow rows, one contiguous piece per tile
   int32_t bulk;               // row pieces come by bulk copies
   int32_t mode, slot;
+  uint64_t wait_ns;  // limit of a wait at the team barrier
+  uint32_t need;     // arrivals that end it: ctas (one more in a test of the limit)
   int32_t lgs;  // log2 of the lanes that share an output column
   uint32_t we;       // wide form: 16-byte words per element
   FastDiv<uint32_t> wediv, tcdiv, rbdiv;
@@ -367,51 +370,38 @@ __device__ __forceinline__ void hold_store(char *slice, const char *from, const 
   }
 }
 
-// ---- team barrier ---------------------------------------------------------------
-// Grid teams: an arrival counter and a generation word per (slot, team).  The
-// last arrival resets the counter and raises the generation, so the words
-// need no clearing between launches.  The launch is cooperative (all CTAs
-// resident); the wait is bounded all the same.
-__device__ __forceinline__ uint32_t ld_relaxed_u32(const uint32_t *p) {
-  uint32_t v;
-  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
+// ---- team barrier (team_barrier.cuh) ----------------------------------------------
 __device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t *p) {
   uint32_t v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
+struct TeamWord {
+  uint32_t *p;
+  __device__ __forceinline__ uint32_t load() const { return ld_acquire_u32(p); }
+  __device__ __forceinline__ uint32_t add1() const {
+    uint32_t old;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(p) : "memory");
+    return old;
+  }
+  __device__ __forceinline__ void store(uint32_t v) const {
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+  }
+  __device__ __forceinline__ uint32_t cas(uint32_t old, uint32_t v) const { return atomicCAS(p, old, v); }
+};
 
-__device__ __forceinline__ bool hold_grid_wait(uint32_t *bar, uint32_t ctas, uint32_t gen) {
+__device__ __forceinline__ bool hold_grid_wait(uint32_t *bar, const HoldArgs &a, uint32_t gen) {
+  const TeamWord w{bar};
   const uint64_t t0 = global_ns();
   uint32_t spins = 0;
-  while (ld_acquire_u32(bar + 1) == gen) {
-    if ((++spins & 1023u) == 0 && global_ns() - t0 > kWaitNs) {
-      // withdraw the arrival, so that the words are clear for later launches,
-      // unless the barrier completed meanwhile
-      uint32_t c = ld_relaxed_u32(bar);
-      while (c != 0 && c < ctas) {
-        const uint32_t was = atomicCAS(bar, c, c - 1);
-        if (was == c) return false;
-        c = was;
-      }
-      for (int i = 0; i < 1 << 20; i++)
-        if (ld_acquire_u32(bar + 1) != gen) return true;
-      return false;
-    }
-  }
+  while (team_gen(w.load()) == gen)
+    if ((++spins & 1023u) == 0 && global_ns() - t0 > a.wait_ns) return !team_withdraw(w, a.need, gen);
   return true;
 }
 
 // Arrives; true when this was the last arrival, which also ends the barrier.
-__device__ __forceinline__ bool hold_grid_arrive(uint32_t *bar, uint32_t ctas, uint32_t gen) {
-  uint32_t old;
-  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(bar) : "memory");
-  if (old != ctas - 1) return false;
-  asm volatile("st.relaxed.gpu.global.u32 [%0], 0;" ::"l"(bar) : "memory");
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(bar + 1), "r"(gen + 1) : "memory");
-  return true;
+__device__ __forceinline__ bool hold_grid_arrive(uint32_t *bar, const HoldArgs &a, uint32_t gen) {
+  return team_arrive(TeamWord{bar}, a.need, gen);
 }
 
 template <int EB, int FORM>
@@ -431,7 +421,7 @@ __global__ void __launch_bounds__(kHoldThreads, 2)
   uint32_t phase = 0;
   uint32_t *bar = bars ? bars + ((size_t)a.slot * kHoldTeams + team) * 8 : nullptr;
   uint32_t gen = 0;
-  if (a.mode == HOLD_GRID && threadIdx.x == 0) gen = ld_relaxed_u32(bar + 1);
+  if (a.mode == HOLD_GRID && threadIdx.x == 0) gen = team_gen(TeamWord{bar}.load());
   auto tile_pos = [&](uint32_t t, uint32_t &r0, uint32_t &c0) {
     const uint32_t tr = a.tcdiv.div(t);
     r0 = tr * a.tm;
@@ -481,8 +471,8 @@ __global__ void __launch_bounds__(kHoldThreads, 2)
       asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
     } else if (a.mode == HOLD_GRID) {
       if (threadIdx.x == 0) {
-        ok_s = hold_grid_arrive(bar, a.ctas, gen) || hold_grid_wait(bar, a.ctas, gen);
-        gen++;
+        ok_s = hold_grid_arrive(bar, a, gen) || hold_grid_wait(bar, a, gen);
+        gen += kTeamGen;
       }
       __syncthreads();
       if (!ok_s) {
@@ -732,7 +722,7 @@ __global__ void __launch_bounds__(kTmemThreads, 1)
   }
   uint32_t *bar = bars + ((size_t)a.slot * kHoldTeams + team) * 8;
   uint32_t gen = 0;
-  if (threadIdx.x == 0) gen = ld_relaxed_u32(bar + 1);
+  if (threadIdx.x == 0) gen = team_gen(TeamWord{bar}.load());
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -769,7 +759,7 @@ __global__ void __launch_bounds__(kTmemThreads, 1)
       break;
     }
     bool last = false;
-    if (threadIdx.x == 0) last = hold_grid_arrive(bar, a.ctas, gen);
+    if (threadIdx.x == 0) last = hold_grid_arrive(bar, a, gen);
     if (mine) {
       if (a.lgs == 5)
         tmem_fill<EB, FORM, true>(slice, from, a, r0, c0, smem_raw, s0, taddr);
@@ -787,8 +777,8 @@ __global__ void __launch_bounds__(kTmemThreads, 1)
       hold_loaded(&mb);
     }
     if (threadIdx.x == 0) {
-      ok_s = last || hold_grid_wait(bar, a.ctas, gen);
-      gen++;
+      ok_s = last || hold_grid_wait(bar, a, gen);
+      gen += kTeamGen;
     }
     __syncthreads();
     if (!ok_s) {
@@ -848,7 +838,7 @@ __device__ __noinline__ void round_store(const RoundTensor &t, const RoundTile &
 __global__ void __launch_bounds__(kHoldThreads, 2)
     k_hold_rounds(const RoundTensor *__restrict__ tensors, const RoundTile *__restrict__ tiles,
                   const uint32_t *__restrict__ first, uint32_t rounds, uint32_t buf_bytes, uint32_t *counter,
-                  int *status) {
+                  uint32_t extra, uint64_t wait_ns, int *status) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ int ok_s;
   __shared__ uint64_t mb;
@@ -888,12 +878,12 @@ __global__ void __launch_bounds__(kHoldThreads, 2)
     if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
     if (r + 1 < rounds) load(r + 1);
     if (threadIdx.x == 0) {
-      const uint32_t target = (r + 1) * G;
+      const uint32_t target = (r + 1) * G + extra;
       const uint64_t t0 = global_ns();
       uint32_t spins = 0;
       int ok = 1;
       while (ld_acquire_u32(counter) < target) {
-        if ((++spins & 1023u) == 0 && global_ns() - t0 > kWaitNs) {
+        if ((++spins & 1023u) == 0 && global_ns() - t0 > wait_ns) {
           ok = 0;
           break;
         }

@@ -359,6 +359,8 @@ void hold_args(HoldArgs &a, const HoldGeom &g, int64_t m, int64_t n, int eb, int
            (int64_t)g.tn * eb >= 256;
   a.tile_bytes = (uint32_t)hold_tile_bytes(g.tm, g.tn, g.P, eb, g.form, g.packed);
   a.mode = g.mode;
+  a.wait_ns = kWaitNs;
+  a.need = g.ctas;
   a.we = (uint32_t)we;
   a.wediv = FastDiv<uint32_t>((uint64_t)we);
   a.tcdiv = FastDiv<uint32_t>(g.TC);
@@ -549,7 +551,7 @@ int launch_hold_rag(const RaggedPlan &rp, char *data, int64_t d3, int64_t slice_
 }
 
 int launch_slice(const HoldPlan &hp, char *data, int64_t d3, int64_t m, int64_t n, int eb, int64_t we,
-                 cudaStream_t st, LaunchStats *ls, int64_t h2) {
+                 cudaStream_t st, LaunchStats *ls, int64_t h2, uint64_t stall_ns) {
   if (d3 <= 0 || m <= 0 || n <= 0) return T213_OK;
   const bool vec = hp.vec.ok && (uintptr_t)data % 16 == 0;
   const HoldGeom &g = vec ? hp.vec : hp.any;
@@ -577,6 +579,14 @@ int launch_slice(const HoldPlan &hp, char *data, int64_t d3, int64_t m, int64_t 
     a.slot = hold_slot(st);
     if (a.slot < 0) return kHoldNoSlot;
   }
+  if (stall_ns) {
+    if (g.mode != HOLD_GRID) {
+      set_error("the slice's team has no barrier in memory");
+      return T213_ERR_UNSUPPORTED;
+    }
+    a.wait_ns = stall_ns;
+    a.need++;
+  }
   const int rc = hold_enqueue(f, g, a, data, st);
   if (rc) return rc;
   if (ls) ls->launches++;
@@ -589,6 +599,8 @@ struct HoldRounds {
   RoundTile *d_tiles = nullptr;
   uint32_t *d_first = nullptr, *d_counter = nullptr;
   uint32_t rounds = 0, buf_bytes = 0, ctas = 0;
+  uint32_t extra = 0;          // arrivals that no CTA makes
+  uint64_t wait_ns = kWaitNs;  // limit of a wait at a round's barrier
 };
 
 namespace {
@@ -778,6 +790,11 @@ HoldRounds *hold_rounds_create(const t213_tensor_desc *tensors, const std::vecto
   return r;
 }
 
+void hold_rounds_debug_stall(HoldRounds *r, uint64_t wait_ns) {
+  r->extra = 1;
+  r->wait_ns = wait_ns;
+}
+
 int hold_rounds_count(const HoldRounds *r) { return (int)r->rounds; }
 
 int hold_rounds_launch(HoldRounds *r, int *status_word, cudaStream_t st) {
@@ -794,7 +811,8 @@ int hold_rounds_launch(HoldRounds *r, int *status_word, cudaStream_t st) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   e = cudaLaunchKernelEx(&cfg, k_hold_rounds, (const RoundTensor *)r->d_tensors, (const RoundTile *)r->d_tiles,
-                         (const uint32_t *)r->d_first, r->rounds, r->buf_bytes, r->d_counter, status_word);
+                         (const uint32_t *)r->d_first, r->rounds, r->buf_bytes, r->d_counter, r->extra, r->wait_ns,
+                         status_word);
   return e == cudaSuccess ? T213_OK : cuda_status(e, "k_hold_rounds launch");
 }
 
