@@ -84,6 +84,7 @@ _SIGS = {
     "t213_pass_timing_read": ([ctypes.c_char_p, ctypes.POINTER(ctypes.c_double), _pi64], ctypes.c_int),
     "t213_pass_timing_reset": ([], ctypes.c_int),
     "t213_release_cache": ([], ctypes.c_int),
+    "t213_slice_debug_stall": ([_vp, _i64, _i64, _i64, _i32, _i64, _vp], ctypes.c_int),
     "t213_device_status": ([_vp, ctypes.POINTER(_i32)], ctypes.c_int),
     "t213_batch_create": ([ctypes.POINTER(TensorDesc), _i32, ctypes.POINTER(_vp)], ctypes.c_int),
     "t213_batch_execute": ([_vp, _vp], ctypes.c_int),

@@ -803,7 +803,7 @@ int t213_batch_status(t213_batch B, t213_stream_t stream) {
   if (v) {
     if (cudaMemsetAsync(B->d_status, 0, sizeof(int), (cudaStream_t)stream) == cudaSuccess)
       cudaStreamSynchronize((cudaStream_t)stream);
-    set_error("a bounded wait of the persistent batch kernel ran out");
+    set_error("a bounded wait of the batch's kernels ran out");
   }
   return v;
 }
@@ -844,17 +844,22 @@ int t213_batch_debug_stall(t213_batch B, int64_t wait_ns, int32_t stall_pass) {
   if (stall_pass < 0)
     for (size_t i = 0; i < B->h_passes.size() && stall_pass < 0; i++)
       if (B->h_passes[i].dep_ctr >= 0) stall_pass = (int32_t)i;
-  if (stall_pass < 0 || stall_pass >= (int32_t)B->h_passes.size() || B->h_passes[stall_pass].dep_ctr < 0) {
-    set_error("t213_batch_debug_stall: no pass with a dependency to stall");
+  const bool rounds = stall_pass < 0 && B->rounds;
+  if (!rounds && (stall_pass < 0 || stall_pass >= (int32_t)B->h_passes.size() || B->h_passes[stall_pass].dep_ctr < 0)) {
+    set_error("t213_batch_debug_stall: no pass with a dependency to stall, and no rounds");
     return T213_ERR_INVALID_ARGUMENT;
   }
   cudaError_t e = cudaDeviceSynchronize();  // no execute may still read the pass table
   if (e != cudaSuccess) return cuda_status(e, "t213_batch_debug_stall");
-  // one item more than the predecessor pass has: its counter never gets there
-  B->h_passes[stall_pass].dep_target += 1;
-  e = cudaMemcpy(B->d_passes + stall_pass, &B->h_passes[stall_pass], sizeof(BPass), cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) return cuda_status(e, "t213_batch_debug_stall upload");
-  B->wait_ns = (uint64_t)wait_ns;
+  if (rounds) {
+    hold_rounds_debug_stall(B->rounds, (uint64_t)wait_ns);
+  } else {
+    // one item more than the predecessor pass has: its counter never gets there
+    B->h_passes[stall_pass].dep_target += 1;
+    e = cudaMemcpy(B->d_passes + stall_pass, &B->h_passes[stall_pass], sizeof(BPass), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return cuda_status(e, "t213_batch_debug_stall upload");
+    B->wait_ns = (uint64_t)wait_ns;
+  }
   // the captured graph holds the old launch parameters
   if (B->exec) cudaGraphExecDestroy(B->exec);
   if (B->graph) cudaGraphDestroy(B->graph);

@@ -1714,6 +1714,23 @@ int t213_plan_launches(int64_t d1, int64_t d2, int64_t d3, int32_t elem_bytes, i
   return T213_OK;
 }
 
+int t213_slice_debug_stall(void *data, int64_t d1, int64_t d2, int64_t d3, int32_t elem_bytes, int64_t wait_ns,
+                           t213_stream_t stream) {
+  int rc = check_args(data, d1, d2, d3, elem_bytes);
+  if (rc) return rc;
+  if (wait_ns <= 0 || d1 < 2 || d2 < 2 || d3 < 1) {
+    set_error("t213_slice_debug_stall: bad arguments");
+    return T213_ERR_INVALID_ARGUMENT;
+  }
+  std::shared_ptr<Plan> P = get_plan(d1, d2, d3, elem_bytes, T213_PLAN_SLICE, 0, &rc);
+  if (!P) return rc;
+  rc = launch_slice(P->passes[0].hold, (char *)data, d3, d2, d1, elem_bytes, 1, (cudaStream_t)stream, nullptr, 0,
+                    (uint64_t)wait_ns);
+  if (rc != kHoldNoSlot) return rc;
+  set_error("the slice's CTAs cannot all be resident");
+  return T213_ERR_UNSUPPORTED;
+}
+
 int t213_device_status(t213_stream_t stream, int32_t *device_status) {
   if (!device_status) return T213_ERR_INVALID_ARGUMENT;
   int rc = T213_OK;

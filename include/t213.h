@@ -185,6 +185,13 @@ int t213_pass_timing_reset(void);
  * T213_OK, or T213_ERR_TIMEOUT if a kernel's bounded wait on an asynchronous
  * copy ran out since the last read. */
 int t213_device_status(t213_stream_t stream, int32_t *device_status);
+/* Test hook of the one-pass plan's failure path: runs one call of that plan on
+ * a slice large enough for a team of more than 16 CTAs, whose barrier waits for
+ * one arrival more than there are CTAs and gives up after wait_ns nanoseconds.
+ * The launch completes with the tensor untouched, and t213_device_status
+ * returns T213_ERR_TIMEOUT once.  Replaces no reference interface. */
+int t213_slice_debug_stall(void *data, int64_t d1, int64_t d2, int64_t d3, int32_t elem_bytes, int64_t wait_ns,
+                           t213_stream_t stream);
 /* Frees cached plans and workspace on the current device. */
 int t213_release_cache(void);
 
@@ -213,7 +220,9 @@ int t213_batch_describe(t213_batch batch, char *buf, size_t buflen);
 /* Test hook of the batch's failure path.  Limits every dependency wait of the
  * persistent kernel to wait_ns nanoseconds and makes pass stall_pass (-1: the
  * first pass that has a predecessor) wait for one item more than its
- * predecessor has, so that wait can only end by running out.  The next
+ * predecessor has, so that wait can only end by running out.  With -1 and
+ * tensors in rounds it is the barrier of every round that gets this limit and
+ * waits for one arrival more than there are CTAs.  The next
  * t213_batch_execute runs with these settings (a captured graph is dropped),
  * its CTAs leave on the timeout, the launch completes, and t213_batch_status
  * then returns T213_ERR_TIMEOUT once.  The batch's tensors are left partly
