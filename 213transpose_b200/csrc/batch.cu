@@ -726,6 +726,15 @@ static int batch_enqueue(t213_batch B, cudaStream_t st) {
   }
   if (B->rounds) {
     int rc = hold_rounds_launch(B->rounds, B->d_status, st);
+    if (rc == kHoldNoSlot) {  // a stream of a few of the device's SMs: their own plans
+      rc = T213_OK;
+      for (size_t i = 0; i < B->tensors.size() && !rc; i++) {
+        if (!B->in_rounds[i]) continue;
+        const t213_tensor_desc &d = B->tensors[i];
+        std::shared_ptr<Plan> P = get_plan(d.d1, d.d2, d.d3, d.elem_bytes, T213_PLAN_AUTO, 0, &rc);
+        if (P) rc = run_plan(*P, (char *)d.data, st, nullptr);
+      }
+    }
     if (rc) return rc;
   }
   if (B->spill_ws) {  // the largest at once: the plans, captured one after the other, share it

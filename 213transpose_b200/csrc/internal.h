@@ -254,6 +254,8 @@ HoldRounds *hold_rounds_create(const t213_tensor_desc *tensors, const std::vecto
                                std::vector<int> &taken, int *status);
 void hold_rounds_destroy(HoldRounds *r);
 int hold_rounds_count(const HoldRounds *r);
+// kHoldNoSlot: the CTAs would not all be resident on the stream's SMs, and
+// nothing was launched.
 int hold_rounds_launch(HoldRounds *r, int *status_word, cudaStream_t st);
 // Later launches wait for an arrival that no CTA makes, at most wait_ns long.
 void hold_rounds_debug_stall(HoldRounds *r, uint64_t wait_ns);

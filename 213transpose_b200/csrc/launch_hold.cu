@@ -798,6 +798,7 @@ void hold_rounds_debug_stall(HoldRounds *r, uint64_t wait_ns) {
 int hold_rounds_count(const HoldRounds *r) { return (int)r->rounds; }
 
 int hold_rounds_launch(HoldRounds *r, int *status_word, cudaStream_t st) {
+  if (2 * stream_sms(st) < (int)r->ctas) return kHoldNoSlot;  // two CTAs an SM
   cudaError_t e = cudaMemsetAsync(r->d_counter, 0, sizeof(uint32_t), st);
   if (e != cudaSuccess) return cuda_status(e, "batch rounds counter");
   cudaLaunchConfig_t cfg = {};
@@ -813,6 +814,10 @@ int hold_rounds_launch(HoldRounds *r, int *status_word, cudaStream_t st) {
   e = cudaLaunchKernelEx(&cfg, k_hold_rounds, (const RoundTensor *)r->d_tensors, (const RoundTile *)r->d_tiles,
                          (const uint32_t *)r->d_first, r->rounds, r->buf_bytes, r->d_counter, r->extra, r->wait_ns,
                          status_word);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    cudaGetLastError();
+    return kHoldNoSlot;
+  }
   return e == cudaSuccess ? T213_OK : cuda_status(e, "k_hold_rounds launch");
 }
 

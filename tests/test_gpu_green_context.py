@@ -71,3 +71,25 @@ def test_joined_permutation_steps_on_some_sms(cuda, oracle, t213, green_stream):
     green_stream.synchronize()
     assert np.array_equal(from_device(dev), want)
     assert t213.device_status() == 0
+
+
+def test_batch_on_some_sms(cuda, oracle, t213, green_stream):
+    """Rounds need all SMs: their tensors run their own plans there, and the
+    rounds again on a stream that has them all."""
+    shapes = [(1000, 999, 4, 4), (257, 129, 3, 2), (512, 384, 5, 4), (45, 600, 1, 16), (2000, 1999, 1, 4), (64, 48, 30, 1)]
+    hosts = [oracle.random_bits(d1 * d2 * d3, eb, 70 + i) for i, (d1, d2, d3, eb) in enumerate(shapes)]
+    dev = [to_device(cuda, x) for x in hosts]
+    b = t213.Batch([(d, *s) for d, s in zip(dev, shapes)])
+    assert "rounds: 0 of" not in b.describe()
+    try:
+        for st in (green_stream, green_stream, cuda.cuda.Stream(), green_stream):
+            for d, x in zip(dev, hosts):
+                d.copy_(cuda.from_numpy(x.view(np.uint8).reshape(-1)))
+            cuda.cuda.synchronize()
+            b.execute(st)
+            assert b.status(st) == 0
+            for d, x, (d1, d2, d3, eb) in zip(dev, hosts, shapes):
+                want = oracle.gather213(x.view(np.dtype((np.void, eb))), d1, d2, d3).view(np.uint8)
+                assert np.array_equal(from_device(d), want), (d1, d2, d3, eb)
+    finally:
+        b.close()
