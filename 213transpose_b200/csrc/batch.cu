@@ -541,6 +541,100 @@ int group_exec_run(GroupExec *g, const t213_tensor_desc *tensors, int32_t count,
 
 }  // namespace t213
 
+namespace {
+
+// ---- small slices -------------------------------------------------------------
+enum Route : char { ROUTE_ROUNDS = 0, ROUTE_PERSISTENT = 1, ROUTE_OWN = 2 };
+constexpr int64_t kSmallSlice = 128 << 10;
+constexpr int64_t kSmallItem = 256 << 10;  // bytes of an item of the persistent kernel, about
+
+// The route of each automatic tensor of `which`.  Slices of up to 128 KB are a
+// tile or two each, and the rounds spend about 2 us of a CTA on a tile however
+// small; the persistent kernel transposes a slice as one band of its own in
+// 0.4 us and more, and the tensor's own launch streams slices at up to the
+// copy rate.  So the three are estimated, in us, with constants fitted to 230
+// batches of 1-64 equal tensors on B200: rounds / the route taken, us: fp32
+// (48, 60, 300) x 16 62 / 39 persistent, (40, 64, 156) x 64 121 / 68 persistent,
+// (48, 60, 12000) x 4 570 / 198 own, fp64 (16, 16, 100000) x 4 2800 / 342 own,
+// 4 tensors of 6 KB 10.3 / 8.2 persistent; own plans / persistent, bf16
+// (20, 30, 400) x 64 209 / 108, fp32 (4, 4, 1000) x 64 135 / 414.
+std::vector<char> small_slices(const t213_tensor_desc *tensors, const std::vector<int> &which, int *status) {
+  *status = T213_OK;
+  const double sms = dev_info().sms;
+  struct Item {
+    size_t k;
+    double alt, work, last;  // on the other route; SM time in the persistent kernel, and of one of its items
+    bool rounds;
+  };
+  std::vector<char> route(which.size(), ROUTE_ROUNDS);
+  std::vector<Item> items;
+  bool others = false;  // rounds run anyway
+  for (size_t k = 0; k < which.size(); k++) {
+    const t213_tensor_desc &d = tensors[which[k]];
+    const int eb = d.elem_bytes;
+    const int64_t sb = d.d1 * d.d2 * eb;
+    if (d.d1 > kSmallSlice || d.d2 > kSmallSlice || sb > kSmallSlice) {
+      others = true;
+      continue;
+    }
+    // what both kinds of rows are aligned to, and the better of the two
+    const int64_t a1 = (d.d1 * eb) & -(d.d1 * eb), a2 = (d.d2 * eb) & -(d.d2 * eb);
+    const int64_t al = std::min(a1, a2), am = std::max(a1, a2);
+    const bool wide = eb >= 8 || al >= 8 || (eb == 2 && al >= 4 && am >= 8);  // rows move in words of several elements
+    const double n = (double)d.d3, mb = n * (double)sb * 1e-6;
+    const bool crumbs = crumbs_fit(d.d2, d.d1, eb, d.d3);
+    const double rounds = crumbs || d.d3 > 1 << 16 ? 1e30 : n * (eb == 1 ? 2.2 + (double)sb / 2800 : 1.7 + (double)sb / 4700) / (2 * sms);
+    auto P = get_plan(d.d1, d.d2, d.d3, eb, T213_PLAN_AUTO, 0, status);
+    if (!P) return route;
+    double own = 1e30;
+    if (P->passes.size() == 1 && P->passes[0].type != PT_RAGGED) {
+      const PassType type = P->passes[0].type;
+      const double per_mb = type == PT_CRUMBS  ? (eb == 1 ? 0.9 : eb == 2 ? 0.75 : 0.45)
+                            : type == PT_SLICE ? (eb == 1 ? 0.9 : 0.65)
+                            : wide             ? (eb == 1 ? 1.6 : 0.7)
+                                               : (eb == 1 ? 3.3 : eb == 2 ? 1.7 : 1.0);
+      own = (type == PT_CRUMBS ? 2.0 : 2.5) + mb * per_mb;
+    }
+    const double alt = std::min(rounds, own);
+    if (own <= rounds) route[k] = ROUTE_OWN;
+    // one band of the whole slice, if the persistent kernel's buffers hold it
+    if (n * (double)sb > (double)direct_threshold() || sb > kBatchHalf || !band_fits(d.d2, d.d1, eb)) {
+      others = others || route[k] == ROUTE_ROUNDS;
+      continue;
+    }
+    const double rate = wide      ? (eb == 1 ? 7000 : eb == 2 && al < 16 ? 10000 : eb == 8 && am < 16 ? 7000 : 15500)
+                        : eb == 4 ? (am >= 8 ? 6000 : 3200)
+                                  : (eb == 2 ? 2000 : 1200);
+    const double slice = 0.4 + (double)sb / rate;
+    items.push_back(
+        {k, alt, n * slice, std::min(n, std::max(1.0, (double)(kSmallItem / sb))) * slice, route[k] == ROUTE_ROUNDS});
+  }
+  // The persistent kernel takes those of the quickest items that gain the most
+  // together: it costs 6.5 us and its longest item, or its share of the SMs;
+  // the rounds 10.5 us when they run at all.
+  std::sort(items.begin(), items.end(), [](const Item &a, const Item &b) { return a.last < b.last; });
+  double alt = 0, work = 0, best = 0;
+  size_t take = 0;
+  int left = 0;  // of the rest, in rounds
+  for (const Item &it : items) left += it.rounds;
+  bool any = false;
+  for (size_t q = 0; q < items.size(); q++) {
+    alt += items[q].alt;
+    work += items[q].work;
+    any = any || items[q].rounds;
+    left -= items[q].rounds;
+    const double gain = alt + (any && !left && !others ? 10.5 : 0.0) - 6.5 - std::max(items[q].last, work / sms);
+    if (gain > best) {
+      best = gain;
+      take = q + 1;
+    }
+  }
+  for (size_t q = 0; q < take; q++) route[items[q].k] = ROUTE_PERSISTENT;
+  return route;
+}
+
+}  // namespace
+
 extern "C" {
 
 int t213_transpose_looped(const t213_tensor_desc *tensors, int32_t count, t213_stream_t stream) {
@@ -570,7 +664,6 @@ int t213_batch_create(const t213_tensor_desc *tensors, int32_t count, t213_batch
     return code;
   };
 
-  int64_t auto_bytes = 0;
   std::vector<int> auto_tensors;
   for (int32_t i = 0; i < count; i++) {
     const t213_tensor_desc &d = tensors[i];
@@ -585,48 +678,48 @@ int t213_batch_create(const t213_tensor_desc *tensors, int32_t count, t213_batch
         ((rc = check_args(d.data, d.d1, d.d2, d.d3, d.elem_bytes)) || (rc = check_plan_kind(d.plan_kind))))
       return fail(rc);
     B->total_bytes += d.d1 * d.d2 * d.d3 * d.elem_bytes;
-    if (d.plan_kind == T213_PLAN_AUTO && d.d1 > 1 && d.d2 > 1 && d.d3 > 0) {
-      auto_tensors.push_back(i);
-      auto_bytes += d.d1 * d.d2 * d.d3 * d.elem_bytes;
-    }
+    if (d.plan_kind == T213_PLAN_AUTO && d.d1 > 1 && d.d2 > 1 && d.d3 > 0) auto_tensors.push_back(i);
   }
 
-  // ---- rounds -------------------------------------------------------------------
+  // ---- routes -------------------------------------------------------------------
   // Tensors of the automatic choice whose slices fit a round share one launch
-  // of the one-pass kernel; the others of that choice then run their own plan
-  // after it, on the caller's stream, since both take the whole chip.
-  // Measured on B200, rounds against the persistent kernel, us: 8 tensors of
-  // 0.3 MB 12 / 86, 64 of 0.1 MB 16 / 100, 8 of 16 MB 87 / 198; the batched
-  // workload of 512 tensors 6346 / 10558.  A batch of up to three small
-  // tensors stays in the persistent kernel, whose dependency waits
-  // t213_batch_debug_stall lets run out.
+  // of the one-pass kernel; the others of that choice run their own plan after
+  // it, on the caller's stream, since both take the whole chip.  Measured on
+  // B200, rounds against the persistent kernel, us: 1 tensor of 1.6 MB 10 / 89, 8
+  // of 0.3 MB 12 / 86, 64 of 0.1 MB 16 / 100, 8 of 16 MB 87 / 198; the batched
+  // workload of 512 tensors 6346 / 10558.  Small slices may do better on
+  // either of the other routes (small_slices).
+  std::vector<char> route = small_slices(tensors, auto_tensors, &rc);
+  if (rc) return fail(rc);
   B->in_rounds.assign(count, 0);
-  B->serial = auto_tensors.size() > 3 || auto_bytes >= (8 << 20);
-  if (B->serial) {
-    std::vector<int> taken;
-    B->rounds = hold_rounds_create(tensors, auto_tensors, taken, &rc);
+  std::vector<int> taken, offered;
+  for (size_t k = 0; k < auto_tensors.size(); k++)
+    if (route[k] == ROUTE_ROUNDS) offered.push_back(auto_tensors[k]);
+  if (!offered.empty()) {
+    B->rounds = hold_rounds_create(tensors, offered, taken, &rc);
     if (rc) return fail(rc);
     for (int i : taken) B->in_rounds[i] = 1;
   }
 
   // ---- plans ---------------------------------------------------------------
+  B->plans.resize(count);
+  for (size_t k = 0; k < auto_tensors.size(); k++) {
+    const int i = auto_tensors[k];
+    const t213_tensor_desc &d = tensors[i];
+    if (B->in_rounds[i]) continue;
+    const bool persistent = route[k] == ROUTE_PERSISTENT;
+    B->plans[i] = get_plan(d.d1, d.d2, d.d3, d.elem_bytes, persistent ? T213_PLAN_BANDS : T213_PLAN_AUTO,
+                           persistent ? d.d2 : 0, &rc);
+    if (!B->plans[i]) return fail(rc);
+    if (!persistent) B->spill.push_back(i);
+  }
+  B->serial = B->rounds || !B->spill.empty();
   for (int32_t i = 0; i < count; i++) {
     const t213_tensor_desc &d = tensors[i];
-    std::shared_ptr<Plan> P;
-    if (d.d1 * d.d2 * d.d3 > 0 && !B->in_rounds[i]) {
-      if (d.plan_kind == T213_PLAN_AUTO && B->serial) {
-        P = get_plan(d.d1, d.d2, d.d3, d.elem_bytes, T213_PLAN_AUTO, 0, &rc);
-        if (!P) return fail(rc);
-        if (!P->passes.empty()) B->spill.push_back(i);
-      } else {
-        P = d.plan_kind == T213_PLAN_AUTO ? group_plan(d.d1, d.d2, d.d3, d.elem_bytes, &rc, true) : nullptr;
-        if (!P)
-          P = get_plan(d.d1, d.d2, d.d3, d.elem_bytes, d.plan_kind == T213_PLAN_AUTO ? kPlanSweeps : d.plan_kind, 0, &rc);
-        if (!P) return fail(rc);
-        if (!plan_fits_batch(*P) || d.d1 * d.d2 * d.d3 * d.elem_bytes > direct_threshold()) B->spill.push_back(i);
-      }
-    }
-    B->plans.push_back(P);
+    if (d.plan_kind == T213_PLAN_AUTO || d.d1 * d.d2 * d.d3 == 0) continue;
+    B->plans[i] = get_plan(d.d1, d.d2, d.d3, d.elem_bytes, d.plan_kind, 0, &rc);
+    if (!B->plans[i]) return fail(rc);
+    if (!plan_fits_batch(*B->plans[i]) || d.d1 * d.d2 * d.d3 * d.elem_bytes > direct_threshold()) B->spill.push_back(i);
   }
 
   std::vector<char> skip = B->in_rounds;
@@ -715,9 +808,9 @@ static int batch_enqueue(t213_batch B, cudaStream_t st) {
     if ((e = cudaEventRecord(B->fork, st)) || (e = cudaStreamWaitEvent(B->side, B->fork, 0)))
       return cuda_status(e, "batch fork");
   }
-  e = cudaMemsetAsync(B->d_ctrs, 0, (B->n_ctrs + 1) * sizeof(unsigned long long), st);
-  if (e != cudaSuccess) return cuda_status(e, "batch counters reset");
   if (!B->h_items.empty()) {
+    e = cudaMemsetAsync(B->d_ctrs, 0, (B->n_ctrs + 1) * sizeof(unsigned long long), st);
+    if (e != cudaSuccess) return cuda_status(e, "batch counters reset");
     k_batch<<<B->grid, kBatchThreads, (size_t)(kBatchSmem + kBatchBarBytes), st>>>(
         B->d_passes, B->d_items, (int64_t)B->h_items.size(), B->d_ctrs, B->d_ctrs + B->n_ctrs, B->d_status,
         B->wait_ns);
