@@ -53,8 +53,6 @@ struct HoldArgs {
   int32_t packed;             // narrow rows, one contiguous piece per tile
   int32_t bulk;               // row pieces come by bulk copies
   int32_t mode, slot;
-  uint64_t wait_ns;  // limit of a wait at the team barrier
-  uint32_t need;     // arrivals that end it: ctas (one more in a test of the limit)
   int32_t lgs;  // log2 of the lanes that share an output column
   uint32_t we;       // wide form: 16-byte words per element
   FastDiv<uint32_t> wediv, tcdiv, rbdiv;
@@ -64,6 +62,8 @@ struct HoldArgs {
   FastDiv<uint32_t> qdiv;
   uint32_t nb, seg_bytes;
   int32_t rest_bytes;
+  uint32_t need;     // arrivals that end a team barrier: ctas (one more in a test of the limit)
+  uint64_t wait_ns;  // limit of a wait there
   __device__ __forceinline__ uint64_t seg_at(uint32_t s) const {
     return (uint64_t)((int64_t)s * seg_bytes + (int64_t)qdiv.div(s) * rest_bytes);
   }
