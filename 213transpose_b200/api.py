@@ -274,7 +274,7 @@ tuner = _Tuner()
 
 
 class Batch:
-    """Many tensors transposed by one persistent, graph-captured launch
+    """Many tensors transposed by shared, graph-captured launches
     (t213_batch_*).  `tensors` is a list of (data, d1, d2, d3) or
     (data, d1, d2, d3, elem_bytes[, plan]) tuples; data are CUDA tensors or raw
     device pointers (then elem_bytes is required)."""

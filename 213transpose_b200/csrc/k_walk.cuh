@@ -18,9 +18,9 @@
 //
 // Bound by memory, in practice by the loads in flight (three pieces of 16 KB
 // a CTA, three CTAs an SM) and by the step barrier where segments are short.
-// The whole ragged transpose of fp32 (1000003, 37, 1), 148 MB, takes 138 us
+// The whole ragged transpose of fp32 (1000003, 37, 1), 148 MB, takes 136 us
 // against 587 us of the gathers through a scratch copy that it replaced; fp64
-// (101, 100003, 2) 154 against 318, bf16 (31424, 3160, 1) 216 against 1091.
+// (101, 100003, 2) 160 against 318, bf16 (31424, 3160, 1) 204 against 1091.
 #pragma once
 
 #include "common.cuh"

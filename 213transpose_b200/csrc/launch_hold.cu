@@ -296,9 +296,9 @@ uint32_t *hold_bars(int *status) {
 
 // Tensor memory as the second buffer, where one team takes slices that fill
 // more than half of the chip one after the other.  Measured on B200, with and
-// without, us: bf16 (4099, 2053, 8) 97.5 / 108.9, fp32 (3001, 2000, 4) 49.6 /
-// 51.1, fp64 (2408, 1432, 4) 52.9 / 55.8, ragged bands of fp32 (561, 62490, 2)
-// 267 / 288 and (7402, 10752, 1) 325 / 344.  Several teams beside each other
+// without, us: bf16 (4099, 2053, 8) 88.5 / 89.0, fp32 (3001, 2000, 4) 48.2 /
+// 49.4, fp64 (2408, 1432, 4) 52.1 / 53.5, ragged fp32 (561, 62490, 2) 260 / 267
+// and (7402, 10752, 1) 308 / 317.  Several teams beside each other
 // already overlap, and two CTAs per SM serve them better: fp32 (1500, 1301, 8)
 // 37.8 / 34.1.
 void hold_try_tmem(HoldGeom &g, int64_t m, int64_t n, int eb, int64_t d3, int form, bool bands = true) {
@@ -353,8 +353,8 @@ void hold_args(HoldArgs &a, const HoldGeom &g, int64_t m, int64_t n, int eb, int
   a.H = (uint32_t)hold_region(g.tm, g.P, eb, g.form);
   a.packed = g.packed;
   // bulk copies from 256 bytes a row piece: one instruction a row instead of
-  // one a 512 bytes (ragged bands of fp32 (1000003, 37, 1) 142 -> 132 us, fp32
-  // (3001, 2000, 4) 51.9 -> 51.1); shorter pieces are many small copies
+  // one a 512 bytes (without / with, us: fp32 (3001, 2000, 4) 54.1 / 48.2, ragged
+  // fp32 (1000003, 37, 1) 144 / 136); shorter pieces are many small copies
   a.bulk = !g.packed && (g.form == HOLD_SCALAR || g.form == HOLD_RAG_DST || g.form == HOLD_RAG_SRC) &&
            (int64_t)g.tn * eb >= 256;
   a.tile_bytes = (uint32_t)hold_tile_bytes(g.tm, g.tn, g.P, eb, g.form, g.packed);
@@ -607,7 +607,7 @@ namespace {
 
 // Slices of more than this share of a round run their own plan, which has
 // twice the room.  Measured on B200, shares of 0.35 / 0.5 / 0.75, us: batches
-// of 64 tensors (630 MB) 405 / 404 / 421 and 457 / 453 / 460, of 512 tensors
+// of 64 tensors 400 / 408 / 441 (630 MB) and 749 / 752 / 752, of 512 tensors
 // 6372 / 6346 / 6458.
 constexpr double kRoundShare = 0.5;
 

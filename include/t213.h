@@ -211,9 +211,10 @@ typedef struct t213_tensor_desc {
 typedef struct t213_batch_st *t213_batch;
 
 int t213_batch_create(const t213_tensor_desc *tensors, int32_t count, t213_batch *out);
-/* One launch for the whole batch (graph replay after the first call). */
+/* Everything the batch needs, enqueued on the stream (a graph replay after the
+ * first call on it). */
 int t213_batch_execute(t213_batch batch, t213_stream_t stream);
-/* Status word written by the persistent kernel (0 = ok, T213_ERR_TIMEOUT if a
+/* Status word written by the batch's own kernels (0 = ok, T213_ERR_TIMEOUT if a
  * bounded wait ran out).  Synchronises the stream. */
 int t213_batch_status(t213_batch batch, t213_stream_t stream);
 int t213_batch_describe(t213_batch batch, char *buf, size_t buflen);
@@ -230,10 +231,12 @@ int t213_batch_describe(t213_batch batch, char *buf, size_t buflen);
  * waits (src/memory_ops.cu:18-33, src/skinny.cu:31-60) are unbounded. */
 int t213_batch_debug_stall(t213_batch batch, int64_t wait_ns, int32_t stall_pass);
 int t213_batch_destroy(t213_batch batch);
-/* Autotunes every shape class present in the list (timing the applicable
- * plan families on scratch memory of the class's largest tensor) so that
- * t213_batch_create and the plain call pick the measured winner.
- * Synchronous; the tensors' data are not touched. */
+/* Autotunes every shape present in the list (timing the applicable plan
+ * families on scratch memory of the largest tensor) so that the plain call, and
+ * t213_batch_create for the tensors that run their own plans, pick the measured
+ * winner.  Tensors that share a batch's launches are not bound by it: their
+ * plan is the batch's (t213_batch_describe says how many).  Synchronous; the
+ * tensors' data are not touched. */
 int t213_batch_tune(const t213_tensor_desc *tensors, int32_t count, t213_stream_t stream);
 /* Baseline form: the plain call looped over the same list on one stream. */
 int t213_transpose_looped(const t213_tensor_desc *tensors, int32_t count, t213_stream_t stream);
