@@ -406,15 +406,14 @@ void bind_carry(std::vector<BPass> &passes, const std::vector<size_t> &carry_off
 
 namespace t213 {
 
-std::shared_ptr<Plan> group_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int *status, bool search_slice) {
+std::shared_ptr<Plan> group_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int *status) {
   std::shared_ptr<Plan> P = get_plan(d1, d2, d3, eb, T213_PLAN_AUTO, 0, status);
   if (!P) return nullptr;
   if (P->kind == T213_PLAN_SLICE || P->kind == kPlanRagged || P->kind == kPlanCrumbs) {
-    // A caller that plans as requests arrive leaves the tensors whose one-pass
-    // form is the aligned one, which run best on their own launch; the others
-    // take their best plan of two sweeps or more.
+    // Tensors whose one-pass form is the aligned one run best on their own
+    // launch; the others take their best plan of two sweeps or more.
     const bool aligned = P->kind == T213_PLAN_SLICE && (d1 * eb) % 16 == 0 && (d2 * eb) % 16 == 0 && d1 * d2 * d3 * eb <= (16ll << 20);
-    if (aligned && !search_slice) return nullptr;
+    if (aligned) return nullptr;
     P = get_plan(d1, d2, d3, eb, kPlanSweeps, 0, status);
     if (!P) return nullptr;
   }
@@ -508,7 +507,7 @@ int group_exec_run(GroupExec *g, const t213_tensor_desc *tensors, int32_t count,
     const t213_tensor_desc &d = tensors[i];
     if (d.d1 * d.d2 * d.d3 == 0) continue;
     int rc = T213_OK;
-    plans[i] = group_plan(d.d1, d.d2, d.d3, d.elem_bytes, &rc, false);
+    plans[i] = group_plan(d.d1, d.d2, d.d3, d.elem_bytes, &rc);
     if (!plans[i]) return T213_ERR_UNSUPPORTED;
   }
   BatchTables T;
@@ -584,15 +583,16 @@ std::vector<char> small_slices(const t213_tensor_desc *tensors, const std::vecto
     const double n = (double)d.d3, mb = n * (double)sb * 1e-6;
     const bool crumbs = crumbs_fit(d.d2, d.d1, eb, d.d3);
     const double rounds = crumbs || d.d3 > 1 << 16 ? 1e30 : n * (eb == 1 ? 2.2 + (double)sb / 2800 : 1.7 + (double)sb / 4700) / (2 * sms);
-    auto P = get_plan(d.d1, d.d2, d.d3, eb, T213_PLAN_AUTO, 0, status);
-    if (!P) return route;
-    double own = 1e30;
-    if (P->passes.size() == 1 && P->passes[0].type != PT_RAGGED) {
+    double own = 2.0 + mb * 0.45;  // at best: the plan itself is only asked for where that could be the route
+    if (own <= rounds) {
+      auto P = get_plan(d.d1, d.d2, d.d3, eb, T213_PLAN_AUTO, 0, status);
+      if (!P) return route;
       const PassType type = P->passes[0].type;
-      const double per_mb = type == PT_CRUMBS  ? (eb == 1 ? 0.9 : eb == 2 ? 0.75 : 0.45)
-                            : type == PT_SLICE ? (eb == 1 ? 0.9 : 0.65)
-                            : wide             ? (eb == 1 ? 1.6 : 0.7)
-                                               : (eb == 1 ? 3.3 : eb == 2 ? 1.7 : 1.0);
+      const double per_mb = P->passes.size() > 1 ? 4.0
+                            : type == PT_CRUMBS  ? (eb == 1 ? 0.9 : eb == 2 ? 0.75 : 0.45)
+                            : type == PT_SLICE   ? (eb == 1 ? 0.9 : 0.65)
+                            : wide               ? (eb == 1 ? 1.6 : 0.7)
+                                                 : (eb == 1 ? 3.3 : eb == 2 ? 1.7 : 1.0);
       own = (type == PT_CRUMBS ? 2.0 : 2.5) + mb * per_mb;
     }
     const double alt = std::min(rounds, own);

@@ -78,9 +78,8 @@ GroupExec *group_exec_create(int64_t max_passes, int64_t max_items, size_t carry
 void group_exec_destroy(GroupExec *g);
 // The plan a tensor takes inside the persistent kernel (the automatic choice,
 // else the cheapest other family whose passes fit its shared memory); null if
-// none fits, and, unless search_slice, when the automatic choice is the
-// one-pass slice plan (which runs on its own launch).
-std::shared_ptr<Plan> group_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int *status, bool search_slice);
+// none fits, and for tensors that run best on their own launch.
+std::shared_ptr<Plan> group_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int *status);
 // Enqueues one k_batch launch over the tensors on st (tables copied from the
 // executor's pinned staging, counters reset), then copies the kernel's status
 // word to the executor's host mirror and records its event.  The executor's

@@ -1055,9 +1055,10 @@ std::shared_ptr<Plan> get_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int k
       cands.push_back({T213_PLAN_BANDS_T, tc, estimate_cost(T213_PLAN_BANDS_T, m, n, tc, eb, d3)});
       // The one-pass plan (T213_PLAN_SLICE) is the fastest wherever a slice
       // fits the chip, but for four classes (B200, us).  Many slices of a few KB
-      // at most are k_crumbs's (crumbs_fit).  Square slices of whole tiles are one sweep of tile swaps without a barrier: 16-byte
-      // (1024, 1024, 4) 24.8 against 31.1, fp32 (2048, 2048, 8) 51.2 against
-      // 58.2; at 8 MB and below they tie or lose.  Many slices of less than
+      // at most are k_crumbs's (crumbs_fit).  Square slices of whole tiles are
+      // one sweep of tile swaps without a barrier: 16-byte (1024, 1024, 4) 24.8
+      // against 31.1, fp32 (2048, 2048, 8) 51.2 against 58.2; at 8 MB and below
+      // they tie or lose.  Many slices of less than
       // 32 KB are one sweep of bands or tiles that takes the next slice's load
       // ahead: fp32 (48, 60, 12000) 51 against 81, (16, 16, 20000) 20 against
       // 86, (100, 100, 1000), 40 KB, 21 either way.  A small slice that needs
