@@ -199,6 +199,8 @@ std::string describe_col_gather(int64_t m, int64_t n, int eb, const void *data);
 // The variant launch_col_gather picks for this functor (the cluster-local
 // kernel when the functor's form and the strip halo allow it).
 std::string describe_col_gather_fn(const FnSpec &f, int64_t m, int64_t n, int eb, const void *data);
+// Columns of the strips that launch_col_gather gathers with this functor.
+int64_t col_strip_width(const FnSpec &f, int64_t m, int64_t n, int eb);
 std::string describe_row_gather(int64_t m, int64_t n, int eb, const void *data);
 // Number of launches the gathers enqueue.
 int count_col_gather(int64_t d3, int64_t m, int64_t n, int eb);

@@ -579,6 +579,11 @@ std::string describe_col_gather_fn(const FnSpec &f, int64_t m, int64_t n, int eb
   return describe_col_gather(m, n, eb, data);
 }
 
+int64_t col_strip_width(const FnSpec &f, int64_t m, int64_t n, int eb) {
+  const LocalCfg lc = local_col_config(f, m, n, eb, nullptr);
+  return lc.ok ? lc.W : col_config(m, n, eb, nullptr).W;
+}
+
 std::string describe_col_gather(int64_t m, int64_t n, int eb, const void *data) {
   ColCfg c = col_config(m, n, eb, data);
   char buf[160];

@@ -816,12 +816,8 @@ int build_plan(Plan &P, int kind, int64_t t) {
 // Bytes of the column strips that a plan gathers.
 int64_t col_strip_bytes(const Plan &P) {
   int64_t w = 1 << 20;
-  for (const PassDesc &p : P.passes) {
-    if (p.type != PT_COL) continue;
-    const std::string d = describe_col_gather_fn(p.fn, p.m, p.n, P.eb, nullptr);
-    const size_t at = d.find("W=");
-    if (at != std::string::npos) w = std::min<int64_t>(w, std::atoll(d.c_str() + at + 2) * P.eb);
-  }
+  for (const PassDesc &p : P.passes)
+    if (p.type == PT_COL) w = std::min(w, col_strip_width(p.fn, p.m, p.n, P.eb) * P.eb);
   return w;
 }
 
