@@ -412,7 +412,8 @@ std::shared_ptr<Plan> group_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int
   if (P->kind == T213_PLAN_SLICE || P->kind == kPlanRagged || P->kind == kPlanCrumbs) {
     // Tensors whose one-pass form is the aligned one run best on their own
     // launch; the others take their best plan of two sweeps or more.
-    const bool aligned = P->kind == T213_PLAN_SLICE && (d1 * eb) % 16 == 0 && (d2 * eb) % 16 == 0 && d1 * d2 * d3 * eb <= (16ll << 20);
+    const bool aligned =
+        P->kind == T213_PLAN_SLICE && (d1 * eb) % 16 == 0 && (d2 * eb) % 16 == 0 && d1 * d2 * d3 * eb <= (16ll << 20);
     if (aligned) return nullptr;
     P = get_plan(d1, d2, d3, eb, kPlanSweeps, 0, status);
     if (!P) return nullptr;
@@ -582,7 +583,8 @@ std::vector<char> small_slices(const t213_tensor_desc *tensors, const std::vecto
     const bool wide = eb >= 8 || al >= 8 || (eb == 2 && al >= 4 && am >= 8);  // rows move in words of several elements
     const double n = (double)d.d3, mb = n * (double)sb * 1e-6;
     const bool crumbs = crumbs_fit(d.d2, d.d1, eb, d.d3);
-    const double rounds = crumbs || d.d3 > 1 << 16 ? 1e30 : n * (eb == 1 ? 2.2 + (double)sb / 2800 : 1.7 + (double)sb / 4700) / (2 * sms);
+    const double tile = eb == 1 ? 2.2 + (double)sb / 2800 : 1.7 + (double)sb / 4700;
+    const double rounds = crumbs || d.d3 > 1 << 16 ? 1e30 : n * tile / (2 * sms);
     double own = 2.0 + mb * 0.45;  // at best: the plan itself is only asked for where that could be the route
     if (own <= rounds) {
       auto P = get_plan(d.d1, d.d2, d.d3, eb, T213_PLAN_AUTO, 0, status);
@@ -794,8 +796,8 @@ int t213_batch_create(const t213_tensor_desc *tensors, int32_t count, t213_batch
            "batch: %d tensors, %.1f MB; persistent kernel: %d tensors, %zu passes, %zu "
            "items, grid %d x %d threads; graph nodes: %d tensors, %.1f MB; rounds: %d of %d tensors",
            count, B->total_bytes / 1e6, count - (int)B->spill.size() - n_rounds,
-           B->h_passes.size(), B->h_items.size(), B->grid, kBatchThreads, (int)B->spill.size(), direct_bytes / 1e6, B->rounds ? hold_rounds_count(B->rounds) : 0,
-           n_rounds);
+           B->h_passes.size(), B->h_items.size(), B->grid, kBatchThreads, (int)B->spill.size(), direct_bytes / 1e6,
+           B->rounds ? hold_rounds_count(B->rounds) : 0, n_rounds);
   B->desc = buf;
   *out = B;
   return T213_OK;

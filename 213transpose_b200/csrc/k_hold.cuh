@@ -235,133 +235,133 @@ __device__ __forceinline__ void hold_store(char *slice, const char *from, const 
     // 64 tensors, 630 MB, 431 us with 16, 426 with 8)
     constexpr uint32_t U = EB == 16 ? 4 : EB == 4 && !ROUNDS ? 16 : 8;
     auto units = [&](auto whole) {
-    // `whole`: the 32 lanes share a column
-    constexpr bool W32 = decltype(whole)::value;
-    const uint32_t lgs = W32 ? 5u : (uint32_t)a.lgs;
-    const uint32_t L = 1u << lgs, G = W32 ? 1u : 32u >> lgs, li = W32 ? lane : lane & (L - 1), sub = W32 ? 0u : lane >> lgs;
-    const uint32_t plo = a.n * EB;
-    const uint32_t lo = (uint32_t)(uintptr_t)from + (FORM == HOLD_RAG_SRC ? c0 * EB : (r0 * a.n + c0) * EB);
-    const uint32_t sr = s0 + r0;  // RAG_SRC: the segment of the tile's first row
-    const uint32_t words = N == 1 ? rows : (rows + 2 * N - 2) / N;  // one more covers every offset
-    const uint32_t nrb = (words + L - 1) >> lgs, ncg = (cols + U * G * N - 1) / (U * G * N) * N;
-    const bool full = rows == a.tm;
-    for (uint32_t u = warp; u < nrb * ncg; u += nw) {
-      const uint32_t cg = full ? a.rbdiv.div(u) : u / nrb;
-      const uint32_t w = ((u - cg * nrb) << lgs) + li;
-      const uint32_t j0 = cg / N * (U * G * N) + cg % N * G + sub;
-      if (w >= words || j0 >= cols) continue;
-      [[maybe_unused]] const uint32_t o = ((c0 + j0) * a.m + r0) * EB;
-      [[maybe_unused]] const uint32_t gs = G * N * a.m * EB;
-      const uint32_t ps = G * N * EB;
-      const uint32_t left = (cols - 1 - j0) / (G * N) + 1;  // column steps of this lane
-      if constexpr (N == 1) {
-        const unsigned char *p = s + hold_row<EB, FORM>(a, w, lo, plo, sr) + j0 * EB;
-        E v[U];
-        if constexpr (FORM == HOLD_RAG_DST) {
-          const uint32_t sj = s0 + c0 + j0;
-          char *g = slice + (size_t)((r0 + w) * EB) + a.seg_at(sj);
-          uint32_t col = sj - a.qdiv.div(sj) * a.qdiv.get();  // the segment's place in its row
-#pragma unroll
-          for (uint32_t q = 0; q < U; q++)
-            if (q < left) v[q] = *reinterpret_cast<const E *>(p + q * ps);
-#pragma unroll
-          for (uint32_t q = 0; q < U; q++) {
-            if (q < left) *reinterpret_cast<E *>(g) = v[q];
-            if constexpr (W32) {
-              const bool wrap = ++col == a.qdiv.get();
-              g += (size_t)a.seg_bytes + (wrap ? (uint32_t)a.rest_bytes : 0u);
-              if (wrap) col = 0;
+      // `whole`: the 32 lanes share a column
+      constexpr bool W32 = decltype(whole)::value;
+      const uint32_t lgs = W32 ? 5u : (uint32_t)a.lgs;
+      const uint32_t L = 1u << lgs, G = W32 ? 1u : 32u >> lgs, li = W32 ? lane : lane & (L - 1), sub = W32 ? 0u : lane >> lgs;
+      const uint32_t plo = a.n * EB;
+      const uint32_t lo = (uint32_t)(uintptr_t)from + (FORM == HOLD_RAG_SRC ? c0 * EB : (r0 * a.n + c0) * EB);
+      const uint32_t sr = s0 + r0;  // RAG_SRC: the segment of the tile's first row
+      const uint32_t words = N == 1 ? rows : (rows + 2 * N - 2) / N;  // one more covers every offset
+      const uint32_t nrb = (words + L - 1) >> lgs, ncg = (cols + U * G * N - 1) / (U * G * N) * N;
+      const bool full = rows == a.tm;
+      for (uint32_t u = warp; u < nrb * ncg; u += nw) {
+        const uint32_t cg = full ? a.rbdiv.div(u) : u / nrb;
+        const uint32_t w = ((u - cg * nrb) << lgs) + li;
+        const uint32_t j0 = cg / N * (U * G * N) + cg % N * G + sub;
+        if (w >= words || j0 >= cols) continue;
+        [[maybe_unused]] const uint32_t o = ((c0 + j0) * a.m + r0) * EB;
+        [[maybe_unused]] const uint32_t gs = G * N * a.m * EB;
+        const uint32_t ps = G * N * EB;
+        const uint32_t left = (cols - 1 - j0) / (G * N) + 1;  // column steps of this lane
+        if constexpr (N == 1) {
+          const unsigned char *p = s + hold_row<EB, FORM>(a, w, lo, plo, sr) + j0 * EB;
+          E v[U];
+          if constexpr (FORM == HOLD_RAG_DST) {
+            const uint32_t sj = s0 + c0 + j0;
+            char *g = slice + (size_t)((r0 + w) * EB) + a.seg_at(sj);
+            uint32_t col = sj - a.qdiv.div(sj) * a.qdiv.get();  // the segment's place in its row
+  #pragma unroll
+            for (uint32_t q = 0; q < U; q++)
+              if (q < left) v[q] = *reinterpret_cast<const E *>(p + q * ps);
+  #pragma unroll
+            for (uint32_t q = 0; q < U; q++) {
+              if (q < left) *reinterpret_cast<E *>(g) = v[q];
+              if constexpr (W32) {
+                const bool wrap = ++col == a.qdiv.get();
+                g += (size_t)a.seg_bytes + (wrap ? (uint32_t)a.rest_bytes : 0u);
+                if (wrap) col = 0;
+              } else {
+                g = slice + (size_t)((r0 + w) * EB) + a.seg_at(sj + (q + 1) * G);
+              }
+            }
+            continue;
+          }
+          char *g = slice + (size_t)(o + w * EB);
+          if (left >= U) {
+            if constexpr (W32) {  // consecutive columns: reads at constant offsets
+  #pragma unroll
+              for (uint32_t q = 0; q < U; q++) v[q] = *reinterpret_cast<const E *>(p + q * EB);
             } else {
-              g = slice + (size_t)((r0 + w) * EB) + a.seg_at(sj + (q + 1) * G);
+  #pragma unroll
+              for (uint32_t q = 0; q < U; q++) v[q] = *reinterpret_cast<const E *>(p + q * ps);
+            }
+  #pragma unroll
+            for (uint32_t q = 0; q < U; q++, g += gs) *reinterpret_cast<E *>(g) = v[q];
+          } else {
+  #pragma unroll
+            for (uint32_t q = 0; q < U; q++)
+              if (q < left) *reinterpret_cast<E *>(g + (size_t)(q * gs)) = *reinterpret_cast<const E *>(p + q * ps);
+          }
+        } else if constexpr (FORM == HOLD_RAG_DST) {
+          // the offset of an output row in its first word is the column's own:
+          // the N rows of the word are picked out of the 2 N - 1 that they can be
+          uint32_t ro[2 * N - 1];
+  #pragma unroll
+          for (uint32_t b = 0; b < 2 * N - 1; b++)
+            ro[b] = hold_row<EB, FORM>(a, min((uint32_t)max((int32_t)(w * N + b) - (int32_t)(N - 1), 0), rows - 1), lo, plo, sr);
+          const uint32_t sj = s0 + c0 + j0;
+          char *g0 = slice + (size_t)(r0 * EB);
+  #pragma unroll 4
+          for (uint32_t q = 0; q < min(left, U); q++) {
+            char *g = g0 + a.seg_at(sj + q * (G * N));
+            const uint32_t h = ((uint32_t)(uintptr_t)g & 3u) / EB, at = N - 1 - h;
+            uint32_t x[2 * N - 1];
+  #pragma unroll
+            for (uint32_t b = 0; b < 2 * N - 1; b++) x[b] = ro[b];
+  #pragma unroll
+            for (uint32_t k = 1; k < N; k *= 2) {
+  #pragma unroll
+              for (uint32_t b = 0; b + k < 2 * N - 1; b++) x[b] = at & k ? x[b + k] : x[b];
+            }
+            const unsigned char *p = s + j0 * EB + q * ps;
+            uint32_t v = 0;
+  #pragma unroll
+            for (uint32_t b = 0; b < N; b++) v |= (uint32_t) * reinterpret_cast<const E *>(p + x[b]) << (8 * EB * b);
+            const int32_t e0 = (int32_t)(w * N) - (int32_t)h;
+            g += (int64_t)e0 * EB;
+            if (e0 >= 0 && e0 + (int32_t)N <= (int32_t)rows) {
+              *reinterpret_cast<uint32_t *>(g) = v;
+            } else {
+  #pragma unroll
+              for (uint32_t b = 0; b < N; b++)
+                if ((uint32_t)(e0 + (int32_t)b) < rows) *reinterpret_cast<E *>(g + b * EB) = (E)(v >> (8 * EB * b));
             }
           }
-          continue;
-        }
-        char *g = slice + (size_t)(o + w * EB);
-        if (left >= U) {
-          if constexpr (W32) {  // consecutive columns: reads at constant offsets
-#pragma unroll
-            for (uint32_t q = 0; q < U; q++) v[q] = *reinterpret_cast<const E *>(p + q * EB);
-          } else {
-#pragma unroll
-            for (uint32_t q = 0; q < U; q++) v[q] = *reinterpret_cast<const E *>(p + q * ps);
-          }
-#pragma unroll
-          for (uint32_t q = 0; q < U; q++, g += gs) *reinterpret_cast<E *>(g) = v[q];
         } else {
-#pragma unroll
-          for (uint32_t q = 0; q < U; q++)
-            if (q < left) *reinterpret_cast<E *>(g + (size_t)(q * gs)) = *reinterpret_cast<const E *>(p + q * ps);
-        }
-      } else if constexpr (FORM == HOLD_RAG_DST) {
-        // the offset of an output row in its first word is the column's own:
-        // the N rows of the word are picked out of the 2 N - 1 that they can be
-        uint32_t ro[2 * N - 1];
-#pragma unroll
-        for (uint32_t b = 0; b < 2 * N - 1; b++)
-          ro[b] = hold_row<EB, FORM>(a, min((uint32_t)max((int32_t)(w * N + b) - (int32_t)(N - 1), 0), rows - 1), lo, plo, sr);
-        const uint32_t sj = s0 + c0 + j0;
-        char *g0 = slice + (size_t)(r0 * EB);
-#pragma unroll 4
-        for (uint32_t q = 0; q < min(left, U); q++) {
-          char *g = g0 + a.seg_at(sj + q * (G * N));
-          const uint32_t h = ((uint32_t)(uintptr_t)g & 3u) / EB, at = N - 1 - h;
-          uint32_t x[2 * N - 1];
-#pragma unroll
-          for (uint32_t b = 0; b < 2 * N - 1; b++) x[b] = ro[b];
-#pragma unroll
-          for (uint32_t k = 1; k < N; k *= 2) {
-#pragma unroll
-            for (uint32_t b = 0; b + k < 2 * N - 1; b++) x[b] = at & k ? x[b + k] : x[b];
-          }
-          const unsigned char *p = s + j0 * EB + q * ps;
-          uint32_t v = 0;
-#pragma unroll
-          for (uint32_t b = 0; b < N; b++) v |= (uint32_t) * reinterpret_cast<const E *>(p + x[b]) << (8 * EB * b);
+          const uint32_t h = (((uint32_t)(uintptr_t)slice + o) & 3u) / EB;
           const int32_t e0 = (int32_t)(w * N) - (int32_t)h;
-          g += (int64_t)e0 * EB;
-          if (e0 >= 0 && e0 + (int32_t)N <= (int32_t)rows) {
-            *reinterpret_cast<uint32_t *>(g) = v;
-          } else {
-#pragma unroll
-            for (uint32_t b = 0; b < N; b++)
-              if ((uint32_t)(e0 + (int32_t)b) < rows) *reinterpret_cast<E *>(g + b * EB) = (E)(v >> (8 * EB * b));
-          }
-        }
-      } else {
-        const uint32_t h = (((uint32_t)(uintptr_t)slice + o) & 3u) / EB;
-        const int32_t e0 = (int32_t)(w * N) - (int32_t)h;
-        const unsigned char *p[N];
-#pragma unroll
-        for (uint32_t b = 0; b < N; b++)
-          p[b] = s + hold_row<EB, FORM>(a, min((uint32_t)max(e0 + (int32_t)b, 0), rows - 1), lo, plo, sr) + j0 * EB;
-        uint32_t v[U];
-#pragma unroll
-        for (uint32_t q = 0; q < U; q++) {
-          v[q] = 0;
-          if (q < left) {
-#pragma unroll
-            for (uint32_t b = 0; b < N; b++)
-              v[q] |= (uint32_t) * reinterpret_cast<const E *>(p[b] + q * ps) << (8 * EB * b);
-          }
-        }
-        char *g = slice + (size_t)o + (int64_t)e0 * EB;
-        if (e0 >= 0 && e0 + (int32_t)N <= (int32_t)rows) {
-#pragma unroll
-          for (uint32_t q = 0; q < U; q++, g += gs)
-            if (q < left) *reinterpret_cast<uint32_t *>(g) = v[q];
-        } else {
-          // a word across the end of the column's piece: its elements one by one
-#pragma unroll
+          const unsigned char *p[N];
+  #pragma unroll
           for (uint32_t b = 0; b < N; b++)
-            if ((uint32_t)(e0 + (int32_t)b) < rows) {
-#pragma unroll
-              for (uint32_t q = 0; q < U; q++)
-                if (q < left) *reinterpret_cast<E *>(g + (size_t)(q * gs) + b * EB) = (E)(v[q] >> (8 * EB * b));
+            p[b] = s + hold_row<EB, FORM>(a, min((uint32_t)max(e0 + (int32_t)b, 0), rows - 1), lo, plo, sr) + j0 * EB;
+          uint32_t v[U];
+  #pragma unroll
+          for (uint32_t q = 0; q < U; q++) {
+            v[q] = 0;
+            if (q < left) {
+  #pragma unroll
+              for (uint32_t b = 0; b < N; b++)
+                v[q] |= (uint32_t) * reinterpret_cast<const E *>(p[b] + q * ps) << (8 * EB * b);
             }
+          }
+          char *g = slice + (size_t)o + (int64_t)e0 * EB;
+          if (e0 >= 0 && e0 + (int32_t)N <= (int32_t)rows) {
+  #pragma unroll
+            for (uint32_t q = 0; q < U; q++, g += gs)
+              if (q < left) *reinterpret_cast<uint32_t *>(g) = v[q];
+          } else {
+            // a word across the end of the column's piece: its elements one by one
+  #pragma unroll
+            for (uint32_t b = 0; b < N; b++)
+              if ((uint32_t)(e0 + (int32_t)b) < rows) {
+  #pragma unroll
+                for (uint32_t q = 0; q < U; q++)
+                  if (q < left) *reinterpret_cast<E *>(g + (size_t)(q * gs) + b * EB) = (E)(v[q] >> (8 * EB * b));
+              }
+          }
         }
       }
-    }
     };
     if (a.lgs == 5)
       units(std::true_type{});

@@ -1085,55 +1085,55 @@ std::shared_ptr<Plan> get_plan(int64_t d1, int64_t d2, int64_t d3, int eb, int k
         }
       }
       if (!best) {
-      // The Catanzaro decomposition both ways: the reference's dispatcher
-      // takes C2R when d1 >= d2, else R2C (src/transpose.cu:117-123); here
-      // both are costed, since which one keeps its rows inside shared
-      // memory decides the faster one for tall or wide slices.
-      for (int k : {T213_PLAN_C2R, T213_PLAN_R2C}) {
-        Plan tmp;
-        tmp.d1 = d1;
-        tmp.d2 = d2;
-        tmp.d3 = d3;
-        tmp.eb = eb;
-        build_plan(tmp, k, 0);
-        // ties go to the reference's choice
-        const bool ref_choice = (k == T213_PLAN_C2R) == (d1 >= d2);
-        cands.push_back({k, 0, plan_cost(tmp) * (ref_choice ? 1.0 : 1.0001)});
-      }
-      if (kind == T213_PLAN_AUTO && !one_pass) {
-        // The ragged bands against the others: the estimates of the classes
-        // that lose to them, or win, are set right here, where they are the
-        // alternative (kRaggedCost has the measurements).
-        for (Cand &c : cands) {
+        // The Catanzaro decomposition both ways: the reference's dispatcher
+        // takes C2R when d1 >= d2, else R2C (src/transpose.cu:117-123); here
+        // both are costed, since which one keeps its rows inside shared
+        // memory decides the faster one for tall or wide slices.
+        for (int k : {T213_PLAN_C2R, T213_PLAN_R2C}) {
+          Plan tmp;
+          tmp.d1 = d1;
+          tmp.d2 = d2;
+          tmp.d3 = d3;
+          tmp.eb = eb;
+          build_plan(tmp, k, 0);
+          // ties go to the reference's choice
+          const bool ref_choice = (k == T213_PLAN_C2R) == (d1 >= d2);
+          cands.push_back({k, 0, plan_cost(tmp) * (ref_choice ? 1.0 : 1.0001)});
+        }
+        if (kind == T213_PLAN_AUTO && !one_pass) {
+          // The ragged bands against the others: the estimates of the classes
+          // that lose to them, or win, are set right here, where they are the
+          // alternative (kRaggedCost has the measurements).
+          for (Cand &c : cands) {
+            if (c.est >= 1e8) continue;
+            if (c.kind == T213_PLAN_C2R || c.kind == T213_PLAN_R2C) {
+              Plan tmp;
+              tmp.d1 = d1;
+              tmp.d2 = d2;
+              tmp.d3 = d3;
+              tmp.eb = eb;
+              build_plan(tmp, c.kind, 0);
+              if (gather_plan_cost(tmp) > plan_cost(tmp)) c.est *= 2;
+            } else if (!(m == n && c.t == m)) {
+              const bool bands = c.kind != T213_PLAN_BLOCKS;
+              if (c.t * eb % 16 == 0 && c.t * eb >= 448)
+                c.est = bands ? std::min(c.est, kRaggedCost - 0.1) : c.est;
+              else if (!(bands && eb >= 8 && c.t * eb >= 1024))
+                c.est += 4;
+            }
+          }
+          cands.push_back({kPlanRagged, 0, kRaggedCost});
+        }
+        std::sort(cands.begin(), cands.end(), [](const Cand &a, const Cand &b) { return a.est < b.est; });
+        for (const Cand &c : cands) {
           if (c.est >= 1e8) continue;
-          if (c.kind == T213_PLAN_C2R || c.kind == T213_PLAN_R2C) {
-            Plan tmp;
-            tmp.d1 = d1;
-            tmp.d2 = d2;
-            tmp.d3 = d3;
-            tmp.eb = eb;
-            build_plan(tmp, c.kind, 0);
-            if (gather_plan_cost(tmp) > plan_cost(tmp)) c.est *= 2;
-          } else if (!(m == n && c.t == m)) {
-            const bool bands = c.kind != T213_PLAN_BLOCKS;
-            if (c.t * eb % 16 == 0 && c.t * eb >= 448)
-              c.est = bands ? std::min(c.est, kRaggedCost - 0.1) : c.est;
-            else if (!(bands && eb >= 8 && c.t * eb >= 1024))
-              c.est += 4;
+          auto P = new_plan(d1, d2, d3, eb);
+          if (build_plan(*P, c.kind, c.t) == T213_OK) {
+            P->est_cost = plan_cost(*P);
+            best = P;
+            break;
           }
         }
-        cands.push_back({kPlanRagged, 0, kRaggedCost});
-      }
-      std::sort(cands.begin(), cands.end(), [](const Cand &a, const Cand &b) { return a.est < b.est; });
-      for (const Cand &c : cands) {
-        if (c.est >= 1e8) continue;
-        auto P = new_plan(d1, d2, d3, eb);
-        if (build_plan(*P, c.kind, c.t) == T213_OK) {
-          P->est_cost = plan_cost(*P);
-          best = P;
-          break;
-        }
-      }
       }
       if (!best) {
         *status = T213_ERR_UNSUPPORTED;
